@@ -28,12 +28,6 @@
 namespace clb
 {
 constexpr int kStackDepth    = 24; // bound checked against the built tree depth
-// Leaf triangles tested per traversal step.  A node's triangles are tested
-// one per step and the next node is visited only after them, so the visit
-// order is unchanged; but a lane with a long leaf no longer holds its warp in
-// a loop while the other lanes wait: they take their own node steps meanwhile
-// (1 was faster than 2, 4, 8 or all at once on configs 2 and 5).
-constexpr int kTrisPerStep = 1;
 constexpr int kTraceBlock    = 128;
 constexpr uint32_t kMissPrim = 0xffffffffu;
 
@@ -186,7 +180,12 @@ __device__ __forceinline__ uint32_t intersectNode(const uint4* __restrict__ node
 }
 
 // Per-ray traversal state, advanced one step at a time: a node test (when no
-// triangle of the previous node is pending) and one triangle test.
+// triangle of the previous node is pending) and one triangle test.  A node's
+// triangles are tested one per step and the next node is visited only after
+// them, so the visit order is unchanged; but a lane with a long leaf does not
+// hold its warp in a loop while the other lanes wait: they take their own node
+// steps meanwhile (1 was faster than 2, 4, 8 or all at once on configs 2 and
+// 5; triangle tests in only every second or third step were within 1%).
 struct Trav
 {
     RayPre   pre;
@@ -217,15 +216,15 @@ __device__ __forceinline__ void travInit(Trav& s, f3 o, f3 d, float tmin, float 
     s.b1 = s.b2 = 0.0f;
 }
 
-// One traversal step.  ANY: stop at the first hit in (tmin, tmax) (shadow
+// One traversal step.  ANY (a constant in the wave kernels): stop at the first hit in (tmin, tmax) (shadow
 // rays; the reference searches for the closest hit there, optix.cu:99-109,
 // which gives the same visibility).  Closest: smallest t in (tmin, tmax),
 // ties to the lower primitive id.  `stack` points at this thread's column of
 // a shared [bvh.stackDepth][kTraceBlock] array.  Returns true when the ray is
 // finished (s.best: primitive id or kMissPrim; s.bt, s.b1, s.b2).
-template <bool ANY, bool STATS>
+template <bool STATS>
 __device__ __forceinline__ bool travStep(const BvhView& bvh, Trav& s, uint2* stack, TraceCounters* cnt, uint32_t* err,
-                                         const uint8_t* keyLut)
+                                         const uint8_t* keyLut, const bool ANY)
 {
     if (s.tg.y == 0u && s.ng.y > 0x00ffffffu)
     {
@@ -251,7 +250,7 @@ __device__ __forceinline__ bool travStep(const BvhView& bvh, Trav& s, uint2* sta
         s.ng = make_uint2(cb, (hits & 0xff000000u) | im);
         s.tg = make_uint2(tb, hits & 0x00ffffffu);
     }
-    for (int tk = 0; tk < kTrisPerStep && s.tg.y; ++tk)
+    if (s.tg.y)
     {
         uint32_t k = __ffs(s.tg.y) - 1;
         s.tg.y &= ~(1u << k);
@@ -299,7 +298,7 @@ __device__ __forceinline__ uint32_t traverse(const BvhView& bvh, f3 o, f3 d, flo
 {
     Trav s;
     travInit(s, o, d, tmin, tmax);
-    while (!travStep<ANY, STATS>(bvh, s, stack, cnt, err, keyLut))
+    while (!travStep<STATS>(bvh, s, stack, cnt, err, keyLut, ANY))
     {
     }
     *tHit  = s.bt;
@@ -373,9 +372,9 @@ __device__ __forceinline__ f3 xformDir(const float4* __restrict__ m, f3 d)
     return {a.x * d.x + a.y * d.y + a.z * d.z, b.x * d.x + b.y * d.y + b.z * d.z, c.x * d.x + c.y * d.y + c.z * d.z};
 }
 
-template <bool ANY, bool STATS>
+template <bool STATS>
 __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* stack, TraceCounters* cnt, uint32_t* err,
-                                          const uint8_t* keyLut)
+                                          const uint8_t* keyLut, const bool ANY)
 {
     if (s.tg.y == 0u && s.ng.y > 0x00ffffffu)
     {
@@ -496,7 +495,7 @@ __device__ __forceinline__ uint32_t traverse2(const BvhView& bvh, f3 o, f3 d, fl
 {
     Trav2 s;
     trav2Init(bvh, s, o, d, tmin, tmax);
-    while (!trav2Step<ANY, STATS>(bvh, s, stack, cnt, err, keyLut))
+    while (!trav2Step<STATS>(bvh, s, stack, cnt, err, keyLut, ANY))
     {
     }
     *tHit  = s.bt;

@@ -55,10 +55,10 @@ __device__ __forceinline__ uint32_t warpAppend(uint32_t* counter, bool pred)
     return base + __popc(mask & ((1u << laneId()) - 1u));
 }
 
-__device__ __forceinline__ uint32_t warpFetch(uint32_t* counter)
+__device__ __forceinline__ uint32_t warpFetch(uint32_t* counter, uint32_t chunk)
 {
     uint32_t base = 0u;
-    if (laneId() == 0u) base = atomicAdd(counter, 32u);
+    if (laneId() == 0u) base = atomicAdd(counter, chunk);
     return __shfl_sync(kFull, base, 0);
 }
 
@@ -255,10 +255,9 @@ __device__ __noinline__ void flushRecords(GuideDev g, const uint4* psInfo, Count
 // vertex k holds the throughput T_k that reached it and the path radiance
 // L_k before its emitter sample; (L - L_k) / T_k is the radiance the path
 // gathered from k on, an estimate of the outgoing radiance at k.
-__device__ __noinline__ void flushCacheRecords(CacheDev c, const float4* psE, Counters* ctr, uint32_t slot, float lx,
+__device__ __noinline__ void flushCacheRecords(CacheDev c, uint32_t mask, Counters* ctr, uint32_t slot, float lx,
                                                float ly, float lz)
 {
-    uint32_t      mask = __float_as_uint(psE[slot].w) & ~kCacheTrainBit;
     const float4* h    = c.hist + size_t(slot) * c.histDepth * kCacheHistF4;
     while (mask)
     {
@@ -280,6 +279,25 @@ __device__ __noinline__ void flushCacheRecords(CacheDev c, const float4* psE, Co
     }
 }
 
+// A finished path's radiance into its pixel's sums.
+__device__ __forceinline__ void addToFilm(const Params& P, uint32_t pix, f3 L)
+{
+    float* f = reinterpret_cast<float*>(P.q.film + pix);
+    atomicAdd(f + 0, L.x);
+    atomicAdd(f + 1, L.y);
+    atomicAdd(f + 2, L.z);
+    if (P.q.film64)
+    {
+        double* g = P.q.film64 + 6 * size_t(pix);
+        atomicAdd(g + 0, double(L.x));
+        atomicAdd(g + 1, double(L.y));
+        atomicAdd(g + 2, double(L.z));
+        atomicAdd(g + 3, double(L.x) * double(L.x));
+        atomicAdd(g + 4, double(L.y) * double(L.y));
+        atomicAdd(g + 5, double(L.z) * double(L.z));
+    }
+}
+
 // Film write of finished paths, then regeneration of their slots.  Called by
 // every lane of the warp.
 __device__ __forceinline__ void finishPaths(const Params& P, const WaveParams& wp, int nxt, bool finish, uint32_t slot,
@@ -287,26 +305,12 @@ __device__ __forceinline__ void finishPaths(const Params& P, const WaveParams& w
 {
     if (finish && wp.recStride && slot % wp.recStride == 0u)
         flushRecords(P.g, P.q.psInfo, P.q.ctr, slot, wp.recStride, L.x, L.y, L.z);
-    if (finish && wp.cacheTrain && (__float_as_uint(P.q.psE[slot].w) & ~kCacheTrainBit))
-        flushCacheRecords(P.c, P.q.psE, P.q.ctr, slot, L.x, L.y, L.z);
-    if (finish)
+    if (finish && wp.cacheTrain)
     {
-        uint32_t pix = P.q.psInfo[slot].x;
-        float*   f   = reinterpret_cast<float*>(P.q.film + pix);
-        atomicAdd(f + 0, L.x);
-        atomicAdd(f + 1, L.y);
-        atomicAdd(f + 2, L.z);
-        if (P.q.film64)
-        {
-            double* g = P.q.film64 + 6 * size_t(pix);
-            atomicAdd(g + 0, double(L.x));
-            atomicAdd(g + 1, double(L.y));
-            atomicAdd(g + 2, double(L.z));
-            atomicAdd(g + 3, double(L.x) * double(L.x));
-            atomicAdd(g + 4, double(L.y) * double(L.y));
-            atomicAdd(g + 5, double(L.z) * double(L.z));
-        }
+        const uint32_t mask = __float_as_uint(P.q.psE[slot].w) & ~kCacheTrainBit;
+        if (mask) flushCacheRecords(P.c, mask, P.q.ctr, slot, L.x, L.y, L.z);
     }
+    if (finish) addToFilm(P, P.q.psInfo[slot].x, L);
     uint32_t mask = __ballot_sync(kFull, finish);
     if (mask == 0u) return;
     uint32_t           leader = __ffs(mask) - 1u;
@@ -394,7 +398,7 @@ __device__ __forceinline__ int classifyHit(const BvhView& bvh, const ClassifyVie
 }
 
 // Warp-local supply of queue entries for the persistent traversal kernels.
-// A warp takes 32 consecutive entries per atomicAdd and hands them to its
+// A warp takes `chunk` (32) consecutive entries per atomicAdd and hands them to its
 // idle lanes in lane order, so that a lane whose ray has finished takes the
 // next ray while the others continue (the warp no longer waits for its
 // longest ray), and the rays of a warp stay within a few chunks of the queue.
@@ -408,7 +412,8 @@ __device__ __forceinline__ void supplyInit(uint2* ws)
 
 // Every lane calls it with the same `want` (the lanes to supply); returns
 // the supplied lane's entry, kMissPrim for the others.
-__device__ __forceinline__ uint32_t supplyLanes(uint2* ws, uint32_t* fetch, uint32_t n, uint32_t want)
+__device__ __forceinline__ uint32_t supplyLanes(uint2* ws, uint32_t* fetch, uint32_t n, uint32_t want,
+                                                uint32_t chunk = 32u)
 {
     const uint32_t lane = laneId(), lt = (1u << lane) - 1u;
     uint2          w    = *ws;
@@ -417,8 +422,8 @@ __device__ __forceinline__ uint32_t supplyLanes(uint2* ws, uint32_t* fetch, uint
     {
         if (w.x >= w.y)
         {
-            const uint32_t nb = warpFetch(fetch);
-            w                 = nb >= n ? make_uint2(kMissPrim, kMissPrim) : make_uint2(nb, min(nb + 32u, n));
+            const uint32_t nb = warpFetch(fetch, chunk);
+            w                 = nb >= n ? make_uint2(kMissPrim, kMissPrim) : make_uint2(nb, min(nb + chunk, n));
             if (nb >= n) break;
         }
         const uint32_t avail = w.y - w.x, r = __popc(want & lt);
@@ -431,6 +436,21 @@ __device__ __forceinline__ uint32_t supplyLanes(uint2* ws, uint32_t* fetch, uint
     if (lane == 0u) *ws = w;
     __syncwarp();
     return item;
+}
+
+// Rays per warp: all 32 lanes, or with fewer rays than the grid has lanes an
+// even share of them, since a step costs a warp what its lanes' divergent loads
+// and branches cost together.
+__device__ __forceinline__ uint32_t laneShare(uint32_t n)
+{
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    return min(32u, max(1u, (n + warps - 1u) / warps));
+}
+// Of the idle lanes, those to supply so that at most `share` lanes have a ray.
+__device__ __forceinline__ uint32_t shareOf(uint32_t idle, uint32_t share)
+{
+    for (uint32_t x = 32u - share; x > 0u && idle; --x) idle &= idle - 1u;
+    return idle;
 }
 
 // Ray indices of the wave queues stay below this (kTraceClosest and the
@@ -499,9 +519,9 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
             {
                 bool done;
                 if constexpr (TWO)
-                    done = trav2Step<false, STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut);
+                    done = trav2Step<STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut, false);
                 else
-                    done = travStep<false, STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut);
+                    done = travStep<STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut, false);
                 if (done)
                 {
                     if constexpr (TWO)
@@ -662,9 +682,9 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
             {
                 bool done;
                 if constexpr (TWO)
-                    done = trav2Step<true, STATS>(P.sc.bvh, s, stack + threadIdx.x, &tc, &P.q.ctr->error, keyLut);
+                    done = trav2Step<STATS>(P.sc.bvh, s, stack + threadIdx.x, &tc, &P.q.ctr->error, keyLut, true);
                 else
-                    done = travStep<true, STATS>(P.sc.bvh, s, stack + threadIdx.x, &tc, &P.q.ctr->error, keyLut);
+                    done = travStep<STATS>(P.sc.bvh, s, stack + threadIdx.x, &tc, &P.q.ctr->error, keyLut, true);
                 if (done)
                 {
                     P.q.vis[ray] = s.best == kMissPrim ? 1 : 0;
@@ -676,9 +696,21 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
     if (STATS) warpStats(tc, &P.q.ctr->statNodesS, &P.q.ctr->statTrisS);
 }
 
+// One path vertex in registers: the path's state before and after it, and what
+// the vertex adds to the queues.
+struct VertexState
+{
+    uint32_t slot, depth, cst; // cst: radiance-cache training bit and recorded depths
+    f3       d, T, E, L;       // ray direction; throughput, escape weight / BSDF pdf, radiance (updated)
+    bool     shadow1 = false, shadow2 = false, pushRay = false, finish = false;
+    uint32_t info2 = 0u, recBit = 0u; // next depth and random counter; recorded guide vertex
+    f3       pHit{0, 0, 0}, ndir{0, 0, 0};                            // vertex, next direction
+    f3       sdir{0, 0, 0}, Li{0, 0, 0}, sdir2{0, 0, 0}, Ld{0, 0, 0}; // shadow rays and their radiance
+};
+
 // CMP: 1 = the reference's estimator (all CL_COMPAT_* flags), 0 = the
 // corrected one, 2 = a mix read at run time; ALIAS: alias-table dome sampling.
-// MAT: the shading class this launch serves (BSDF type 0-2, or 3 = escaped
+// MAT: the shading class served (BSDF type 0-2, or 3 = escaped
 // rays), from the class queues written by kTraceClosest; -1 = every ray of
 // the ray queue.  Specialising keeps each instantiation free of the other
 // modes' and materials' code.
@@ -687,13 +719,11 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
 // sampled with probability a = the sum of its lobe weights (1 - bsdf_fraction,
 // or learned); every pdf of the BSDF strategy - emitter-sample MIS, the
 // throughput update and the escaped-ray MIS - becomes (1 - a) p_bsdf + a p_guide.
-template <bool DL, int CMP, bool ALIAS, int MAT, bool GUIDE = false>
-__global__ void __launch_bounds__(128) kShade(Params P, int cur)
+template <bool DL, int CMP, bool ALIAS, int MAT, bool GUIDE>
+__device__ __forceinline__ void shadeVertex(const Params& P, const WaveParams& wp, VertexState& vs, Rng& rng, uint32_t i,
+                                            float4 hh, uint4 ti, const HitAttr& a0)
 {
-    const WaveParams wp = *P.wp;
-    const SceneDev&  sc = P.sc;
-    const uint32_t   n  = MAT < 0 ? loadCount(&P.q.ctr->rayCount[cur]) : loadCount(&P.q.ctr->classCount[MAT < 0 ? 0 : MAT]);
-    const int        nxt = cur ^ 1;
+    const SceneDev& sc = P.sc;
     // The guided mixture pdf needs the sampling densities of the BSDF: a
     // guided kernel never takes the reference's pdf functions (setGuiding also
     // refuses every CL_COMPAT_* flag).
@@ -702,315 +732,326 @@ __global__ void __launch_bounds__(128) kShade(Params P, int cur)
     const bool compatEsc   = CMP == 2 ? (wp.flags & CL_COMPAT_ESCAPE) != 0 : CMP == 1;
     const bool alias       = ALIAS;
     const uint32_t N       = sc.numEmitters;
+    const uint32_t slot = vs.slot, depth = vs.depth, prim = __float_as_uint(hh.y);
+    const f3       d    = vs.d;
+    uint32_t &     cst = vs.cst, &info2 = vs.info2, &recBit = vs.recBit;
+    f3 &           L = vs.L, &T = vs.T, &E = vs.E, &pHit = vs.pHit, &sdir = vs.sdir, &Li = vs.Li, &sdir2 = vs.sdir2,
+       &           Ld = vs.Ld, &ndir = vs.ndir;
+    bool &         shadow1 = vs.shadow1, &shadow2 = vs.shadow2, &pushRay = vs.pushRay, &finish = vs.finish;
+    f3             tIn{0, 0, 0};
+    if (MAT == kClassEscaped || (MAT < 0 && prim == kMissPrim))
+    {
+        // evaluateEscapedRays (raygeneration.cu:105-136)
+        if (sc.hasDome)
+        {
+            f3 Le = domeEval(sc.dome, d, !compatEsc);
+            if (depth == 1u)
+                L = L + Le;
+            else if (compatEsc)
+                L = L + T * (Le * E);
+            else
+            {
+                float pd = domePdf(sc.dome, d, true) / float(N);
+                float w  = E.x / (E.x + pd);
+                L        = L + T * (Le * w);
+            }
+        }
+        finish = true;
+    }
+    else if (!DL && P.c.termDepth && depth == P.c.termDepth && !(cst & kCacheTrainBit))
+    {
+        // The path ends in the radiance cache (kCacheMlp's prediction).
+        float4 cl = P.c.L[i];
+        L         = L + T * f3{cl.x, cl.y, cl.z};
+        finish    = true;
+    }
+    else if (!DL && depth == wp.maxDepth)
+        finish = true;
+    else
+    {
+        HitAttr a    = (MAT >= 0 && MAT != kClassEscaped) ? a0 : hitAttributesTri(sc, ti, hh.z, hh.w);
+        MatTex  tx;
+        Bsdf    bsdf = loadMaterial(sc.mats, a.material, &tx);
+        if (tx.refl | tx.rough) applyTextures(sc.tex, tx, a.uv, &bsdf);
+        if (!DL && (cst & kCacheTrainBit) && wp.cacheTrain && depth <= P.c.histDepth)
+        {
+            // Radiance-cache training path: vertex history (flushCacheRecords).
+            float4* h = P.c.hist + (size_t(slot) * P.c.histDepth + depth - 1u) * kCacheHistF4;
+            f3 pn = (a.p - f3{P.g.boxMin[0], P.g.boxMin[1], P.g.boxMin[2]}) * P.g.boxScale;
+            h[0]  = make_float4(pn.x, pn.y, pn.z, T.x);
+            h[1]  = make_float4(a.ns.x, a.ns.y, a.ns.z, T.y);
+            h[2]  = make_float4(-d.x, -d.y, -d.z, T.z);
+            h[3]  = make_float4(L.x, L.y, L.z, 0.0f);
+            cst |= 1u << (depth - 1u);
+            reinterpret_cast<uint32_t*>(P.q.psE + slot)[3] = cst;
+        }
+        if (MAT >= 0) bsdf.type = uint32_t(MAT);
+        pHit         = a.p;
+        f3    wo     = -d;
+        guide::Lobes G;
+        float        gf = 1.0f; // probability of BSDF sampling: 1 - sum of the lobe weights
+        // Vertices shallower than the guide's minimum depth were not inferred, and near-specular
+        // ones (GGX alpha below the guide's minimum) are not guided: BSDF sampling alone (zero
+        // lobe weights), no training record.
+        const bool guided =
+            GUIDE && depth >= P.g.minDepth && (bsdf.type == kDiffuse || bsdf.alpha >= P.g.minAlpha);
+        if (GUIDE && !guided)
+#pragma unroll
+            for (int k = 0; k < guide::kLobes; ++k)
+            {
+                G.l[k] = make_float4(0.0f, 0.0f, 1.0f, 1.0f);
+                G.w[k] = 0.0f;
+            }
+        if (guided)
+        {
+            const float4* lb = P.g.lobes + size_t(i) * kLobeF4;
+#pragma unroll
+            for (int k = 0; k < guide::kLobes; ++k) G.l[k] = lb[k];
+            float4 w0 = lb[8], w1 = lb[9];
+            G.w[0] = w0.x, G.w[1] = w0.y, G.w[2] = w0.z, G.w[3] = w0.w;
+            G.w[4] = w1.x, G.w[5] = w1.y, G.w[6] = w1.z, G.w[7] = w1.w;
+            gf = 1.0f - (((w0.x + w0.y) + (w0.z + w0.w)) + ((w1.x + w1.y) + (w1.z + w1.w)));
+        }
+        f2    u      = rng.next2D();
+        // Shading frame (Material::getShadingFrame, material.h:128-147).
+        // Path tracing passes (ng, ns) swapped (raygeneration.cu:324-330):
+        // without a normal map the frame's normal is then the geometric
+        // one (the compat quirk); with one, the map's tangent frame and
+        // the pull-up use the shading normal, kept in both estimators.
+        // The reference's direct-lighting kernel builds {dpdv, dpdu, ns}
+        // itself and ignores normal maps (raygeneration.cu:179,237).
+        Frame fr;
+        if (tx.normal && !(DL && compatFrame))
+        {
+            float4 nt = texLookup(sc.tex, tx.normal, a.uv);
+            fr = normalMappedFrame(wo, a.dpdu, a.dpdv, a.ns, f3{nt.x, nt.y, nt.z}, bsdf.type != kDielectric);
+        }
+        else
+            fr = Frame{a.dpdv, a.dpdu, (!DL && compatFrame) ? a.ng : a.ns};
+        // Emitter sampling with MIS (raygeneration.cu:332-384 / 174-227).
+        if (N > 0u)
+        {
+            uint32_t pick = min(uint32_t(floorf(u.x * float(N))), N - 1u);
+            f2       us{u.x * float(N) - float(pick), u.y};
+            f3       ldir{0, 0, 0};
+            float    lpdf = 0.0f;
+            const EmitterDev& em = sc.emitters[pick];
+            f3 value = em.type == 0u ? directionalSample(em.dl, us, &ldir, &lpdf)
+                                     : domeSample(sc.dome, us, alias, &ldir, &lpdf);
+            if (compatEsc) value = value * float(N);
+            if (lpdf == 0.0f) value = {0.0f, 0.0f, 0.0f};
+            if (nonzero(value) && lpdf > 0.0f)
+            {
+                f3 wiL = fr.toLocal(ldir), woL = fr.toLocal(wo);
+                f3 f   = bsdfEval(bsdf, woL, wiL);
+                if (nonzero(f))
+                {
+                    float bp = bsdfPdf(bsdf, woL, wiL, compatPdf);
+                    if (GUIDE) bp = gf * bp + guide::mixturePdf(G, ldir);
+                    float c  = (DL && compatEsc) ? wiL.z : fabsf(wiL.z);
+                    f3    baseV = DL ? value : T * value;
+                    float w, pl;
+                    if (compatEsc)
+                    {
+                        w  = misBalanced(lpdf, bp);
+                        pl = lpdf;
+                    }
+                    else
+                    {
+                        pl = lpdf / float(N);
+                        w  = em.type == 1u ? misBalanced(pl, bp) : 1.0f;
+                    }
+                    Li      = baseV * f;
+                    Li      = Li * c;
+                    Li      = Li * w;
+                    Li      = Li / pl;
+                    sdir    = ldir;
+                    shadow1 = true;
+                }
+            }
+        }
+        // BSDF sampling with MIS (raygeneration.cu:391-455 / 234-281).
+        float us  = GUIDE ? rng.next1D() : 0.0f;
+        f2    u2  = rng.next2D();
+        f3    woL = fr.toLocal(wo);
+        f3    wiL{0, 0, 0};
+        float bp = 0.0f;
+        f3    f{0.0f, 0.0f, 0.0f};
+        f3    gdir{0.0f, 0.0f, 0.0f};
+        if (!GUIDE || us < gf)
+            f = bsdfSample(bsdf, woL, u2, &wiL, &bp);
+        else
+        {
+            gdir = guide::mixtureSample(G, us - gf, u2.x, u2.y);
+            wiL  = fr.toLocal(gdir);
+            f    = bsdfEval(bsdf, woL, wiL);
+            bp   = bsdfPdf(bsdf, woL, wiL, false);
+        }
+        const float bpB = bp; // BSDF pdf of the sampled direction (training records)
+        if (GUIDE && nonzero(f))
+        {
+            if (us < gf) gdir = fr.toWorld(wiL);
+            bp = gf * bp + guide::mixturePdf(G, gdir);
+        }
+        // The corrected estimator stops paths whose sampled pdf is not
+        // positive (0 or NaN at the rim of the cosine warp); the
+        // reference's update divides by it (raygeneration.cu:430).
+        if (!nonzero(f) || (!compatEsc && !(bp > 0.0f)))
+            finish = true;
+        else
+        {
+            f3    dir      = GUIDE ? gdir : fr.toWorld(wiL);
+            float lightPdf = sc.hasDome ? domePdf(sc.dome, dir, !compatEsc) : 0.0f;
+            if (DL)
+            {
+                if (sc.hasDome && !(compatEsc && !(lightPdf > 0.0f)))
+                {
+                    float c  = compatEsc ? wiL.z : fabsf(wiL.z);
+                    float pl = compatEsc ? lightPdf : lightPdf / float(N);
+                    Ld       = domeEval(sc.dome, dir, !compatEsc);
+                    float w  = misBalanced(bp, pl);
+                    f3    kk{f.x * c * w / bp, f.y * c * w / bp, f.z * c * w / bp};
+                    Ld      = Ld * kk;
+                    sdir2   = dir;
+                    shadow2 = true;
+                }
+                finish = true;
+            }
+            else
+            {
+                float c = fabsf(wiL.z);
+                f3    tk{f.x * c / bp, f.y * c / bp, f.z * c / bp};
+                tIn        = T;
+                T          = T * tk;
+                bool alive = true;
+                if (wp.rrStart > 0u && depth >= wp.rrStart)
+                {
+                    float q = maxComp(T);
+                    q       = q < 1.0f ? q : 1.0f;
+                    float r = rng.next1D();
+                    if (r >= q)
+                        alive = false;
+                    else
+                        T = T / q;
+                }
+                if (alive)
+                {
+                    if (compatEsc)
+                    {
+                        if (!(lightPdf > 0.0f))
+                            alive = false;
+                        else
+                        {
+                            float w = misBalanced(bp, lightPdf);
+                            E       = {f.x * c * w / bp, f.y * c * w / bp, f.z * c * w / bp};
+                        }
+                    }
+                    else
+                        E = {bp, 0.0f, 0.0f};
+                }
+                if (alive)
+                {
+                    pushRay = true;
+                    ndir    = dir;
+                    info2   = (depth + 1u) | (rng.ctr << 8);
+                    if (guided && wp.recStride && slot % wp.recStride == 0u && depth <= P.g.histDepth)
+                    {
+                        // Training history of this vertex (flushRecords).
+                        float4* h = P.g.hist + (size_t(slot / wp.recStride) * P.g.histDepth + depth - 1u) *
+                                                   kHistF4;
+                        f3 pn = (a.p - f3{P.g.boxMin[0], P.g.boxMin[1], P.g.boxMin[2]}) * P.g.boxScale;
+                        h[0]  = make_float4(pn.x, pn.y, pn.z, tIn.x);
+                        h[1]  = make_float4(a.ns.x, a.ns.y, a.ns.z, tIn.y);
+                        h[2]  = make_float4(wo.x, wo.y, wo.z, tIn.z);
+                        h[3]  = make_float4(dir.x, dir.y, dir.z, bpB);
+                        h[4]  = make_float4(L.x, L.y, L.z, 0.0f);
+                        recBit = 1u << (depth - 1u);
+                    }
+                }
+                else
+                    finish = true;
+            }
+        }
+    }
+}
+
+template <bool DL, int CMP, bool ALIAS, int MAT, bool GUIDE = false>
+__global__ void __launch_bounds__(128) kShade(Params P, int cur)
+{
+    const WaveParams wp = *P.wp;
+    const SceneDev&  sc = P.sc;
+    const uint32_t   n  = loadCount(&P.q.ctr->classCount[MAT]);
+    const int        nxt = cur ^ 1;
     // Static assignment of 32-ray batches to warps (grid-stride): a dynamic
     // fetch would put a same-address atomicAdd at the head of every batch's
     // chain of dependent gathers.
     const uint32_t gw = gridDim.x * (blockDim.x >> 5);
     for (uint32_t base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32u; base < n; base += gw * 32u)
     {
-        uint32_t i     = base + laneId();
-        bool     valid = i < n;
-        if (MAT >= 0 && valid) i = P.q.classIdx[size_t(MAT) * P.q.slots + i];
-        bool     pushShadow = false, shadow1 = false, shadow2 = false, pushRay = false, finish = false;
-        uint32_t slot = 0u, info2 = 0u, recBit = 0u, vDepth = 0u, cst = 0u;
-        f3       tIn{0, 0, 0};
-        f3       L{0, 0, 0}, T{1, 1, 1}, E{0, 0, 0}, pHit{0, 0, 0}, sdir{0, 0, 0}, Li{0, 0, 0}, sdir2{0, 0, 0},
-            Ld{0, 0, 0}, ndir{0, 0, 0};
+        uint32_t    i = base + laneId();
+        const bool  valid = i < n;
+        VertexState v{};
         if (valid)
         {
-            slot          = P.q.rqSlot[cur][i];
+            i             = P.q.classIdx[size_t(MAT) * P.q.slots + i];
+            v.slot        = P.q.rqSlot[cur][i];
             float4 hh     = P.q.hit[i];
             uint4  ti     = MAT == kClassEscaped ? make_uint4(0u, 0u, 0u, 0u) : P.q.hitIdx[i];
             float4 rd     = P.q.rqD[cur][i];
             // Surface classes: the hit exists, so its vertex gathers start with the
             // path-state loads instead of after the depth tests that need them.
             HitAttr a0{};
-            if constexpr (MAT >= 0 && MAT != kClassEscaped) a0 = hitAttributesTri(sc, ti, hh.z, hh.w);
-            uint4  info   = P.q.psInfo[slot];
-            uint32_t depth = info.z & 0xffu;
-            vDepth         = depth;
+            if constexpr (MAT != kClassEscaped) a0 = hitAttributesTri(sc, ti, hh.z, hh.w);
+            uint4  info = P.q.psInfo[v.slot];
+            v.depth     = info.z & 0xffu;
             Rng    rng{info.x % wp.W, info.x / wp.W, info.y, info.z >> 8};
-            T             = ld3(P.q.psT[slot]);
-            float4 e4     = P.q.psE[slot];
-            E             = ld3(e4);
-            cst           = __float_as_uint(e4.w);
-            L             = ld3(P.q.psL[slot]);
-            f3       d    = ld3(rd);
-            uint32_t prim = __float_as_uint(hh.y);
-            if (MAT == kClassEscaped || (MAT < 0 && prim == kMissPrim))
-            {
-                // evaluateEscapedRays (raygeneration.cu:105-136)
-                if (sc.hasDome)
-                {
-                    f3 Le = domeEval(sc.dome, d, !compatEsc);
-                    if (depth == 1u)
-                        L = L + Le;
-                    else if (compatEsc)
-                        L = L + T * (Le * E);
-                    else
-                    {
-                        float pd = domePdf(sc.dome, d, true) / float(N);
-                        float w  = E.x / (E.x + pd);
-                        L        = L + T * (Le * w);
-                    }
-                }
-                finish = true;
-            }
-            else if (!DL && P.c.termDepth && depth == P.c.termDepth && !(cst & kCacheTrainBit))
-            {
-                // The path ends in the radiance cache (kCacheMlp's prediction).
-                float4 cl = P.c.L[i];
-                L         = L + T * f3{cl.x, cl.y, cl.z};
-                finish    = true;
-            }
-            else if (!DL && depth == wp.maxDepth)
-                finish = true;
-            else
-            {
-                HitAttr a    = (MAT >= 0 && MAT != kClassEscaped) ? a0 : hitAttributesTri(sc, ti, hh.z, hh.w);
-                MatTex  tx;
-                Bsdf    bsdf = loadMaterial(sc.mats, a.material, &tx);
-                if (tx.refl | tx.rough) applyTextures(sc.tex, tx, a.uv, &bsdf);
-                if (!DL && (cst & kCacheTrainBit) && wp.cacheTrain && depth <= P.c.histDepth)
-                {
-                    // Radiance-cache training path: vertex history (flushCacheRecords).
-                    float4* h = P.c.hist + (size_t(slot) * P.c.histDepth + depth - 1u) * kCacheHistF4;
-                    f3 pn = (a.p - f3{P.g.boxMin[0], P.g.boxMin[1], P.g.boxMin[2]}) * P.g.boxScale;
-                    h[0]  = make_float4(pn.x, pn.y, pn.z, T.x);
-                    h[1]  = make_float4(a.ns.x, a.ns.y, a.ns.z, T.y);
-                    h[2]  = make_float4(-d.x, -d.y, -d.z, T.z);
-                    h[3]  = make_float4(L.x, L.y, L.z, 0.0f);
-                    cst |= 1u << (depth - 1u);
-                    reinterpret_cast<uint32_t*>(P.q.psE + slot)[3] = cst;
-                }
-                if (MAT >= 0) bsdf.type = uint32_t(MAT);
-                pHit         = a.p;
-                f3    wo     = -d;
-                guide::Lobes G;
-                float        gf = 1.0f; // probability of BSDF sampling: 1 - sum of the lobe weights
-                // Vertices shallower than the guide's minimum depth were not inferred, and near-specular
-                // ones (GGX alpha below the guide's minimum) are not guided: BSDF sampling alone (zero
-                // lobe weights), no training record.
-                const bool guided =
-                    GUIDE && depth >= P.g.minDepth && (bsdf.type == kDiffuse || bsdf.alpha >= P.g.minAlpha);
-                if (GUIDE && !guided)
-#pragma unroll
-                    for (int k = 0; k < guide::kLobes; ++k)
-                    {
-                        G.l[k] = make_float4(0.0f, 0.0f, 1.0f, 1.0f);
-                        G.w[k] = 0.0f;
-                    }
-                if (guided)
-                {
-                    const float4* lb = P.g.lobes + size_t(i) * kLobeF4;
-#pragma unroll
-                    for (int k = 0; k < guide::kLobes; ++k) G.l[k] = lb[k];
-                    float4 w0 = lb[8], w1 = lb[9];
-                    G.w[0] = w0.x, G.w[1] = w0.y, G.w[2] = w0.z, G.w[3] = w0.w;
-                    G.w[4] = w1.x, G.w[5] = w1.y, G.w[6] = w1.z, G.w[7] = w1.w;
-                    gf = 1.0f - (((w0.x + w0.y) + (w0.z + w0.w)) + ((w1.x + w1.y) + (w1.z + w1.w)));
-                }
-                f2    u      = rng.next2D();
-                // Shading frame (Material::getShadingFrame, material.h:128-147).
-                // Path tracing passes (ng, ns) swapped (raygeneration.cu:324-330):
-                // without a normal map the frame's normal is then the geometric
-                // one (the compat quirk); with one, the map's tangent frame and
-                // the pull-up use the shading normal, kept in both estimators.
-                // The reference's direct-lighting kernel builds {dpdv, dpdu, ns}
-                // itself and ignores normal maps (raygeneration.cu:179,237).
-                Frame fr;
-                if (tx.normal && !(DL && compatFrame))
-                {
-                    float4 nt = texLookup(sc.tex, tx.normal, a.uv);
-                    fr = normalMappedFrame(wo, a.dpdu, a.dpdv, a.ns, f3{nt.x, nt.y, nt.z}, bsdf.type != kDielectric);
-                }
-                else
-                    fr = Frame{a.dpdv, a.dpdu, (!DL && compatFrame) ? a.ng : a.ns};
-                // Emitter sampling with MIS (raygeneration.cu:332-384 / 174-227).
-                if (N > 0u)
-                {
-                    uint32_t pick = min(uint32_t(floorf(u.x * float(N))), N - 1u);
-                    f2       us{u.x * float(N) - float(pick), u.y};
-                    f3       ldir{0, 0, 0};
-                    float    lpdf = 0.0f;
-                    const EmitterDev& em = sc.emitters[pick];
-                    f3 value = em.type == 0u ? directionalSample(em.dl, us, &ldir, &lpdf)
-                                             : domeSample(sc.dome, us, alias, &ldir, &lpdf);
-                    if (compatEsc) value = value * float(N);
-                    if (lpdf == 0.0f) value = {0.0f, 0.0f, 0.0f};
-                    if (nonzero(value) && lpdf > 0.0f)
-                    {
-                        f3 wiL = fr.toLocal(ldir), woL = fr.toLocal(wo);
-                        f3 f   = bsdfEval(bsdf, woL, wiL);
-                        if (nonzero(f))
-                        {
-                            float bp = bsdfPdf(bsdf, woL, wiL, compatPdf);
-                            if (GUIDE) bp = gf * bp + guide::mixturePdf(G, ldir);
-                            float c  = (DL && compatEsc) ? wiL.z : fabsf(wiL.z);
-                            f3    baseV = DL ? value : T * value;
-                            float w, pl;
-                            if (compatEsc)
-                            {
-                                w  = misBalanced(lpdf, bp);
-                                pl = lpdf;
-                            }
-                            else
-                            {
-                                pl = lpdf / float(N);
-                                w  = em.type == 1u ? misBalanced(pl, bp) : 1.0f;
-                            }
-                            Li      = baseV * f;
-                            Li      = Li * c;
-                            Li      = Li * w;
-                            Li      = Li / pl;
-                            sdir    = ldir;
-                            shadow1 = true;
-                        }
-                    }
-                }
-                // BSDF sampling with MIS (raygeneration.cu:391-455 / 234-281).
-                float us  = GUIDE ? rng.next1D() : 0.0f;
-                f2    u2  = rng.next2D();
-                f3    woL = fr.toLocal(wo);
-                f3    wiL{0, 0, 0};
-                float bp = 0.0f;
-                f3    f{0.0f, 0.0f, 0.0f};
-                f3    gdir{0.0f, 0.0f, 0.0f};
-                if (!GUIDE || us < gf)
-                    f = bsdfSample(bsdf, woL, u2, &wiL, &bp);
-                else
-                {
-                    gdir = guide::mixtureSample(G, us - gf, u2.x, u2.y);
-                    wiL  = fr.toLocal(gdir);
-                    f    = bsdfEval(bsdf, woL, wiL);
-                    bp   = bsdfPdf(bsdf, woL, wiL, false);
-                }
-                const float bpB = bp; // BSDF pdf of the sampled direction (training records)
-                if (GUIDE && nonzero(f))
-                {
-                    if (us < gf) gdir = fr.toWorld(wiL);
-                    bp = gf * bp + guide::mixturePdf(G, gdir);
-                }
-                // The corrected estimator stops paths whose sampled pdf is not
-                // positive (0 or NaN at the rim of the cosine warp); the
-                // reference's update divides by it (raygeneration.cu:430).
-                if (!nonzero(f) || (!compatEsc && !(bp > 0.0f)))
-                    finish = true;
-                else
-                {
-                    f3    dir      = GUIDE ? gdir : fr.toWorld(wiL);
-                    float lightPdf = sc.hasDome ? domePdf(sc.dome, dir, !compatEsc) : 0.0f;
-                    if (DL)
-                    {
-                        if (sc.hasDome && !(compatEsc && !(lightPdf > 0.0f)))
-                        {
-                            float c  = compatEsc ? wiL.z : fabsf(wiL.z);
-                            float pl = compatEsc ? lightPdf : lightPdf / float(N);
-                            Ld       = domeEval(sc.dome, dir, !compatEsc);
-                            float w  = misBalanced(bp, pl);
-                            f3    kk{f.x * c * w / bp, f.y * c * w / bp, f.z * c * w / bp};
-                            Ld      = Ld * kk;
-                            sdir2   = dir;
-                            shadow2 = true;
-                        }
-                        finish = true;
-                    }
-                    else
-                    {
-                        float c = fabsf(wiL.z);
-                        f3    tk{f.x * c / bp, f.y * c / bp, f.z * c / bp};
-                        tIn        = T;
-                        T          = T * tk;
-                        bool alive = true;
-                        if (wp.rrStart > 0u && depth >= wp.rrStart)
-                        {
-                            float q = maxComp(T);
-                            q       = q < 1.0f ? q : 1.0f;
-                            float r = rng.next1D();
-                            if (r >= q)
-                                alive = false;
-                            else
-                                T = T / q;
-                        }
-                        if (alive)
-                        {
-                            if (compatEsc)
-                            {
-                                if (!(lightPdf > 0.0f))
-                                    alive = false;
-                                else
-                                {
-                                    float w = misBalanced(bp, lightPdf);
-                                    E       = {f.x * c * w / bp, f.y * c * w / bp, f.z * c * w / bp};
-                                }
-                            }
-                            else
-                                E = {bp, 0.0f, 0.0f};
-                        }
-                        if (alive)
-                        {
-                            pushRay = true;
-                            ndir    = dir;
-                            info2   = (depth + 1u) | (rng.ctr << 8);
-                            if (guided && wp.recStride && slot % wp.recStride == 0u && depth <= P.g.histDepth)
-                            {
-                                // Training history of this vertex (flushRecords).
-                                float4* h = P.g.hist + (size_t(slot / wp.recStride) * P.g.histDepth + depth - 1u) *
-                                                           kHistF4;
-                                f3 pn = (a.p - f3{P.g.boxMin[0], P.g.boxMin[1], P.g.boxMin[2]}) * P.g.boxScale;
-                                h[0]  = make_float4(pn.x, pn.y, pn.z, tIn.x);
-                                h[1]  = make_float4(a.ns.x, a.ns.y, a.ns.z, tIn.y);
-                                h[2]  = make_float4(wo.x, wo.y, wo.z, tIn.z);
-                                h[3]  = make_float4(dir.x, dir.y, dir.z, bpB);
-                                h[4]  = make_float4(L.x, L.y, L.z, 0.0f);
-                                recBit = 1u << (depth - 1u);
-                            }
-                        }
-                        else
-                            finish = true;
-                    }
-                }
-            }
-            pushShadow = shadow1 || shadow2;
+            v.T         = ld3(P.q.psT[v.slot]);
+            float4 e4   = P.q.psE[v.slot];
+            v.E         = ld3(e4);
+            v.cst       = __float_as_uint(e4.w);
+            v.L         = ld3(P.q.psL[v.slot]);
+            v.d         = ld3(rd);
+            shadeVertex<DL, CMP, ALIAS, MAT, GUIDE>(P, wp, v, rng, i, hh, ti, a0);
         }
+        const bool pushShadow = v.shadow1 || v.shadow2;
         // Shadow queue (one entry per path vertex).
         uint32_t sIdx = warpAppend(&P.q.ctr->shadowCount, pushShadow);
         if (pushShadow)
         {
             if (sIdx < P.q.shadowCap)
             {
-                uint32_t tag     = slot | (finish ? kLastFlag : 0u);
-                P.q.sqO[sIdx]    = make_float4(pHit.x, pHit.y, pHit.z, __uint_as_float(tag));
-                P.q.sqD[sIdx]    = make_float4(sdir.x, sdir.y, sdir.z, shadow1 ? 1.0f : 0.0f);
-                P.q.sqL[sIdx]    = make_float4(Li.x, Li.y, Li.z, __uint_as_float(vDepth));
+                uint32_t tag     = v.slot | (v.finish ? kLastFlag : 0u);
+                P.q.sqO[sIdx]    = make_float4(v.pHit.x, v.pHit.y, v.pHit.z, __uint_as_float(tag));
+                P.q.sqD[sIdx]    = make_float4(v.sdir.x, v.sdir.y, v.sdir.z, v.shadow1 ? 1.0f : 0.0f);
+                P.q.sqL[sIdx]    = make_float4(v.Li.x, v.Li.y, v.Li.z, __uint_as_float(v.depth));
                 if (DL)
                 {
-                    P.q.sqD2[sIdx] = make_float4(sdir2.x, sdir2.y, sdir2.z, shadow2 ? 1.0f : 0.0f);
-                    P.q.sqL2[sIdx] = make_float4(Ld.x, Ld.y, Ld.z, 0.0f);
+                    P.q.sqD2[sIdx] = make_float4(v.sdir2.x, v.sdir2.y, v.sdir2.z, v.shadow2 ? 1.0f : 0.0f);
+                    P.q.sqL2[sIdx] = make_float4(v.Ld.x, v.Ld.y, v.Ld.z, 0.0f);
                 }
             }
             else
                 atomicOr(&P.q.ctr->error, 4u);
         }
         // Next-bounce ray queue.
-        uint32_t rIdx = warpAppend(&P.q.ctr->rayCount[nxt], pushRay);
-        if (pushRay && rIdx >= P.q.slots)
+        uint32_t rIdx = warpAppend(&P.q.ctr->rayCount[nxt], v.pushRay);
+        if (v.pushRay && rIdx >= P.q.slots)
         {
             atomicOr(&P.q.ctr->error, 8u);
-            pushRay = false;
+            v.pushRay = false;
         }
-        if (pushRay)
+        if (v.pushRay)
         {
-            P.q.rqO[nxt][rIdx]    = make_float4(pHit.x, pHit.y, pHit.z, kRayEps);
-            P.q.rqD[nxt][rIdx]    = make_float4(ndir.x, ndir.y, ndir.z, FLT_MAX);
-            P.q.rqSlot[nxt][rIdx] = slot;
-            P.q.psInfo[slot].z    = info2;
-            if (GUIDE && recBit) P.q.psInfo[slot].w |= recBit;
-            P.q.psT[slot]         = make_float4(T.x, T.y, T.z, 0.0f);
-            P.q.psE[slot]         = make_float4(E.x, E.y, E.z, __uint_as_float(cst));
+            P.q.rqO[nxt][rIdx]    = make_float4(v.pHit.x, v.pHit.y, v.pHit.z, kRayEps);
+            P.q.rqD[nxt][rIdx]    = make_float4(v.ndir.x, v.ndir.y, v.ndir.z, FLT_MAX);
+            P.q.rqSlot[nxt][rIdx] = v.slot;
+            P.q.psInfo[v.slot].z    = v.info2;
+            if (GUIDE && v.recBit) P.q.psInfo[v.slot].w |= v.recBit;
+            P.q.psT[v.slot]         = make_float4(v.T.x, v.T.y, v.T.z, 0.0f);
+            P.q.psE[v.slot]         = make_float4(v.E.x, v.E.y, v.E.z, __uint_as_float(v.cst));
         }
-        if (pushRay || (pushShadow && finish)) P.q.psL[slot] = make_float4(L.x, L.y, L.z, 0.0f);
-        finishPaths(P, wp, nxt, finish && !pushShadow, slot, L);
+        if (v.pushRay || (pushShadow && v.finish)) P.q.psL[v.slot] = make_float4(v.L.x, v.L.y, v.L.z, 0.0f);
+        finishPaths(P, wp, nxt, v.finish && !pushShadow, v.slot, v.L);
     }
 }
 
@@ -1052,6 +1093,190 @@ __global__ void __launch_bounds__(128) kShadowResolve(Params P, int cur)
                 P.q.psL[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         }
         finishPaths(P, wp, nxt, finish, slot, L);
+    }
+}
+
+// The rest of a pass in one launch.  A wave of few rays costs the latency of
+// its longest ray in each of its kernels, whatever their number, so once no
+// path is left to start and at most kTailMaxRays rays are queued, persistent
+// warps take the queued paths and trace each to its end (closest hit, shading,
+// shadow ray, next bounce) with no barrier between the paths' bounces.  The
+// order of a path's additions is the wave kernels'.  A lane holds one path in
+// registers.  Traversal steps run for all lanes that have a ray, closest-hit
+// and shadow rays alike; the vertices are shaded once no lane of the warp is in
+// a traversal: a vertex costs about 20 us of dependent instructions and
+// gathers, and the warp pays it for all its lanes (shading a quarter of the
+// lanes at a time took 1.1 to 1.5 times as long).  With fewer paths than lanes
+// each warp takes an even share of them: a step costs a warp what its lanes'
+// divergent loads and branches cost together.
+// kTailMaxRays: measured with 0 (no tail), 8192, 24576, 32768 and 65536 rays on
+// a 256x256 frame of 10 k triangles (device time 675, 538, 584, 576 and 621
+// us), a 1920x1080 frame of 1.2 M triangles at one sample (3.85, 3.82, 3.71,
+// 3.70 and 3.70 ms), 1280x720x2 over 577 two-level instances at depth 16 (7.5,
+// 6.41, 6.35, 6.36 and 6.40 ms), and four trained samples of the radiance cache
+// at 960x540 (10.3 ms without, 5.35 ms with any of them: after its third wave a
+// pass holds only its 32 k training paths, which last to depth 16).
+// Not for guided passes (every vertex needs its network evaluation first);
+// with the radiance cache only once the waves have brought every path past
+// its query (wp.tailNeed).
+constexpr uint32_t kTailMaxRays = 24576;
+constexpr int      kTailBlocks  = 4; // resident blocks per SM (128 registers)
+enum TailState : uint32_t { kTailIdle, kTailClosest, kTailShadow, kTailShade, kTailResolve };
+
+template <int CMP, bool ALIAS, bool TWO>
+__global__ void __launch_bounds__(kTraceBlock, kTailBlocks) kPathTail(Params P, int cur)
+{
+    extern __shared__ uint2 stack[];
+    __shared__ uint8_t      keyLut[kKeyLutBytes];
+    __shared__ uint2        supply[kTraceBlock / 32];
+    Counters* const  c = P.q.ctr;
+    const uint32_t   n = loadCount(&c->rayCount[cur]);
+    const WaveParams wp = *P.wp;
+    if (n == 0u || n > wp.tailMax || loadCount(&c->drained) < wp.tailNeed) return; // the same in every block
+    fillKeyLut(keyLut);
+    const SceneDev& sc = P.sc;
+    const uint32_t  share = laneShare(n);
+    TraceCounters   tc{0u, 0u};
+    uint2*          ws = supply + (threadIdx.x >> 5);
+    supplyInit(ws);
+    typename TravOf<TWO>::T s;
+    VertexState             v{};
+    Rng                     rng{0u, 0u, 0u, 0u};
+    uint32_t                state = kTailIdle, pix = 0u;
+    unsigned long long      nClosest = 0ull, nShadow = 0ull;
+    bool                    more = true; // the warp's supply is not exhausted (warp-uniform)
+    for (;;)
+    {
+        const uint32_t ended = __ballot_sync(kFull, state >= kTailShade);
+        const uint32_t busy  = __ballot_sync(kFull, state == kTailClosest || state == kTailShadow);
+        bool           start = false;
+        f3             so{0, 0, 0}, sd{0, 0, 0};
+        float          smin = kRayEps;
+        if (ended && !busy)
+        {
+            if (state == kTailResolve)
+            {
+                if (s.best == kMissPrim) v.L = v.L + v.Li;
+                if (v.finish)
+                    state = kTailIdle;
+                else
+                {
+                    state = kTailClosest;
+                    start = true;
+                    so    = v.pHit;
+                    sd    = v.ndir;
+                }
+            }
+            else if (state == kTailShade)
+            {
+                uint4 ti = make_uint4(0u, 0u, 0u, 0u);
+                if (s.best != kMissPrim)
+                {
+                    if constexpr (TWO)
+                    {
+                        ti   = __ldg(&P.sc.triIdx[__ldg(&sc.bvh.inst[s.bestInst].triBase) + s.best]);
+                        ti.w = s.bestInst;
+                    }
+                    else
+                        ti = __ldg(&P.sc.triIdx[s.best]);
+                }
+                v.shadow1 = v.pushRay = v.finish = false;
+                shadeVertex<false, CMP, ALIAS, -1, false>(
+                    P, wp, v, rng, 0u, make_float4(s.bt, __uint_as_float(s.best), s.b1, s.b2), ti, HitAttr{});
+                v.depth += 1u;
+                start = v.shadow1 || v.pushRay;
+                so    = v.pHit;
+                sd    = v.shadow1 ? v.sdir : v.ndir;
+                state = v.shadow1 ? kTailShadow : v.pushRay ? kTailClosest : kTailIdle;
+            }
+            if (((ended >> laneId()) & 1u) && state == kTailIdle)
+            {
+                const uint32_t mask = v.cst & ~kCacheTrainBit;
+                if (wp.cacheTrain && mask) flushCacheRecords(P.c, mask, c, v.slot, v.L.x, v.L.y, v.L.z);
+                addToFilm(P, pix, v.L);
+            }
+        }
+        const uint32_t idle = __ballot_sync(kFull, state == kTailIdle);
+        const uint32_t want = shareOf(idle, share);
+        if (more && want)
+        {
+            const uint32_t item = supplyLanes(ws, &c->fetchTrace, n, want, share);
+            more                = ws->x != kMissPrim;
+            if (item != kMissPrim)
+            {
+                const float4 o = P.q.rqO[cur][item], d = P.q.rqD[cur][item];
+                v.slot            = P.q.rqSlot[cur][item];
+                const uint4  info = P.q.psInfo[v.slot];
+                const float4 e4   = P.q.psE[v.slot];
+                pix               = info.x;
+                rng               = Rng{info.x % wp.W, info.x / wp.W, info.y, info.z >> 8};
+                v.depth           = info.z & 0xffu;
+                v.T               = ld3(P.q.psT[v.slot]);
+                v.E               = ld3(e4);
+                v.cst             = __float_as_uint(e4.w);
+                v.L               = ld3(P.q.psL[v.slot]);
+                state             = kTailClosest;
+                start             = true;
+                so                = f3{o.x, o.y, o.z};
+                sd                = f3{d.x, d.y, d.z};
+                smin              = o.w;
+            }
+        }
+        if (start)
+        {
+            if (state == kTailClosest)
+            {
+                v.d = sd;
+                ++nClosest;
+            }
+            else
+                ++nShadow;
+            if constexpr (TWO)
+                trav2Init(sc.bvh, s, so, sd, smin, FLT_MAX);
+            else
+                travInit(s, so, sd, smin, FLT_MAX);
+        }
+        if (__all_sync(kFull, state == kTailIdle))
+        {
+            if (!more) break;
+            continue;
+        }
+        if (state == kTailClosest || state == kTailShadow)
+            for (uint32_t k = 0; k < kRefillSteps; ++k)
+            {
+                bool done;
+                if constexpr (TWO)
+                    done = trav2Step<false>(sc.bvh, s, stack + threadIdx.x, &tc, &c->error, keyLut, state == kTailShadow);
+                else
+                    done = travStep<false>(sc.bvh, s, stack + threadIdx.x, &tc, &c->error, keyLut, state == kTailShadow);
+                if (done)
+                {
+                    state = state == kTailShadow ? kTailResolve : kTailShade;
+                    break;
+                }
+            }
+    }
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        nClosest += __shfl_xor_sync(kFull, nClosest, o);
+        nShadow += __shfl_xor_sync(kFull, nShadow, o);
+    }
+    if (laneId() == 0u && nClosest)
+    {
+        atomicAdd(&c->raysClosest, nClosest);
+        atomicAdd(&c->raysShadow, nShadow);
+    }
+    // The last block to end leaves the queue empty: every block has read the count by then.
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        if (atomicAdd(&c->tailBlocks, 1u) == gridDim.x - 1u)
+        {
+            c->rayCount[cur] = 0u;
+            c->fetchTrace    = 0u;
+            c->tailBlocks    = 0u;
+        }
     }
 }
 
@@ -1316,9 +1541,10 @@ __global__ void kRaygen(Params P, uint32_t count)
     startPath(P, wp, s, s, 0, s);
 }
 
-__global__ void kAdvance(Counters* c, int cur)
+__global__ void kAdvance(Counters* c, const WaveParams* wp, int cur)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (c->pathNext >= wp->totalPaths) c->drained += 1u;
     c->raysClosest += c->rayCount[cur];
     c->raysShadow += c->shadowCount;
     c->rayCount[cur] = 0u;
@@ -1408,6 +1634,16 @@ template <bool DL> ShadeFn shadeKernelT(int mat, uint32_t flags)
     }
 }
 
+template <bool TWO> ShadeFn tailKernelT(uint32_t flags)
+{
+    const uint32_t c  = flags & CL_COMPAT_ALL;
+    const bool     al = (flags & CL_DOME_ALIAS) != 0u;
+    if (c == CL_COMPAT_ALL) return al ? kPathTail<1, true, TWO> : kPathTail<1, false, TWO>;
+    if (c == 0u) return al ? kPathTail<0, true, TWO> : kPathTail<0, false, TWO>;
+    return al ? kPathTail<2, true, TWO> : kPathTail<2, false, TWO>;
+}
+ShadeFn tailKernel(bool two, uint32_t flags) { return two ? tailKernelT<true>(flags) : tailKernelT<false>(flags); }
+
 ShadeFn shadeKernel(bool dl, int mat, uint32_t flags, bool guided = false)
 {
     if (guided && !dl)
@@ -1437,6 +1673,11 @@ Integrator::~Integrator()
     if (evResolved_) cudaEventDestroy(evResolved_);
     if (evCopied_) cudaEventDestroy(evCopied_);
     if (copyStream_) cudaStreamDestroy(copyStream_);
+    if (evFork_) cudaEventDestroy(evFork_);
+    for (auto& e : evJoin_)
+        if (e) cudaEventDestroy(e);
+    for (auto& s : shadeStream_)
+        if (s) cudaStreamDestroy(s);
     if (evA_) cudaEventDestroy(evA_);
     if (evB_) cudaEventDestroy(evB_);
     for (auto& e : evS_)
@@ -1466,6 +1707,9 @@ cl_status Integrator::init(std::string* err)
     CL_CUDA(cudaStreamCreateWithFlags(&copyStream_, cudaStreamNonBlocking), err);
     CL_CUDA(cudaEventCreateWithFlags(&evResolved_, cudaEventDisableTiming), err);
     CL_CUDA(cudaEventCreateWithFlags(&evCopied_, cudaEventDisableTiming), err);
+    CL_CUDA(cudaEventCreateWithFlags(&evFork_, cudaEventDisableTiming), err);
+    for (auto& e : evJoin_) CL_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), err);
+    for (auto& s : shadeStream_) CL_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), err);
     CL_CUDA(cudaEventCreate(&evA_), err);
     CL_CUDA(cudaEventCreate(&evB_), err);
     for (auto& e : evS_) CL_CUDA(cudaEventCreate(&e), err);
@@ -1489,6 +1733,13 @@ cl_status Integrator::init(std::string* err)
                 &b, dl ? (const void*)kShadowResolve<true> : (const void*)kShadowResolve<false>, 128, 0),
             err);
     shadowBlocks_ = std::max(1, b) * numSMs_;
+    for (int two = 0; two < 2; ++two)
+    {
+        CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void*)tailKernel(two != 0, cfg_.flags),
+                                                              kTraceBlock, traceStackBytes(kStackDepth)),
+                err);
+        tailBlocks_[two] = std::max(1, b) * numSMs_;
+    }
     CL_CUDA(cudaFuncSetAttribute(kGuideInfer, cudaFuncAttributeMaxDynamicSharedMemorySize, kGuideMlpSmem), err);
     CL_CUDA(cudaFuncSetAttribute(kCacheMlp, cudaFuncAttributeMaxDynamicSharedMemorySize, kCacheMlpSmem), err);
     // The whole on-chip memory as shared memory, so that the launch holds the
@@ -2431,8 +2682,17 @@ cl_status Integrator::launchWave(int cur, bool profile, std::string* err)
         kCacheMlp<<<cacheMlpBlocks_, guide::kTcThreads, kCacheMlpSmem, stream_>>>(P, cache_->tcWeights());
     }
     if (profile) CL_CUDA(cudaEventRecord(evS_[4], stream_), err);
+    // The four classes are independent: in a captured wave they are parallel
+    // branches (a wave timed stage by stage runs them one after the other).
+    if (!profile) CL_CUDA(cudaEventRecord(evFork_, stream_), err);
     for (int m = 0; m < 4; ++m)
-        shadeKernel(dl, m, cfg_.flags, m < 3 && ((gmask >> m) & 1u))<<<shadeBlocks_, 128, 0, stream_>>>(P, cur);
+    {
+        cudaStream_t st = profile || m == 3 ? stream_ : shadeStream_[m];
+        if (st != stream_) CL_CUDA(cudaStreamWaitEvent(st, evFork_, 0), err);
+        shadeKernel(dl, m, cfg_.flags, m < 3 && ((gmask >> m) & 1u))<<<shadeBlocks_, 128, 0, st>>>(P, cur);
+        if (st != stream_) CL_CUDA(cudaEventRecord(evJoin_[m], st), err);
+    }
+    for (int m = 0; m < 3 && !profile; ++m) CL_CUDA(cudaStreamWaitEvent(stream_, evJoin_[m], 0), err);
     if (profile) CL_CUDA(cudaEventRecord(evS_[2], stream_), err);
     {
         using ShadowFn = void (*)(Params);
@@ -2448,7 +2708,23 @@ cl_status Integrator::launchWave(int cur, bool profile, std::string* err)
     else
         kShadowResolve<false><<<shadowBlocks_, 128, 0, stream_>>>(P, cur);
     if (profile) CL_CUDA(cudaEventRecord(evS_[3], stream_), err);
-    kAdvance<<<1, 32, 0, stream_>>>(c, cur);
+    kAdvance<<<1, 32, 0, stream_>>>(c, P.wp, cur);
+    CL_CUDA(cudaGetLastError(), err);
+    return CL_OK;
+}
+
+// Passes that end in kPathTail: path tracing without guiding, and not where
+// waves are timed or counted one by one.
+bool Integrator::usesTail() const
+{
+    return type_ == CL_INTEGRATOR_PATH_TRACING && !(guide_ && guideCfg_.class_mask) &&
+           !(cfg_.flags & (CL_PROFILE_STAGES | CL_TRACE_STATS));
+}
+
+cl_status Integrator::launchTail(int cur, std::string* err)
+{
+    const Params P = params();
+    tailKernel(twoLevel_, cfg_.flags)<<<tailBlocks(), kTraceBlock, traceStackBytes(P.sc.bvh.stackDepth), stream_>>>(P, cur);
     CL_CUDA(cudaGetLastError(), err);
     return CL_OK;
 }
@@ -2463,7 +2739,11 @@ cl_status Integrator::captureGraph(std::string* err)
     cudaGraph_t g = nullptr;
     CL_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), err);
     cl_status s = CL_OK;
-    for (int w = 0; w < 4 && s == CL_OK; ++w) s = launchWave(w & 1, false, err);
+    for (int w = 0; w < 4 && s == CL_OK; ++w)
+    {
+        s = launchWave(w & 1, false, err);
+        if (s == CL_OK && usesTail()) s = launchTail((w & 1) ^ 1, err);
+    }
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (s != CL_OK) return s;
     CL_CUDA(e, err);
@@ -2580,12 +2860,15 @@ cl_status Integrator::beginPass(uint32_t spp, bool record, bool cacheTrain, uint
     wp.recStride   = record ? recStride_ : 0u;
     wp.cacheTrain  = cacheTrain ? 1u : 0u;
     wp.totalPaths  = (unsigned long long)W_ * H_ * spp;
+    wp.tailMax     = usesTail() ? kTailMaxRays : 0u;
+    wp.tailNeed    = cache_ ? cacheCfg_.prefix_bounces + 2u : 1u;
     memcpy(wp.cam, &camera_, sizeof(camera_));
     CL_CUDA(cudaMemcpyAsync(wp_.p, hostWp_, sizeof(WaveParams), cudaMemcpyHostToDevice, stream_), err);
     uint32_t init = uint32_t(std::min<unsigned long long>(slots_, wp.totalPaths));
     Counters c0{};
     c0.rayCount[0] = init;
     c0.pathNext    = init;
+    c0.drained     = init == wp.totalPaths ? 1u : 0u;
     CL_CUDA(cudaMemcpyAsync(ctr_.p, &c0, sizeof(Counters), cudaMemcpyHostToDevice, stream_), err);
     CL_CUDA(cudaStreamSynchronize(stream_), err); // hostWp_/c0 reused next call
     waveRaysSeen_ = 0ull;
@@ -2603,7 +2886,15 @@ cl_status Integrator::renderPass(uint32_t spp, bool record, bool cacheTrain, std
     CL_CUDA(cudaEventRecord(evA_, stream_), err);
     kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(params(), init);
     CL_CUDA(cudaGetLastError(), err);
-    if (!profile && !graphValid_) CL_TRY(captureGraph(err));
+    // A pass whose camera rays already fit the tail launch needs no wave.
+    const bool small = usesTail() && init == wp.totalPaths && init <= wp.tailMax && wp.tailNeed <= 1u;
+    if (small)
+    {
+        CL_TRY(launchTail(0, err));
+        waves_ += 1;
+    }
+    else if (!profile && !graphValid_)
+        CL_TRY(captureGraph(err));
 
     Counters* dc = ctr_.as<Counters>();
     // Every path needs at most maxDepth waves and at least one path per slot
@@ -2611,7 +2902,7 @@ cl_status Integrator::renderPass(uint32_t spp, bool record, bool cacheTrain, std
     // correct schedule.
     const unsigned long long maxIter =
         ((unsigned long long)(wp.maxDepth + 1) * (wp.totalPaths / slots_ + 2) + 16) / 4 + 1;
-    for (unsigned long long iter = 0;; ++iter)
+    for (unsigned long long iter = 0; !small; ++iter)
     {
         if (iter >= maxIter)
         {

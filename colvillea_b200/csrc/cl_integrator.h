@@ -44,9 +44,11 @@ struct WaveParams
     uint32_t           W, H, frame0, maxDepth, rrStart, flags, dl;
     uint32_t           recStride; // guiding: slots s with s % recStride == 0 record training data (0: off)
     uint32_t           cacheTrain; // radiance cache: 1 = training paths are traced and recorded this pass
-    uint32_t           pad3;
+    uint32_t           tailMax;    // kPathTail ends the pass once at most this many rays are queued (0: never)
     unsigned long long totalPaths;
     float              cam[12];
+    uint32_t           tailNeed;   // and Counters::drained has reached this
+    uint32_t           pad3;
 };
 
 struct Counters
@@ -63,12 +65,12 @@ struct Counters
     uint32_t           fetchInfer; // guiding: inference fetch over the guided class queues
     uint32_t           recCount;   // guiding: training records appended (may exceed the capacity)
     uint32_t           trainCount; // guiding: records the training step reads (clamped)
-    uint32_t           pad2;
+    uint32_t           drained;    // waves since the pass's last path was started, that wave included
     unsigned long long inferred;   // guiding: network evaluations
     uint32_t           cacheCount; // radiance cache: rays terminating into the cache this wave (compacted)
     uint32_t           cacheRec;   // radiance cache: training records appended (may exceed the capacity)
     uint32_t           cacheTrainCount; // radiance cache: records the training step reads (clamped)
-    uint32_t           pad4;
+    uint32_t           tailBlocks; // blocks of kPathTail that have ended
     unsigned long long cacheQueries; // radiance cache: network evaluations
 };
 
@@ -204,6 +206,8 @@ private:
     cl_status clearFilm(std::string* err);
     cl_status captureGraph(std::string* err);
     cl_status launchWave(int cur, bool profile, std::string* err);
+    bool      usesTail() const;
+    cl_status launchTail(int cur, std::string* err);
     Params    params() const;
     ClassifyView classifyView() const;
     BvhView      bvhView() const;
@@ -214,7 +218,9 @@ private:
     cudaStream_t       stream_ = nullptr;
     int                numSMs_ = 148;
     int                traceBlocks_ = 0, shadeBlocks_ = 0, shadowBlocks_ = 0, traceBlocksTwo_ = 0;
+    int                tailBlocks_[2] = {0, 0};
     int                tBlocks() const { return twoLevel_ ? traceBlocksTwo_ : traceBlocks_; }
+    int                tailBlocks() const { return tailBlocks_[twoLevel_ ? 1 : 0]; }
 
     // Meshes as given (host copies), flattened on instance build.
     struct HostMesh
@@ -288,6 +294,8 @@ private:
     float     msBvhWall_ = 0, msBvhAlloc_ = 0; // last full build: host wall time, and its cudaMalloc share
     std::vector<uint64_t> waveRays_;       // CL_PROFILE_STAGES: closest-hit rays of each wave of the last render
     unsigned long long    waveRaysSeen_ = 0;
+    cudaStream_t shadeStream_[3] = {}; // branches of a captured wave
+    cudaEvent_t  evFork_ = nullptr, evJoin_[3] = {};
     cudaEvent_t evA_ = nullptr, evB_ = nullptr, evS_[6] = {};
 
     // Guiding.
