@@ -471,13 +471,11 @@ template <> struct TravOf<true>
 // traverses one ray at a time and takes the next from the warp's supply when
 // it finishes.  The hits' shading classes are appended by kClassifyHits
 // afterwards, in ray order (a class lookup inside the step loop would stall
-// the whole warp on one lane's dependent gathers).  CLASSIFY: the launch is
-// a wave's (kClassifyHits follows); without it the hits are final (the ray
-// query entry points).  TWO: two-level scene (CL_TWO_LEVEL); with CLASSIFY a
-// hit holds the instance-local triangle id and cv.hitInst its instance, which
-// kClassifyHits turns into the global id and the triangle index entry
-// (object-space vertex ids, the instance in .w).
-template <bool STATS, bool CLASSIFY, bool TWO = false>
+// the whole warp on one lane's dependent gathers).  TWO: two-level scene
+// (CL_TWO_LEVEL); a hit holds the instance-local triangle id and cv.hitInst its
+// instance, which kClassifyHits turns into the global id and the triangle
+// index entry (object-space vertex ids, the instance in .w).
+template <bool STATS, bool TWO = false>
 __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlocksFlat) kTraceClosest(BvhView bvh, const float4* __restrict__ O,
                                                                 const float4* __restrict__ D, const uint32_t* count,
                                                                 uint32_t* fetch, float4* __restrict__ hitOut,
@@ -524,23 +522,9 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
                     done = travStep<STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut, false);
                 if (done)
                 {
-                    if constexpr (TWO)
-                    {
-                        if (CLASSIFY)
-                        {
-                            // The instance-local id; kClassifyHits makes it global.
-                            hitOut[ray]     = make_float4(s.bt, __uint_as_float(s.best), s.b1, s.b2);
-                            cv.hitInst[ray] = s.bestInst;
-                        }
-                        else
-                        {
-                            const uint32_t prim =
-                                s.best == kMissPrim ? kMissPrim : __ldg(&bvh.inst[s.bestInst].primBase) + s.best;
-                            hitOut[ray] = make_float4(s.bt, __uint_as_float(prim), s.b1, s.b2);
-                        }
-                    }
-                    else
-                        hitOut[ray] = make_float4(s.bt, __uint_as_float(s.best), s.b1, s.b2);
+                    // Two-level: the instance-local id; kClassifyHits makes it global.
+                    hitOut[ray] = make_float4(s.bt, __uint_as_float(s.best), s.b1, s.b2);
+                    if constexpr (TWO) cv.hitInst[ray] = s.bestInst;
                     ray = kMissPrim;
                     break;
                 }
@@ -1559,27 +1543,80 @@ __global__ void kAdvance(Counters* c, const WaveParams* wp, int cur)
     }
 }
 
-template <bool TWO>
-__global__ void __launch_bounds__(kTraceBlock) kOccluded(BvhView bvh, const float4* __restrict__ O,
-                                                         const float4* __restrict__ D, uint32_t n,
-                                                         uint8_t* __restrict__ occ, uint32_t* err)
+// Ray queries (cl_trace_rays, cl_occluded_rays, cl_trace_stats): the caller's
+// rows of 8 floats are two float4 per ray and are read as they are, and a hit's
+// values go to the caller's arrays' copies, so the host neither packs nor
+// unpacks (on one host core that was 20 of 35 ms for a million closest and a
+// million occlusion queries).  The same persistent loop as kTraceClosest.
+struct QueryOut
+{
+    float*    t; // closest hits: null where only the counters are wanted
+    uint32_t* prim;
+    float*    b1;
+    float*    b2;
+    uint8_t*  occ; // occlusion
+};
+template <bool ANY, bool STATS, bool TWO>
+__global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlocksFlat) kTraceQuery(BvhView bvh, const float4* __restrict__ rays,
+                                                              uint32_t n, QueryOut out, Counters* ctr)
 {
     extern __shared__ uint2 stack[];
     __shared__ uint8_t      keyLut[kKeyLutBytes];
+    __shared__ uint2        supply[kTraceBlock / 32];
     fillKeyLut(keyLut);
-    uint32_t         i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4        o = O[i], d = D[i];
-    float         t, b1, b2;
     TraceCounters tc{0u, 0u};
-    uint32_t      h, hi;
-    if (TWO)
-        h = traverse2<true, false>(bvh, f3{o.x, o.y, o.z}, f3{d.x, d.y, d.z}, o.w, d.w, &t, &b1, &b2, &hi,
-                                   stack + threadIdx.x, &tc, err, keyLut);
-    else
-        h = traverse<true, false>(bvh, f3{o.x, o.y, o.z}, f3{d.x, d.y, d.z}, o.w, d.w, &t, &b1, &b2,
-                                  stack + threadIdx.x, &tc, err, keyLut);
-    occ[i] = h == kMissPrim ? 0 : 1;
+    uint2*        ws = supply + (threadIdx.x >> 5);
+    supplyInit(ws);
+    typename TravOf<TWO>::T s;
+    uint32_t                ray = kMissPrim;
+    for (;;)
+    {
+        const uint32_t idle = __ballot_sync(kFull, ray == kMissPrim);
+        if (uint32_t(__popc(idle)) >= kRefillIdle)
+        {
+            if (ws->x != kMissPrim)
+            {
+                const uint32_t item = supplyLanes(ws, &ctr->fetchTrace, n, idle);
+                if (item != kMissPrim)
+                {
+                    ray            = item;
+                    const float4 o = __ldg(rays + 2 * size_t(item)), d = __ldg(rays + 2 * size_t(item) + 1);
+                    if constexpr (TWO)
+                        trav2Init(bvh, s, f3{o.x, o.y, o.z}, f3{d.x, d.y, d.z}, o.w, d.w);
+                    else
+                        travInit(s, f3{o.x, o.y, o.z}, f3{d.x, d.y, d.z}, o.w, d.w);
+                }
+            }
+            if (__all_sync(kFull, ray == kMissPrim)) break;
+        }
+        if (ray != kMissPrim)
+            for (uint32_t k = 0; k < kRefillSteps; ++k)
+            {
+                bool done;
+                if constexpr (TWO)
+                    done = trav2Step<STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut, ANY);
+                else
+                    done = travStep<STATS>(bvh, s, stack + threadIdx.x, &tc, &ctr->error, keyLut, ANY);
+                if (done)
+                {
+                    if (ANY)
+                        out.occ[ray] = s.best == kMissPrim ? 0 : 1;
+                    else if (out.t)
+                    {
+                        uint32_t prim = s.best;
+                        if constexpr (TWO)
+                            if (prim != kMissPrim) prim += __ldg(&bvh.inst[s.bestInst].primBase);
+                        out.t[ray]    = s.bt;
+                        out.prim[ray] = prim;
+                        out.b1[ray]   = s.b1;
+                        out.b2[ray]   = s.b2;
+                    }
+                    ray = kMissPrim;
+                    break;
+                }
+            }
+    }
+    if (STATS) warpStats(tc, &ctr->statNodes, &ctr->statTris);
 }
 
 __global__ void kAliasSample(DomeView dome, const float2* __restrict__ u, float* dir, float* pdf, float* val, uint32_t n)
@@ -1717,11 +1754,11 @@ cl_status Integrator::init(std::string* err)
     CL_CUDA(cudaMallocHost((void**)&hostCount_, 64), err);
     int b = 0;
     // Occupancy at the deepest supported stack (the launches use less).
-    CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTraceClosest<false, true>, kTraceBlock,
+    CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTraceClosest<false, false>, kTraceBlock,
                                                           traceStackBytes(kStackDepth)),
             err);
     traceBlocks_ = std::max(1, b) * numSMs_;
-    CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTraceClosest<false, true, true>, kTraceBlock,
+    CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTraceClosest<false, true>, kTraceBlock,
                                                           traceStackBytes(kStackDepth)),
             err);
     traceBlocksTwo_ = std::max(1, b) * numSMs_;
@@ -2523,14 +2560,20 @@ cl_status Integrator::clearFilm(std::string* err)
     return CL_OK;
 }
 
-cl_status Integrator::ensureQueues(std::string* err)
+cl_status Integrator::checkPathSlots(std::string* err) const
 {
-    uint32_t slots = cfg_.path_slots ? cfg_.path_slots : (1u << 21);
-    if (slots > kMaxPathSlots)
+    if (cfg_.path_slots > kMaxPathSlots)
     {
-        *err = "path_slots " + std::to_string(slots) + " above the maximum " + std::to_string(kMaxPathSlots);
+        *err = "path_slots " + std::to_string(cfg_.path_slots) + " above the maximum " + std::to_string(kMaxPathSlots);
         return CL_ERR_INVALID_ARG;
     }
+    return CL_OK;
+}
+
+cl_status Integrator::ensureQueues(std::string* err)
+{
+    CL_TRY(checkPathSlots(err));
+    uint32_t slots = cfg_.path_slots ? cfg_.path_slots : (1u << 21);
     if (slots == slots_ && rqO_[0].p) return CL_OK;
     size_t s = slots;
     for (int q = 0; q < 2; ++q)
@@ -2660,8 +2703,8 @@ cl_status Integrator::launchWave(int cur, bool profile, std::string* err)
     if (profile) CL_CUDA(cudaEventRecord(evS_[0], stream_), err);
     {
         const size_t sb = traceStackBytes(P.sc.bvh.stackDepth);
-        auto         k  = st ? (twoLevel_ ? kTraceClosest<true, true, true> : kTraceClosest<true, true, false>)
-                             : (twoLevel_ ? kTraceClosest<false, true, true> : kTraceClosest<false, true, false>);
+        auto         k  = st ? (twoLevel_ ? kTraceClosest<true, true> : kTraceClosest<true, false>)
+                             : (twoLevel_ ? kTraceClosest<false, true> : kTraceClosest<false, false>);
         k<<<tBlocks(), kTraceBlock, sb, stream_>>>(P.sc.bvh, P.q.rqO[cur], P.q.rqD[cur], &c->rayCount[cur],
                                                       &c->fetchTrace, P.q.hit, c, classifyView());
         if (profile) CL_CUDA(cudaEventRecord(evS_[5], stream_), err);
@@ -3311,6 +3354,29 @@ cl_status Integrator::getBvh(void* nodes, size_t nodeBytes, void* tris, size_t t
     return CL_OK;
 }
 
+// Uploads rays [base, base + m) of a query, launches it and fetches its
+// counters.  The buffers hold kQueryChunk rays at most and are kept.
+cl_status Integrator::launchQuery(const float* rays, uint32_t m, bool any, bool stats, QueryOut* out, std::string* err)
+{
+    if (queryIn_.bytes < size_t(m) * 32) CL_TRY(queryIn_.alloc(size_t(m) * 32, err));
+    if (queryOut_.bytes < size_t(m) * 16) CL_TRY(queryOut_.alloc(size_t(m) * 16, err));
+    float* f = queryOut_.f();
+    *out     = stats ? QueryOut{}
+                     : QueryOut{f, reinterpret_cast<uint32_t*>(f + m), f + 2 * size_t(m), f + 3 * size_t(m),
+                                queryOut_.as<uint8_t>()};
+    CL_CUDA(cudaMemcpyAsync(queryIn_.p, rays, size_t(m) * 32, cudaMemcpyHostToDevice, stream_), err);
+    CL_CUDA(cudaMemsetAsync(ctr_.p, 0, sizeof(Counters), stream_), err);
+    using Fn         = void (*)(BvhView, const float4*, uint32_t, QueryOut, Counters*);
+    const Fn table[3][2] = {{kTraceQuery<false, false, false>, kTraceQuery<false, false, true>},
+                            {kTraceQuery<true, false, false>, kTraceQuery<true, false, true>},
+                            {kTraceQuery<false, true, false>, kTraceQuery<false, true, true>}};
+    const BvhView v = bvhView();
+    table[any ? 1 : stats ? 2 : 0][twoLevel_]<<<tBlocks(), kTraceBlock, traceStackBytes(v.stackDepth), stream_>>>(
+        v, queryIn_.as<const float4>(), m, *out, ctr_.as<Counters>());
+    CL_CUDA(cudaGetLastError(), err);
+    return CL_OK;
+}
+
 cl_status Integrator::traceRays(const float* rays, uint32_t n, float* t, uint32_t* prim, float* b1, float* b2,
                                 std::string* err)
 {
@@ -3325,29 +3391,16 @@ cl_status Integrator::traceRays(const float* rays, uint32_t n, float* t, uint32_
         *err = "null argument";
         return CL_ERR_INVALID_ARG;
     }
-    CL_TRY(ensureQueues(err));
-    std::vector<float4> o(slots_), d(slots_), h(slots_);
-    Counters* dc = ctr_.as<Counters>();
-    for (uint32_t base = 0; base < n; base += slots_)
+    CL_TRY(checkPathSlots(err));
+    for (uint32_t base = 0, m; base < n; base += m)
     {
-        uint32_t m = std::min(slots_, n - base);
-        for (uint32_t i = 0; i < m; ++i)
-        {
-            const float* r = rays + 8 * size_t(base + i);
-            o[i]           = make_float4(r[0], r[1], r[2], r[3]);
-            d[i]           = make_float4(r[4], r[5], r[6], r[7]);
-        }
-        CL_CUDA(cudaMemcpyAsync(rqO_[0].p, o.data(), m * 16, cudaMemcpyHostToDevice, stream_), err);
-        CL_CUDA(cudaMemcpyAsync(rqD_[0].p, d.data(), m * 16, cudaMemcpyHostToDevice, stream_), err);
-        Counters c0{};
-        c0.rayCount[0] = m;
-        CL_CUDA(cudaMemcpyAsync(ctr_.p, &c0, sizeof(c0), cudaMemcpyHostToDevice, stream_), err);
-        (twoLevel_ ? kTraceClosest<false, false, true> : kTraceClosest<false, false, false>)
-            <<<tBlocks(), kTraceBlock, traceStackBytes(bvhView().stackDepth), stream_>>>(
-                bvhView(), rqO_[0].as<float4>(), rqD_[0].as<float4>(), &dc->rayCount[0], &dc->fetchTrace,
-                hit_.as<float4>(), dc, ClassifyView{});
-        CL_CUDA(cudaGetLastError(), err);
-        CL_CUDA(cudaMemcpyAsync(h.data(), hit_.p, m * 16, cudaMemcpyDeviceToHost, stream_), err);
+        m = std::min(kQueryChunk, n - base);
+        QueryOut o;
+        CL_TRY(launchQuery(rays + 8 * size_t(base), m, false, false, &o, err));
+        CL_CUDA(cudaMemcpyAsync(t + base, o.t, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
+        CL_CUDA(cudaMemcpyAsync(prim + base, o.prim, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
+        CL_CUDA(cudaMemcpyAsync(b1 + base, o.b1, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
+        CL_CUDA(cudaMemcpyAsync(b2 + base, o.b2, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
         Counters ch;
         CL_CUDA(cudaMemcpyAsync(&ch, ctr_.p, sizeof(ch), cudaMemcpyDeviceToHost, stream_), err);
         CL_CUDA(cudaStreamSynchronize(stream_), err);
@@ -3355,15 +3408,6 @@ cl_status Integrator::traceRays(const float* rays, uint32_t n, float* t, uint32_
         {
             *err = "traversal error flags " + std::to_string(ch.error);
             return CL_ERR_STATE;
-        }
-        for (uint32_t i = 0; i < m; ++i)
-        {
-            t[base + i]    = h[i].x;
-            uint32_t pb;
-            memcpy(&pb, &h[i].y, 4);
-            prim[base + i] = pb;
-            b1[base + i]   = h[i].z;
-            b2[base + i]   = h[i].w;
         }
     }
     return CL_OK;
@@ -3382,27 +3426,14 @@ cl_status Integrator::occludedRays(const float* rays, uint32_t n, uint8_t* occ, 
         *err = "null argument";
         return CL_ERR_INVALID_ARG;
     }
-    DevBuf o, d, r;
-    CL_TRY(o.alloc(size_t(n) * 16, err));
-    CL_TRY(d.alloc(size_t(n) * 16, err));
-    CL_TRY(r.alloc(n, err));
-    std::vector<float4> ho(n), hd(n);
-    for (uint32_t i = 0; i < n; ++i)
+    for (uint32_t base = 0, m; base < n; base += m)
     {
-        const float* q = rays + 8 * size_t(i);
-        ho[i]          = make_float4(q[0], q[1], q[2], q[3]);
-        hd[i]          = make_float4(q[4], q[5], q[6], q[7]);
+        m = std::min(kQueryChunk, n - base);
+        QueryOut o;
+        CL_TRY(launchQuery(rays + 8 * size_t(base), m, true, false, &o, err));
+        CL_CUDA(cudaMemcpyAsync(occ + base, o.occ, m, cudaMemcpyDeviceToHost, stream_), err);
+        CL_CUDA(cudaStreamSynchronize(stream_), err);
     }
-    CL_CUDA(cudaMemcpyAsync(o.p, ho.data(), size_t(n) * 16, cudaMemcpyHostToDevice, stream_), err);
-    CL_CUDA(cudaMemcpyAsync(d.p, hd.data(), size_t(n) * 16, cudaMemcpyHostToDevice, stream_), err);
-    CL_CUDA(cudaMemsetAsync(ctr_.p, 0, sizeof(Counters), stream_), err);
-    (twoLevel_ ? kOccluded<true> : kOccluded<false>)
-        <<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, traceStackBytes(bvhView().stackDepth), stream_>>>(
-        bvhView(), o.as<float4>(), d.as<float4>(), n,
-        r.as<uint8_t>(), &ctr_.as<Counters>()->error);
-    CL_CUDA(cudaGetLastError(), err);
-    CL_CUDA(cudaMemcpyAsync(occ, r.p, n, cudaMemcpyDeviceToHost, stream_), err);
-    CL_CUDA(cudaStreamSynchronize(stream_), err);
     return CL_OK;
 }
 
@@ -3418,29 +3449,13 @@ cl_status Integrator::traceStats(const float* rays, uint32_t n, uint64_t* nodes,
         *err = "null argument";
         return CL_ERR_INVALID_ARG;
     }
-    CL_TRY(ensureQueues(err));
-    Counters* dc = ctr_.as<Counters>();
-    uint64_t  an = 0, at = 0;
-    std::vector<float4> o(slots_), d(slots_);
-    for (uint32_t base = 0; base < n; base += slots_)
+    CL_TRY(checkPathSlots(err));
+    uint64_t an = 0, at = 0;
+    for (uint32_t base = 0, m; base < n; base += m)
     {
-        uint32_t m = std::min(slots_, n - base);
-        for (uint32_t i = 0; i < m; ++i)
-        {
-            const float* r = rays + 8 * size_t(base + i);
-            o[i]           = make_float4(r[0], r[1], r[2], r[3]);
-            d[i]           = make_float4(r[4], r[5], r[6], r[7]);
-        }
-        CL_CUDA(cudaMemcpyAsync(rqO_[0].p, o.data(), m * 16, cudaMemcpyHostToDevice, stream_), err);
-        CL_CUDA(cudaMemcpyAsync(rqD_[0].p, d.data(), m * 16, cudaMemcpyHostToDevice, stream_), err);
-        Counters c0{};
-        c0.rayCount[0] = m;
-        CL_CUDA(cudaMemcpyAsync(ctr_.p, &c0, sizeof(c0), cudaMemcpyHostToDevice, stream_), err);
-        (twoLevel_ ? kTraceClosest<true, false, true> : kTraceClosest<true, false, false>)
-            <<<tBlocks(), kTraceBlock, traceStackBytes(bvhView().stackDepth), stream_>>>(
-                bvhView(), rqO_[0].as<float4>(), rqD_[0].as<float4>(), &dc->rayCount[0], &dc->fetchTrace,
-                hit_.as<float4>(), dc, ClassifyView{});
-        CL_CUDA(cudaGetLastError(), err);
+        m = std::min(kQueryChunk, n - base);
+        QueryOut o;
+        CL_TRY(launchQuery(rays + 8 * size_t(base), m, false, true, &o, err));
         Counters ch;
         CL_CUDA(cudaMemcpyAsync(&ch, ctr_.p, sizeof(ch), cudaMemcpyDeviceToHost, stream_), err);
         CL_CUDA(cudaStreamSynchronize(stream_), err);
@@ -3503,7 +3518,7 @@ cl_status Integrator::guideProbe(uint32_t cap, float* rows, uint32_t* count, std
     P.g.probeCap   = cap;
     Counters* c    = ctr_.as<Counters>();
     kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(P, init);
-    (twoLevel_ ? kTraceClosest<false, true, true> : kTraceClosest<false, true, false>)
+    (twoLevel_ ? kTraceClosest<false, true> : kTraceClosest<false, false>)
         <<<tBlocks(), kTraceBlock, traceStackBytes(P.sc.bvh.stackDepth), stream_>>>(
             P.sc.bvh, P.q.rqO[0], P.q.rqD[0], &c->rayCount[0], &c->fetchTrace, P.q.hit, c, classifyView());
     (twoLevel_ ? kClassifyHits<true> : kClassifyHits<false>)<<<numSMs_ * 8, kClassifyThreads, 0, stream_>>>(

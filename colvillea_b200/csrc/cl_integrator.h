@@ -13,6 +13,7 @@
 namespace clb
 {
 struct ClassifyView;
+struct QueryOut;
 constexpr int      kMaxEmitters = 8;
 constexpr uint32_t kLastFlag    = 0x80000000u; // shadow entry: path ends after this shadow query
 
@@ -202,7 +203,9 @@ private:
     cl_status trainCache(std::string* err);
     cl_status ensureFilm(std::string* err);
     cl_status resolveFilm(std::string* err);
+    cl_status checkPathSlots(std::string* err) const;
     cl_status ensureQueues(std::string* err);
+    cl_status launchQuery(const float* rays, uint32_t m, bool any, bool stats, QueryOut* out, std::string* err);
     cl_status clearFilm(std::string* err);
     cl_status captureGraph(std::string* err);
     cl_status launchWave(int cur, bool profile, std::string* err);
@@ -270,6 +273,9 @@ private:
 
     // Film and wavefront state.
     DevBuf film_, film64_;
+    // Ray queries: rows of 8 floats in, 4 values (or a byte) per ray out.
+    static constexpr uint32_t kQueryChunk = 1u << 21;
+    DevBuf                    queryIn_, queryOut_;
     // Film readback: mean radiance staged on the device, copied out on its own
     // stream so that a copy overlaps the next render.
     DevBuf       resolve_;
