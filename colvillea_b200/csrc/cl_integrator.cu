@@ -1802,94 +1802,8 @@ cl_status Integrator::buildMeshes(const cl_mesh_desc* meshes, uint32_t n, std::s
         *err = "meshes is null";
         return CL_ERR_INVALID_ARG;
     }
-    std::vector<HostMesh> out(n);
-    for (uint32_t m = 0; m < n; ++m)
-    {
-        const cl_mesh_desc& d = meshes[m];
-        if (!d.positions || !d.indices || !d.tangents || d.num_vertices == 0 || d.num_triangles == 0)
-        {
-            *err = "mesh " + std::to_string(m) + ": positions, tangents and indices are required";
-            return CL_ERR_INVALID_ARG;
-        }
-        HostMesh& h = out[m];
-        size_t    nv = d.num_vertices, nt = d.num_triangles;
-        h.pos.assign(d.positions, d.positions + 3 * nv);
-        h.tan.assign(d.tangents, d.tangents + 3 * nv);
-        h.hasN = d.normals != nullptr;
-        if (h.hasN) h.nrm.assign(d.normals, d.normals + 3 * nv);
-        h.hasUV = d.uvs != nullptr;
-        if (h.hasUV) h.uv.assign(d.uvs, d.uvs + 2 * nv);
-        h.idx.assign(d.indices, d.indices + 3 * nt);
-        for (uint32_t v : h.idx)
-            if (v >= d.num_vertices)
-            {
-                *err = "mesh " + std::to_string(m) + ": vertex index out of range";
-                return CL_ERR_INVALID_ARG;
-            }
-    }
-    meshes_.swap(out);
+    CL_TRY(meshes_.build(meshes, n, stream_, err));
     sceneBuilt_ = false;
-    return CL_OK;
-}
-
-// World-space vertices of one instance: 12 floats per vertex {p.xyz, n.xyz,
-// t.xyz, u, v, flags}; normals by the inverse transpose of the linear part.
-cl_status Integrator::flattenInstance(const HostMesh& m, const float* M, uint32_t i, float* out, std::string* err)
-{
-    bool ident = M[0] == 1 && M[1] == 0 && M[2] == 0 && M[3] == 0 && M[4] == 0 && M[5] == 1 && M[6] == 0 &&
-                 M[7] == 0 && M[8] == 0 && M[9] == 0 && M[10] == 1 && M[11] == 0;
-    double a = M[0], b = M[1], c = M[2], d = M[4], e = M[5], f = M[6], g = M[8], h = M[9], k = M[10];
-    double det = a * (e * k - f * h) - b * (d * k - f * g) + c * (d * h - e * g);
-    if (!ident && std::fabs(det) < 1e-30)
-    {
-        *err = "instance " + std::to_string(i) + ": singular transform";
-        return CL_ERR_INVALID_ARG;
-    }
-    // Inverse transpose of the linear part, row-major: IT[3 r + c] = inverse[c][r].
-    double IT[9] = {(e * k - f * h) / det, -(d * k - f * g) / det, (d * h - e * g) / det,
-                    -(b * k - c * h) / det, (a * k - c * g) / det,  -(a * h - b * g) / det,
-                    (b * f - c * e) / det,  -(a * f - c * d) / det, (a * e - b * d) / det};
-    size_t   mv    = m.pos.size() / 3;
-    uint32_t flags = (m.hasN ? 1u : 0u) | (m.hasUV ? 2u : 0u);
-    for (size_t v = 0; v < mv; ++v)
-    {
-        float p[3], nn[3] = {0, 0, 0}, t[3], uv[2] = {0, 0};
-        for (int q = 0; q < 3; ++q)
-        {
-            p[q] = m.pos[3 * v + q];
-            t[q] = m.tan[3 * v + q];
-            if (m.hasN) nn[q] = m.nrm[3 * v + q];
-        }
-        if (m.hasUV)
-        {
-            uv[0] = m.uv[2 * v];
-            uv[1] = m.uv[2 * v + 1];
-        }
-        if (!ident)
-        {
-            float P2[3], T2[3], N2[3];
-            for (int r = 0; r < 3; ++r)
-            {
-                P2[r] = float(double(M[4 * r]) * p[0] + double(M[4 * r + 1]) * p[1] + double(M[4 * r + 2]) * p[2] +
-                              double(M[4 * r + 3]));
-                T2[r] = float(double(M[4 * r]) * t[0] + double(M[4 * r + 1]) * t[1] + double(M[4 * r + 2]) * t[2]);
-                // n' = (inverse of the linear part)^T n
-                N2[r] = float(IT[3 * r] * nn[0] + IT[3 * r + 1] * nn[1] + IT[3 * r + 2] * nn[2]);
-            }
-            for (int q = 0; q < 3; ++q)
-            {
-                p[q]  = P2[q];
-                t[q]  = T2[q];
-                nn[q] = N2[q];
-            }
-        }
-        float* o = out + v * 12;
-        o[0] = p[0]; o[1] = p[1]; o[2] = p[2]; o[3] = nn[0];
-        o[4] = nn[1]; o[5] = nn[2]; o[6] = t[0]; o[7] = t[1];
-        float ff;
-        memcpy(&ff, &flags, 4);
-        o[8] = t[2]; o[9] = uv[0]; o[10] = uv[1]; o[11] = ff;
-    }
     return CL_OK;
 }
 
@@ -1908,8 +1822,8 @@ cl_status Integrator::buildInstances(const cl_instance_desc* inst, uint32_t n, s
             *err = "instance " + std::to_string(i) + ": mesh_id out of range";
             return CL_ERR_INVALID_ARG;
         }
-        nv += meshes_[inst[i].mesh_id].pos.size() / 3;
-        nt += meshes_[inst[i].mesh_id].idx.size() / 3;
+        nv += meshes_[inst[i].mesh_id].nv;
+        nt += meshes_[inst[i].mesh_id].nt;
     }
     if (nt >= 0x7fffffffu || nv >= 0xffffffffu)
     {
@@ -1922,52 +1836,28 @@ cl_status Integrator::buildInstances(const cl_instance_desc* inst, uint32_t n, s
     instDev_.release();
     // Flatten instances into world space (the reference's TLAS has no
     // transforms, optix.cu:115; identity transforms are copied exactly).
-    std::vector<float>    vtx(nv * 12);
-    std::vector<uint32_t> tidx(nt * 4);
-    std::vector<float>    tri9(nt * 9);
-    std::vector<uint32_t> vtxOff(n);
-    size_t vo = 0, to = 0;
+    std::vector<FlatInst> flat(n);
+    size_t                vo = 0, to = 0;
     for (uint32_t i = 0; i < n; ++i)
     {
-        const HostMesh& m = meshes_[inst[i].mesh_id];
-        CL_TRY(flattenInstance(m, inst[i].transform, i, &vtx[vo * 12], err));
-        vtxOff[i] = uint32_t(vo);
-        size_t mv = m.pos.size() / 3;
-        size_t mt = m.idx.size() / 3;
-        for (size_t t = 0; t < mt; ++t)
-        {
-            uint32_t* o = &tidx[(to + t) * 4];
-            for (int q = 0; q < 3; ++q)
-            {
-                uint32_t gv = uint32_t(vo + m.idx[3 * t + q]);
-                o[q]        = gv;
-                for (int c2 = 0; c2 < 3; ++c2) tri9[(to + t) * 9 + 3 * q + c2] = vtx[size_t(gv) * 12 + c2];
-            }
-            o[3] = inst[i].material_index;
-        }
-        vo += mv;
-        to += mt;
+        CL_TRY(meshes_.flatInst(inst[i].mesh_id, inst[i].transform, uint32_t(vo), uint32_t(to), inst[i].material_index,
+                                "instance " + std::to_string(i), &flat[i], err));
+        vo += flat[i].nv;
+        to += flat[i].nt;
     }
-    CL_TRY(vtx_.alloc(vtx.size() * 4, err));
-    CL_TRY(triIdx_.alloc(tidx.size() * 4, err));
-    CL_TRY(triPos_.alloc(tri9.size() * 4, err));
-    CL_CUDA(cudaMemcpyAsync(vtx_.p, vtx.data(), vtx.size() * 4, cudaMemcpyHostToDevice, stream_), err);
-    CL_CUDA(cudaMemcpyAsync(triIdx_.p, tidx.data(), tidx.size() * 4, cudaMemcpyHostToDevice, stream_), err);
-    CL_CUDA(cudaMemcpyAsync(triPos_.p, tri9.data(), tri9.size() * 4, cudaMemcpyHostToDevice, stream_), err);
+    sceneBuilt_ = false; // until the new one is complete
+    flat_.swap(flat);
+    CL_TRY(uploadFlat(err));
+    CL_TRY(vtx_.alloc(nv * 48, err));
+    CL_TRY(triIdx_.alloc(nt * 16, err));
+    CL_TRY(triPos_.alloc(nt * 36, err));
+    CL_TRY(meshes_.flattenVertices(flatDev_, flat_.data(), 0, n, vtx_.p, stream_, err));
+    CL_TRY(meshes_.flattenTriangles(flatDev_, flat_.data(), n, triIdx_.p, stream_, err));
+    CL_TRY(gatherTrianglePositions(vtx_.p, triIdx_.p, uint32_t(nt), triPos_.f(), stream_, err));
     // Scene box for the guiding network's position input (uniform scale).
-    {
-        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (size_t v = 0; v < nv; ++v)
-            for (int q = 0; q < 3; ++q)
-            {
-                lo[q] = std::min(lo[q], vtx[v * 12 + q]);
-                hi[q] = std::max(hi[q], vtx[v * 12 + q]);
-            }
-        float ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
-        ext       = std::max(ext, 1e-6f) * 1.002f;
-        for (int q = 0; q < 3; ++q) boxMin_[q] = lo[q] - 0.001f * ext;
-        boxScale_ = 1.0f / ext;
-    }
+    float lo[3], hi[3];
+    CL_TRY(vertexBounds(vtx_.p, nv, stream_, lo, hi, err));
+    setSceneBox(lo, hi);
     const auto   w0 = std::chrono::steady_clock::now();
     const double a0 = allocMs();
     CL_CUDA(cudaEventRecord(evA_, stream_), err);
@@ -1984,7 +1874,6 @@ cl_status Integrator::buildInstances(const cl_instance_desc* inst, uint32_t n, s
     sceneBuilt_ = true;
     graphValid_ = false;
     inst_.assign(inst, inst + n);
-    instVtxOff_.swap(vtxOff);
     // Material indices are checked at render time against the material count.
     maxMaterialIndex_ = 0;
     for (uint32_t i = 0; i < n; ++i) maxMaterialIndex_ = std::max(maxMaterialIndex_, inst[i].material_index);
@@ -1999,33 +1888,33 @@ cl_status Integrator::buildInstances(const cl_instance_desc* inst, uint32_t n, s
 // (v0 = v2 = min, v1 = max), so the same device builder makes both levels.
 static const float kIdentity12[12] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0};
 
-cl_status Integrator::uploadMeshPool(uint32_t meshId, std::string* err)
+cl_status Integrator::uploadFlat(std::string* err)
 {
-    const HostMesh&    m  = meshes_[meshId];
-    const size_t       mv = m.pos.size() / 3;
-    std::vector<float> buf(mv * 12);
-    CL_TRY(flattenInstance(m, kIdentity12, meshId, buf.data(), err));
-    CL_CUDA(cudaMemcpyAsync(vtx_.f() + size_t(meshVtxBase_[meshId]) * 12, buf.data(), buf.size() * 4,
-                            cudaMemcpyHostToDevice, stream_),
-            err);
+    const size_t b = flat_.size() * sizeof(FlatInst);
+    if (flatDev_.bytes < b) CL_TRY(flatDev_.alloc(b, err));
+    CL_CUDA(cudaMemcpyAsync(flatDev_.p, flat_.data(), b, cudaMemcpyHostToDevice, stream_), err);
     return CL_OK;
+}
+
+// Scene box for the networks' position input (uniform scale).
+void Integrator::setSceneBox(const float lo[3], const float hi[3])
+{
+    float ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
+    ext       = std::max(ext, 1e-6f) * 1.002f;
+    for (int q = 0; q < 3; ++q) boxMin_[q] = lo[q] - 0.001f * ext;
+    boxScale_ = 1.0f / ext;
 }
 
 cl_status Integrator::buildBlas(uint32_t meshId, BuildArena* arena, cudaStream_t st, std::string* err)
 {
-    const HostMesh&    m  = meshes_[meshId];
-    const size_t       mt = m.idx.size() / 3;
-    std::vector<float> tri9(mt * 9);
-    for (size_t t = 0; t < mt; ++t)
-        for (int q = 0; q < 3; ++q)
-            for (int c = 0; c < 3; ++c) tri9[t * 9 + 3 * q + c] = m.pos[3 * size_t(m.idx[3 * t + q]) + c];
-    BuildArena  local;
-    BuildArena& mem = arena ? *arena : local;
-    ScratchBuf  d;
-    CL_TRY(mem.input(d, tri9.size() * 4, err));
-    CL_CUDA(cudaMemcpyAsync(d.p, tri9.data(), tri9.size() * 4, cudaMemcpyHostToDevice, st), err);
+    const MeshInfo& m = meshes_[meshId];
+    BuildArena      local;
+    BuildArena&     mem = arena ? *arena : local;
+    ScratchBuf      d;
+    CL_TRY(mem.input(d, size_t(m.nt) * 36, err));
+    CL_TRY(gatherTrianglePositions(vtx_.p, triIdx_.as<uint4>() + m.triBase, m.nt, d.f(), st, err));
     if (!blas_[meshId]) blas_[meshId].reset(new WideBvh());
-    return buildWideBvh(d.f(), uint32_t(mt), st, blas_[meshId].get(), err, &mem);
+    return buildWideBvh(d.f(), m.nt, st, blas_[meshId].get(), err, &mem);
 }
 
 // The trees of the instanced meshes.  They are independent, and each build
@@ -2092,23 +1981,13 @@ cl_status Integrator::buildBlasAll(const std::vector<uint32_t>& meshes, std::str
     return CL_OK;
 }
 
-// World box of instance i (every vertex mapped, in double), widened by a
-// relative 1e-6 so that FP32 rounding of the object-space traversal cannot
-// fall outside it.
-void Integrator::instanceBox(uint32_t i, float* lo, float* hi) const
+// World box of an instance from the bounds of its mapped vertices (b: 3
+// minima, 3 maxima, in double), widened by a relative 1e-6 so that FP32
+// rounding of the object-space traversal cannot fall outside it.
+static void instanceBox(const double* b, float* lo, float* hi)
 {
-    const HostMesh& m  = meshes_[inst_[i].mesh_id];
-    const float*    M  = inst_[i].transform;
-    double          l[3] = {1e300, 1e300, 1e300}, h[3] = {-1e300, -1e300, -1e300};
-    for (size_t v = 0; v < m.pos.size() / 3; ++v)
-        for (int r = 0; r < 3; ++r)
-        {
-            double x = double(M[4 * r]) * m.pos[3 * v] + double(M[4 * r + 1]) * m.pos[3 * v + 1] +
-                       double(M[4 * r + 2]) * m.pos[3 * v + 2] + double(M[4 * r + 3]);
-            l[r] = std::min(l[r], x);
-            h[r] = std::max(h[r], x);
-        }
-    double ext = std::max(h[0] - l[0], std::max(h[1] - l[1], h[2] - l[2]));
+    const double *l = b, *h = b + 3;
+    double        ext = std::max(h[0] - l[0], std::max(h[1] - l[1], h[2] - l[2]));
     for (int r = 0; r < 3; ++r)
     {
         double pad = 1e-6 * ext + 1e-6 * std::max(std::fabs(l[r]), std::fabs(h[r])) + 1e-30;
@@ -2124,10 +2003,13 @@ cl_status Integrator::buildTopLevel(BuildArena* arena, std::string* err)
     const uint32_t     n = uint32_t(inst_.size());
     std::vector<float> tri9(size_t(n) * 9);
     float              slo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, shi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    // flatDev_ holds the meshes' identity copies, then the instances.
+    std::vector<double> boxes;
+    CL_TRY(meshes_.instanceBoxes(flatDev_, uint32_t(meshes_.size()), n, &boxes, stream_, err));
     for (uint32_t i = 0; i < n; ++i)
     {
         float lo[3], hi[3];
-        instanceBox(i, lo, hi);
+        instanceBox(&boxes[6 * size_t(i)], lo, hi);
         for (int c = 0; c < 3; ++c)
         {
             tri9[size_t(i) * 9 + c]     = lo[c];
@@ -2137,11 +2019,7 @@ cl_status Integrator::buildTopLevel(BuildArena* arena, std::string* err)
             shi[c]                      = std::max(shi[c], hi[c]);
         }
     }
-    // Scene box for the networks' position input (uniform scale).
-    float ext = std::max(shi[0] - slo[0], std::max(shi[1] - slo[1], shi[2] - slo[2]));
-    ext       = std::max(ext, 1e-6f) * 1.002f;
-    for (int q = 0; q < 3; ++q) boxMin_[q] = slo[q] - 0.001f * ext;
-    boxScale_ = 1.0f / ext;
+    setSceneBox(slo, shi);
     BuildArena  local;
     BuildArena& mem = arena ? *arena : local;
     ScratchBuf  d;
@@ -2194,10 +2072,10 @@ cl_status Integrator::uploadInstances(std::string* err)
         r.nodes    = blas_[mid]->nodes.as<const uint4>();
         r.tris     = blas_[mid]->tris.as<const float4>();
         r.primBase = primBase;
-        r.triBase  = meshTriBase_[mid];
+        r.triBase  = meshes_[mid].triBase;
         r.material = inst_[i].material_index;
         r.flags    = det < 0.0 ? 1u : 0u;
-        primBase += uint32_t(meshes_[mid].idx.size() / 3);
+        primBase += meshes_[mid].nt;
     }
     CL_TRY(instDev_.alloc(size_t(n) * sizeof(InstDev), err));
     CL_CUDA(cudaMemcpyAsync(instDev_.p, h.data(), size_t(n) * sizeof(InstDev), cudaMemcpyHostToDevice, stream_), err);
@@ -2209,34 +2087,30 @@ cl_status Integrator::buildTwoLevel(const cl_instance_desc* inst, uint32_t n, st
 {
     // Pools: every mesh's object-space vertices and triangles.
     const uint32_t nm = uint32_t(meshes_.size());
-    meshVtxBase_.assign(nm, 0u);
-    meshTriBase_.assign(nm, 0u);
-    size_t nv = 0, nt = 0;
+    size_t         nv = 0, nt = 0;
+    // Copies of the meshes in object space, then the instances (for their boxes).
+    std::vector<FlatInst> flat(size_t(nm) + n);
     for (uint32_t m = 0; m < nm; ++m)
     {
-        meshVtxBase_[m] = uint32_t(nv);
-        meshTriBase_[m] = uint32_t(nt);
-        nv += meshes_[m].pos.size() / 3;
-        nt += meshes_[m].idx.size() / 3;
+        const MeshInfo& i = meshes_[m];
+        CL_TRY(meshes_.flatInst(m, kIdentity12, i.vtxBase, i.triBase, 0u, "mesh", &flat[m], err));
+        nv += i.nv;
+        nt += i.nt;
     }
-    std::vector<uint32_t> tidx(nt * 4);
-    for (uint32_t m = 0; m < nm; ++m)
-    {
-        const HostMesh& hm = meshes_[m];
-        for (size_t t = 0; t < hm.idx.size() / 3; ++t)
-        {
-            uint32_t* o = &tidx[(meshTriBase_[m] + t) * 4];
-            for (int q = 0; q < 3; ++q) o[q] = meshVtxBase_[m] + hm.idx[3 * t + q];
-            o[3] = 0u;
-        }
-    }
+    for (uint32_t i = 0; i < n; ++i)
+        CL_TRY(meshes_.flatInst(inst[i].mesh_id, inst[i].transform, 0u, 0u, 0u, "instance " + std::to_string(i),
+                                &flat[size_t(nm) + i], err));
+    sceneBuilt_ = false; // until the new one is complete
+    flat_.swap(flat);
     const auto   w0 = std::chrono::steady_clock::now();
     const double a0 = allocMs();
     CL_CUDA(cudaEventRecord(evA_, stream_), err);
     CL_TRY(vtx_.alloc(nv * 48, err));
     CL_TRY(triIdx_.alloc(nt * 16, err));
-    CL_CUDA(cudaMemcpyAsync(triIdx_.p, tidx.data(), tidx.size() * 4, cudaMemcpyHostToDevice, stream_), err);
-    for (uint32_t m = 0; m < nm; ++m) CL_TRY(uploadMeshPool(m, err));
+    CL_TRY(uploadFlat(err));
+    CL_TRY(meshes_.flattenVertices(flatDev_, flat_.data(), 0, nm, vtx_.p, stream_, err));
+    CL_TRY(meshes_.flattenTriangles(flatDev_, flat_.data(), nm, triIdx_.p, stream_, err));
+    CL_CUDA(cudaStreamSynchronize(stream_), err); // the trees are built on other streams
     std::vector<bool> used(nm, false);
     for (uint32_t i = 0; i < n; ++i) used[inst[i].mesh_id] = true;
     blas_.clear();
@@ -2257,7 +2131,6 @@ cl_status Integrator::buildTwoLevel(const cl_instance_desc* inst, uint32_t n, st
     twoLevel_   = true;
     sceneBuilt_ = true;
     graphValid_ = false;
-    instVtxOff_.clear();
     maxMaterialIndex_ = 0;
     for (uint32_t i = 0; i < n; ++i) maxMaterialIndex_ = std::max(maxMaterialIndex_, inst[i].material_index);
     return CL_OK;
@@ -2268,7 +2141,7 @@ cl_status Integrator::buildTwoLevel(const cl_instance_desc* inst, uint32_t n, st
 // top tree rebuilt over the instances' new boxes.
 cl_status Integrator::updateTwoLevel(uint32_t meshId, uint32_t mode, std::string* err)
 {
-    CL_TRY(uploadMeshPool(meshId, err));
+    CL_TRY(meshes_.flattenVertices(flatDev_, flat_.data(), meshId, 1, vtx_.p, stream_, err));
     float ms = 0.0f;
     msBvhRefit_ = 0.0f;
     CL_CUDA(cudaEventRecord(evA_, stream_), err);
@@ -2281,7 +2154,7 @@ cl_status Integrator::updateTwoLevel(uint32_t meshId, uint32_t mode, std::string
         }
         else
         {
-            CL_TRY(refitWideBvh(blas_[meshId].get(), vtx_.p, triIdx_.as<uint4>() + meshTriBase_[meshId], stream_, err));
+            CL_TRY(refitWideBvh(blas_[meshId].get(), vtx_.p, triIdx_.as<uint4>() + meshes_[meshId].triBase, stream_, err));
             ++refits_;
         }
     }
@@ -2308,10 +2181,10 @@ cl_status Integrator::updateMeshVertices(uint32_t meshId, const float* pos, cons
         *err = "mesh_id out of range";
         return CL_ERR_INVALID_ARG;
     }
-    HostMesh& m = meshes_[meshId];
-    if (!pos || size_t(count) * 3 != m.pos.size())
+    const uint32_t nv = meshes_[meshId].nv;
+    if (!pos || count != nv)
     {
-        *err = "positions are required, with the mesh's vertex count (" + std::to_string(m.pos.size() / 3) + ")";
+        *err = "positions are required, with the mesh's vertex count (" + std::to_string(nv) + ")";
         return CL_ERR_INVALID_ARG;
     }
     if (mode > CL_BVH_UPDATE_REBUILD)
@@ -2319,32 +2192,22 @@ cl_status Integrator::updateMeshVertices(uint32_t meshId, const float* pos, cons
         *err = "unknown BVH update mode";
         return CL_ERR_INVALID_ARG;
     }
-    for (size_t i = 0; i < size_t(count) * 3; ++i)
-        if (!std::isfinite(pos[i]))
-        {
-            *err = "vertex " + std::to_string(i / 3) + ": position is not finite";
-            return CL_ERR_INVALID_ARG;
-        }
-    m.pos.assign(pos, pos + size_t(count) * 3);
-    if (nrm)
+    const bool hadN = meshes_[meshId].hasN;
+    CL_TRY(meshes_.updateVertices(meshId, pos, nrm, tan, stream_, err));
+    if (meshes_[meshId].hasN != hadN)
     {
-        m.nrm.assign(nrm, nrm + size_t(count) * 3);
-        m.hasN = true;
+        // The mesh's copies have normals from now on.
+        const uint32_t src = meshes_[meshId].vtxBase;
+        for (FlatInst& f : flat_)
+            if (f.srcVtx == src) f.flags |= 1u;
+        CL_TRY(uploadFlat(err));
     }
-    if (tan) m.tan.assign(tan, tan + size_t(count) * 3);
     if (twoLevel_) return updateTwoLevel(meshId, mode, err);
 
     // Re-flatten the instances of this mesh into their vertex ranges.
-    std::vector<float> buf;
-    for (size_t i = 0; i < inst_.size(); ++i)
-    {
-        if (inst_[i].mesh_id != meshId) continue;
-        buf.resize(size_t(count) * 12);
-        CL_TRY(flattenInstance(m, inst_[i].transform, uint32_t(i), buf.data(), err));
-        CL_CUDA(cudaMemcpyAsync(vtx_.f() + size_t(instVtxOff_[i]) * 12, buf.data(), buf.size() * 4,
-                                cudaMemcpyHostToDevice, stream_),
-                err);
-    }
+    for (uint32_t i = 0; i < inst_.size(); ++i)
+        if (inst_[i].mesh_id == meshId)
+            CL_TRY(meshes_.flattenVertices(flatDev_, flat_.data(), i, 1, vtx_.p, stream_, err));
 
     // Device time of the refit and/or rebuild (the surface-area cost pass
     // and the vertex upload are not included).

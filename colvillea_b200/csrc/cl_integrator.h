@@ -3,6 +3,7 @@
 
 #include "cl_bvh.cuh"
 #include "cl_dome.h"
+#include "cl_geometry.h"
 #include "cl_guide.h"
 #include "cl_internal.h"
 #include "cl_texture.h"
@@ -225,32 +226,26 @@ private:
     int                tBlocks() const { return twoLevel_ ? traceBlocksTwo_ : traceBlocks_; }
     int                tailBlocks() const { return tailBlocks_[twoLevel_ ? 1 : 0]; }
 
-    // Meshes as given (host copies), flattened on instance build.
-    struct HostMesh
-    {
-        std::vector<float>    pos, nrm, tan, uv;
-        std::vector<uint32_t> idx;
-        bool                  hasN = false, hasUV = false;
-    };
-    std::vector<HostMesh> meshes_;
-    cl_status flattenInstance(const HostMesh& m, const float* M, uint32_t i, float* out, std::string* err);
-    std::vector<cl_instance_desc> inst_;       // as built
-    std::vector<uint32_t>         instVtxOff_; // first flattened vertex of each instance
+    MeshPool                      meshes_; // as given, on the device; flattened on instance build
+    std::vector<cl_instance_desc> inst_;   // as built
+    // Copies of the scene's vertex and triangle arrays: the instances
+    // (flattened scenes), or the meshes and then the instances (two-level).
+    std::vector<FlatInst> flat_;
+    DevBuf                flatDev_;
+    cl_status             uploadFlat(std::string* err);
+    void                  setSceneBox(const float lo[3], const float hi[3]);
     // Two-level scenes (CL_TWO_LEVEL): object-space pools, one tree per mesh,
     // the instance records; bvh_ is then the top tree over the instances.
     bool                   twoLevel_ = false;
     std::vector<std::unique_ptr<WideBvh>> blas_; // per mesh (null: not instanced)
-    std::vector<uint32_t>  meshVtxBase_, meshTriBase_;
     DevBuf                 instDev_;
     uint32_t               twoLevelStack_ = 0;
     cl_status buildTwoLevel(const cl_instance_desc* inst, uint32_t n, std::string* err);
-    cl_status uploadMeshPool(uint32_t meshId, std::string* err);
     cl_status buildBlas(uint32_t meshId, BuildArena* arena, cudaStream_t st, std::string* err);
     cl_status buildBlasAll(const std::vector<uint32_t>& meshes, std::string* err);
     cl_status buildTopLevel(BuildArena* arena, std::string* err);
     cl_status uploadInstances(std::string* err);
     cl_status updateTwoLevel(uint32_t meshId, uint32_t mode, std::string* err);
-    void      instanceBox(uint32_t i, float* lo, float* hi) const;
     // Refit policy (CL_BVH_UPDATE_AUTO): rebuild when the refitted tree's
     // surface-area cost exceeds this multiple of the cost after its build.
     static constexpr double kRefitSahLimit = 1.5;

@@ -30,6 +30,11 @@ struct DevBuf
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
+    void swap(DevBuf& o)
+    {
+        std::swap(p, o.p);
+        std::swap(bytes, o.bytes);
+    }
     void release()
     {
         if (p) cudaFree(p);
