@@ -2141,6 +2141,7 @@ cl_status Integrator::buildTwoLevel(const cl_instance_desc* inst, uint32_t n, st
 // top tree rebuilt over the instances' new boxes.
 cl_status Integrator::updateTwoLevel(uint32_t meshId, uint32_t mode, std::string* err)
 {
+    sceneBuilt_ = false; // until the trees are complete again
     CL_TRY(meshes_.flattenVertices(flatDev_, flat_.data(), meshId, 1, vtx_.p, stream_, err));
     float ms = 0.0f;
     msBvhRefit_ = 0.0f;
@@ -2165,6 +2166,7 @@ cl_status Integrator::updateTwoLevel(uint32_t meshId, uint32_t mode, std::string
     CL_CUDA(cudaEventElapsedTime(&ms, evA_, evB_), err);
     msBvhUpdate_ = ms;
     graphValid_  = false;
+    sceneBuilt_  = true;
     return resetIteration(err);
 }
 

@@ -12,6 +12,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace clb
@@ -81,58 +82,74 @@ struct DevBuf
         }                                                                                                              \
     } while (0)
 
+// Part of a larger allocation, with DevBuf's accessors; it owns nothing.
+struct ScratchBuf
+{
+    void*  p     = nullptr;
+    size_t bytes = 0;
+    float*    f() const { return static_cast<float*>(p); }
+    uint32_t* u() const { return static_cast<uint32_t*>(p); }
+    template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
+// Lays out one allocation (a cudaMalloc or cudaFree takes 0.3 ms whatever its
+// size): parts are taken at 256-byte boundaries, a rewind to a mark lets later
+// parts share the memory of dead ones, and bind() gives the parts their places
+// once the allocation of peak() bytes exists.
+class Carver
+{
+public:
+    void take(ScratchBuf& s, size_t bytes)
+    {
+        parts_.push_back({&s, off_});
+        s.bytes = bytes;
+        off_ += (bytes + 255) / 256 * 256;
+        peak_ = std::max(peak_, off_);
+    }
+    size_t mark() const { return off_; }
+    void   rewind(size_t m) { off_ = m; }
+    size_t peak() const { return peak_; }
+    void   bind(void* base) const
+    {
+        for (const auto& p : parts_) p.first->p = static_cast<char*>(base) + p.second;
+    }
+
+private:
+    std::vector<std::pair<ScratchBuf*, size_t>> parts_;
+    size_t                                      off_ = 0, peak_ = 0;
+};
+
 struct WideBvh
 {
-    DevBuf   nodes; // 5 uint4 per node
-    DevBuf   tris;  // 3 float4 per triangle, leaf order
-    DevBuf   exact; // refit: 6 floats per node, the unquantised box of its triangles
-    DevBuf   scene; // scene bounds (6 ordered ints, refit) and the SAH sum (double at byte 32)
+    DevBuf     mem;   // holds the four below
+    ScratchBuf nodes; // 5 uint4 per node
+    ScratchBuf tris;  // 3 float4 per triangle, leaf order
+    ScratchBuf exact; // refit: 6 floats per node, the unquantised box of its triangles
+    ScratchBuf scene; // scene bounds (6 ordered ints, refit) and the SAH sum (double at byte 32)
     // Nodes of tree level d are [levels[d], levels[d + 1]): the collapse
     // allocates each level's nodes in one launch.
     std::vector<uint32_t> levels;
     uint32_t numNodes = 0, depth = 0, numTris = 0, buildIterations = 0;
     void     release()
     {
-        nodes.release();
-        tris.release();
-        exact.release();
-        scene.release();
+        mem.release();
+        nodes = tris = exact = scene = ScratchBuf{};
         levels.clear();
         numNodes = depth = numTris = 0;
     }
 };
 
-// A builder temporary: device memory taken from a build arena, with DevBuf's
-// accessors; it owns nothing (release() is a no-op).
-struct ScratchBuf
-{
-    void*  p     = nullptr;
-    size_t bytes = 0;
-    void      release() {}
-    float*    f() const { return static_cast<float*>(p); }
-    uint32_t* u() const { return static_cast<uint32_t*>(p); }
-    template <class T> T* as() const { return static_cast<T*>(p); }
-};
-
-// Grow-only device memory for the builder's temporaries: the k-th temporary of
-// a build reuses the k-th block of the previous build that shared the arena
-// (growing it when too small), so a sequence of builds (one per mesh of a
-// two-level scene) allocates, and frees - a synchronising cudaFree - once.
+// Grow-only device memory for a build's temporaries and for the device copy of
+// its input, reused by the builds that share the arena (one per mesh of a
+// two-level scene).
 class BuildArena
 {
 public:
-    void      reset() { used_ = 0; }
-    cl_status take(ScratchBuf& s, size_t bytes, std::string* err)
+    cl_status reserve(size_t bytes, std::string* err)
     {
-        if (used_ == blocks_.size()) blocks_.emplace_back(new DevBuf());
-        DevBuf& b = *blocks_[used_++];
-        if (b.bytes < bytes) CL_TRY(b.alloc(bytes, err));
-        s.p     = b.p;
-        s.bytes = bytes;
-        return CL_OK;
+        return mem_.bytes < bytes ? mem_.alloc(bytes, err) : CL_OK;
     }
-    // Device copy of a build's input, kept apart from the temporaries (which
-    // reset() recycles): one block that grows and is reused by the next build.
+    void*     base() const { return mem_.p; }
     cl_status input(ScratchBuf& s, size_t bytes, std::string* err)
     {
         if (input_.bytes < bytes) CL_TRY(input_.alloc(bytes, err));
@@ -142,9 +159,7 @@ public:
     }
 
 private:
-    std::vector<std::unique_ptr<DevBuf>> blocks_;
-    size_t                               used_ = 0;
-    DevBuf                               input_;
+    DevBuf mem_, input_;
 };
 
 // dTri9: 9 floats per triangle (world-space vertices), device memory.  The
