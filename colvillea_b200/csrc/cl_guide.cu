@@ -111,6 +111,21 @@ __global__ void __launch_bounds__(kTcThreads) kInferUnit(GridView g, const uint4
     tcTeardown(tmem);
 }
 
+// The caller's record rows (kRec floats: guide in9, omega, w, BSDF pdf of
+// omega; cache in9, target RGB) as training records (weight 1 for the cache).
+template <int kRec>
+__global__ void __launch_bounds__(256) kPackRecords(const float* __restrict__ rows, uint32_t n, float4* __restrict__ rec)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float* s = rows + size_t(kRec) * i;
+    float4*      d = rec + size_t(kRecordF4) * i;
+    d[0] = make_float4(s[0], s[1], s[2], kRec == 14 ? s[12 % kRec] : 1.0f);
+    d[1] = make_float4(s[3], s[4], s[5], 0.0f);
+    d[2] = make_float4(s[6], s[7], s[8], 0.0f);
+    d[3] = make_float4(s[9], s[10], s[11], kRec == 14 ? s[13 % kRec] : 0.0f);
+}
+
 // Mixture sample / pdf of given guide outputs (the network's mixture alone).
 __global__ void kSampleUnit(const float* __restrict__ out48, const float* __restrict__ u3, uint32_t n,
                             float* __restrict__ dir, float* __restrict__ pdf)
@@ -886,6 +901,42 @@ template <class S, class L> cl_status HashNet<S, L>::getParams(float* p, uint64_
     return CL_OK;
 }
 
+// Staging of the host entry points: grown to the largest call and kept (an
+// allocation and its release cost 0.6 ms).
+template <class S, class L> cl_status HashNet<S, L>::stage(DevBuf& b, size_t bytes, std::string* err)
+{
+    return b.bytes < bytes ? b.alloc(bytes, err) : CL_OK;
+}
+
+// Outputs of n host rows into io2_; asynchronous.
+template <class S, class L> cl_status HashNet<S, L>::forwardStaged(const float* in9, uint32_t n, std::string* err)
+{
+    CL_TRY(stage(io_, size_t(n) * 36, err));
+    CL_TRY(stage(io2_, size_t(n) * S::kOut * 4, err));
+    CL_CUDA(cudaMemcpyAsync(io_.p, in9, size_t(n) * 36, cudaMemcpyHostToDevice, st_), err);
+    uint32_t* flag = reinterpret_cast<uint32_t*>(scal_.as<unsigned char>() + 48);
+    CL_CUDA(cudaMemsetAsync(flag, 0, 4, st_), err);
+    kInferUnit<S><<<gridFor(n, kTcRows, numSMs_ * 2), kTcThreads, TcLayout<S>::kSmem, st_>>>(grid(), tcWeights(),
+                                                                                            io_.f(), n, io2_.f(), flag);
+    CL_CUDA(cudaGetLastError(), err);
+    return CL_OK;
+}
+
+// Synchronises the stream and reports an inference kernel's timeout.
+template <class S, class L> cl_status HashNet<S, L>::checkInferErr(std::string* err)
+{
+    uint32_t hf = 0u;
+    CL_CUDA(cudaMemcpyAsync(&hf, scal_.as<unsigned char>() + 48, 4, cudaMemcpyDeviceToHost, st_), err);
+    CL_CUDA(cudaStreamSynchronize(st_), err);
+    if (hf & kTcTimeout)
+    {
+        markTcSuspect();
+        *err = "network: a tensor-core wait ran out";
+        return CL_ERR_TIMEOUT;
+    }
+    return CL_OK;
+}
+
 template <class S, class L>
 cl_status HashNet<S, L>::forward(const float* in9, uint32_t n, float* out, std::string* err)
 {
@@ -895,25 +946,9 @@ cl_status HashNet<S, L>::forward(const float* in9, uint32_t n, float* out, std::
         return CL_ERR_INVALID_ARG;
     }
     if (n == 0) return CL_OK;
-    CL_TRY(io_.alloc(size_t(n) * 9 * 4, err));
-    CL_TRY(io2_.alloc(size_t(n) * S::kOut * 4, err));
-    CL_CUDA(cudaMemcpyAsync(io_.p, in9, size_t(n) * 9 * 4, cudaMemcpyHostToDevice, st_), err);
-    uint32_t* flag = reinterpret_cast<uint32_t*>(scal_.as<unsigned char>() + 48);
-    CL_CUDA(cudaMemsetAsync(flag, 0, 4, st_), err);
-    kInferUnit<S><<<gridFor(n, kTcRows, numSMs_ * 2), kTcThreads, TcLayout<S>::kSmem, st_>>>(grid(), tcWeights(),
-                                                                                            io_.f(), n, io2_.f(), flag);
-    CL_CUDA(cudaGetLastError(), err);
+    CL_TRY(forwardStaged(in9, n, err));
     CL_CUDA(cudaMemcpyAsync(out, io2_.p, size_t(n) * S::kOut * 4, cudaMemcpyDeviceToHost, st_), err);
-    uint32_t hf = 0u;
-    CL_CUDA(cudaMemcpyAsync(&hf, flag, 4, cudaMemcpyDeviceToHost, st_), err);
-    CL_CUDA(cudaStreamSynchronize(st_), err);
-    if (hf & kTcTimeout)
-    {
-        markTcSuspect();
-        *err = "network: a tensor-core wait ran out";
-        return CL_ERR_TIMEOUT;
-    }
-    return CL_OK;
+    return checkInferErr(err);
 }
 
 template <class S, class L>
@@ -931,17 +966,15 @@ cl_status HashNet<S, L>::sample(const float* in9, const float* u3, uint32_t n, f
         *err = "network: null buffer";
         return CL_ERR_INVALID_ARG;
     }
-    std::vector<float> out(size_t(n) * S::kOut);
-    CL_TRY(forward(in9, n, out.data(), err));
-    DevBuf u, d, p;
-    CL_TRY(u.alloc(size_t(n) * 12, err));
-    CL_TRY(d.alloc(size_t(n) * 12, err));
-    CL_TRY(p.alloc(size_t(n) * 4, err));
-    CL_CUDA(cudaMemcpyAsync(u.p, u3, size_t(n) * 12, cudaMemcpyHostToDevice, st_), err);
-    kSampleUnit<<<(n + 127) / 128, 128, 0, st_>>>(io2_.f(), u.f(), n, d.f(), p.f());
+    CL_TRY(forwardStaged(in9, n, err));
+    CL_TRY(checkInferErr(err)); // the rows in io_ are free again
+    CL_TRY(stage(rec_, size_t(n) * 16, err));
+    CL_CUDA(cudaMemcpyAsync(io_.p, u3, size_t(n) * 12, cudaMemcpyHostToDevice, st_), err);
+    float *d = rec_.f(), *p = d + 3 * size_t(n);
+    kSampleUnit<<<(n + 127) / 128, 128, 0, st_>>>(io2_.f(), io_.f(), n, d, p);
     CL_CUDA(cudaGetLastError(), err);
-    CL_CUDA(cudaMemcpyAsync(dir, d.p, size_t(n) * 12, cudaMemcpyDeviceToHost, st_), err);
-    CL_CUDA(cudaMemcpyAsync(pdf, p.p, size_t(n) * 4, cudaMemcpyDeviceToHost, st_), err);
+    CL_CUDA(cudaMemcpyAsync(dir, d, size_t(n) * 12, cudaMemcpyDeviceToHost, st_), err);
+    CL_CUDA(cudaMemcpyAsync(pdf, p, size_t(n) * 4, cudaMemcpyDeviceToHost, st_), err);
     CL_CUDA(cudaStreamSynchronize(st_), err);
     return CL_OK;
 }
@@ -960,22 +993,20 @@ cl_status HashNet<S, L>::pdf(const float* in9, const float* dir, uint32_t n, flo
         *err = "network: null buffer";
         return CL_ERR_INVALID_ARG;
     }
-    std::vector<float> out(size_t(n) * S::kOut);
-    CL_TRY(forward(in9, n, out.data(), err));
-    DevBuf d, p;
-    CL_TRY(d.alloc(size_t(n) * 12, err));
-    CL_TRY(p.alloc(size_t(n) * 4, err));
-    CL_CUDA(cudaMemcpyAsync(d.p, dir, size_t(n) * 12, cudaMemcpyHostToDevice, st_), err);
-    kPdfUnit<<<(n + 127) / 128, 128, 0, st_>>>(io2_.f(), d.f(), n, p.f());
+    CL_TRY(forwardStaged(in9, n, err));
+    CL_TRY(checkInferErr(err)); // the rows in io_ are free again
+    CL_TRY(stage(rec_, size_t(n) * 4, err));
+    CL_CUDA(cudaMemcpyAsync(io_.p, dir, size_t(n) * 12, cudaMemcpyHostToDevice, st_), err);
+    kPdfUnit<<<(n + 127) / 128, 128, 0, st_>>>(io2_.f(), io_.f(), n, rec_.f());
     CL_CUDA(cudaGetLastError(), err);
-    CL_CUDA(cudaMemcpyAsync(pdf, p.p, size_t(n) * 4, cudaMemcpyDeviceToHost, st_), err);
+    CL_CUDA(cudaMemcpyAsync(pdf, rec_.p, size_t(n) * 4, cudaMemcpyDeviceToHost, st_), err);
     CL_CUDA(cudaStreamSynchronize(st_), err);
     return CL_OK;
 }
 
 // Host records (kRecFloats per row) -> device records; the record count
-// goes to scal[2] (u32).  Guide rows: in9, omega, w, BSDF pdf of omega;
-// cache rows: in9, target RGB (weight 1).
+// goes to scal[2] (u32).  The host repacked every row into a vector of 16
+// floats before (half of a gradient call over 200,003 records).
 template <class S, class L> cl_status HashNet<S, L>::upload(const float* rec, uint32_t n, std::string* err)
 {
     if (!rec || n == 0)
@@ -983,24 +1014,13 @@ template <class S, class L> cl_status HashNet<S, L>::upload(const float* rec, ui
         *err = "network: empty or null batch";
         return CL_ERR_INVALID_ARG;
     }
-    constexpr int      kf = kRecFloats;
-    std::vector<float> h(size_t(n) * 16, 0.0f);
-    for (uint32_t i = 0; i < n; ++i)
-    {
-        const float* s = rec + kf * size_t(i);
-        float*       d = h.data() + 16 * size_t(i);
-        d[0] = s[0], d[1] = s[1], d[2] = s[2];
-        d[4] = s[3], d[5] = s[4], d[6] = s[5];
-        d[8] = s[6], d[9] = s[7], d[10] = s[8];
-        d[12] = s[9], d[13] = s[10], d[14] = s[11];
-        d[3]  = kf == 14 ? s[12] : 1.0f;
-        d[15] = kf == 14 ? s[13] : 0.0f;
-    }
-    CL_TRY(rec_.alloc(h.size() * 4, err));
-    CL_CUDA(cudaMemcpyAsync(rec_.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st_), err);
+    CL_TRY(stage(io_, size_t(n) * kRecFloats * 4, err));
+    CL_TRY(stage(rec_, size_t(n) * kRecordF4 * 16, err));
+    CL_CUDA(cudaMemcpyAsync(io_.p, rec, size_t(n) * kRecFloats * 4, cudaMemcpyHostToDevice, st_), err);
+    kPackRecords<kRecFloats><<<(n + 255) / 256, 256, 0, st_>>>(io_.f(), n, rec_.as<float4>());
+    CL_CUDA(cudaGetLastError(), err);
     CL_CUDA(cudaMemcpyAsync(scal_.as<unsigned char>() + 16, &n, 4, cudaMemcpyHostToDevice, st_), err);
-    CL_CUDA(cudaStreamSynchronize(st_), err);
-    return CL_OK;
+    return CL_OK; // the callers end in a synchronisation of the stream
 }
 
 template <class S, class L>

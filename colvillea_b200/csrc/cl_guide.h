@@ -55,6 +55,9 @@ public:
     uint64_t        steps() const { return step_; }
 
 private:
+    cl_status stage(DevBuf& b, size_t bytes, std::string* err);
+    cl_status forwardStaged(const float* in9, uint32_t n, std::string* err);
+    cl_status checkInferErr(std::string* err);
     cl_status upload(const float* rec, uint32_t n, std::string* err);
     cl_status computeGradient(const float4* rec, const uint32_t* count, std::string* err);
     cl_status refreshCopies(std::string* err);
