@@ -370,6 +370,8 @@ constexpr size_t kDomeSmemMax = 227u * 1024u;
 
 } // namespace
 
+bool domeNeedsScratch(int w, int h) { return domeTableSmem(w) > kDomeSmemMax || domeTableSmem(h) > kDomeSmemMax; }
+
 cl_status launchDomeBuild(const float4* dTex, int w, int h, cudaStream_t st, const DomeScratch& s, float* pU, float* cU,
                           float* pV, float* cV, uint2* aliasRow, uint2* aliasCol, std::string* err)
 {
@@ -413,20 +415,31 @@ cl_status buildDome(const float* hostTexels, int w, int h, cudaStream_t st, Dome
     out->w = w;
     out->h = h;
     size_t n = size_t(w) * h;
-    CL_TRY(out->tex.alloc(n * 16, err));
-    CL_TRY(out->pU.alloc(size_t(w + 1) * h * 4, err));
-    CL_TRY(out->cU.alloc(size_t(w + 1) * h * 4, err));
-    CL_TRY(out->pV.alloc(size_t(h + 1) * 4, err));
-    CL_TRY(out->cV.alloc(size_t(h + 1) * 4, err));
-    CL_TRY(out->aliasRow.alloc(size_t(h) * 8, err));
-    CL_TRY(out->aliasCol.alloc(n * 8, err));
-    DevBuf weights, rowC, idx, q;
-    CL_TRY(weights.alloc(n * 8, err));
-    CL_TRY(rowC.alloc(size_t(h) * 8, err));
-    CL_TRY(idx.alloc(n * 2 * 4 + size_t(h) * 2 * 4, err));
-    CL_TRY(q.alloc(n * 8 + size_t(h) * 8, err));
+    Carver cv;
+    cv.take(out->tex, n * 16);
+    cv.take(out->pU, size_t(w + 1) * h * 4);
+    cv.take(out->cU, size_t(w + 1) * h * 4);
+    cv.take(out->pV, size_t(h + 1) * 4);
+    cv.take(out->cV, size_t(h + 1) * 4);
+    cv.take(out->aliasRow, size_t(h) * 8);
+    cv.take(out->aliasCol, n * 8);
+    cv.take(out->rowC, size_t(h) * 8);
+    // A dome of the same size replaces the last one in place.
+    if (out->mem.bytes != cv.peak()) CL_TRY(out->mem.alloc(cv.peak(), err));
+    cv.bind(out->mem.p);
+    DevBuf     scratch;
+    ScratchBuf weights, idx, q;
+    if (domeNeedsScratch(w, h))
+    {
+        Carver sc;
+        sc.take(weights, n * 8);
+        sc.take(idx, n * 2 * 4 + size_t(h) * 2 * 4);
+        sc.take(q, n * 8 + size_t(h) * 8);
+        CL_TRY(scratch.alloc(sc.peak(), err));
+        sc.bind(scratch.p);
+    }
     CL_CUDA(cudaMemcpyAsync(out->tex.p, hostTexels, n * 16, cudaMemcpyHostToDevice, st), err);
-    DomeScratch s{weights.as<double>(), rowC.as<double>(), idx.u(), q.as<double>()};
+    DomeScratch s{weights.as<double>(), out->rowC.as<double>(), idx.u(), q.as<double>()};
     CL_TRY(launchDomeBuild(out->tex.as<float4>(), w, h, st, s, out->pU.f(), out->cU.f(), out->pV.f(), out->cV.f(),
                            out->aliasRow.as<uint2>(), out->aliasCol.as<uint2>(), err));
     CL_CUDA(cudaStreamSynchronize(st), err);

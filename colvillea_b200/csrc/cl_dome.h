@@ -8,11 +8,13 @@ namespace clb
 {
 struct DomeTables
 {
-    DevBuf tex;      // float4 w*h
-    DevBuf pU, cU;   // float (w+1)*h
-    DevBuf pV, cV;   // float h+1
-    DevBuf aliasRow; // uint2 h
-    DevBuf aliasCol; // uint2 w*h
+    DevBuf     mem;      // holds the parts below
+    ScratchBuf tex;      // float4 w*h
+    ScratchBuf pU, cU;   // float (w+1)*h
+    ScratchBuf pV, cV;   // float h+1
+    ScratchBuf aliasRow; // uint2 h
+    ScratchBuf aliasCol; // uint2 w*h
+    ScratchBuf rowC;     // build: FP64 row integrals, h
     int    w = 0, h = 0;
 
     DomeView view() const
@@ -31,8 +33,9 @@ struct DomeTables
     }
 };
 
-// Scratch of the build: FP64 texel weights (w*h), FP64 row integrals (h),
-// Vose work lists (2*w*h + 2*h indices) and FP64 scaled weights (w*h + h).
+// Scratch of the build: FP64 row integrals (h) and, for tables too large for
+// shared memory only, FP64 texel weights (w*h), Vose work lists (2*w*h + 2*h
+// indices) and FP64 scaled weights (w*h + h).
 struct DomeScratch
 {
     double*   weights;
@@ -40,6 +43,8 @@ struct DomeScratch
     uint32_t* idx;
     double*   q;
 };
+
+bool domeNeedsScratch(int w, int h);
 
 cl_status launchDomeBuild(const float4* dTex, int w, int h, cudaStream_t st, const DomeScratch& s, float* pU, float* cU,
                           float* pV, float* cV, uint2* aliasRow, uint2* aliasCol, std::string* err);

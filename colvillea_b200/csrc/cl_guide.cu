@@ -827,17 +827,17 @@ template <class S, class L> cl_status HashNet<S, L>::init(cudaStream_t st, std::
             err);
     CL_CUDA(cudaFuncSetAttribute(kInferUnit<S>, cudaFuncAttributePreferredSharedMemoryCarveout, 100), err);
     CL_CUDA(cudaFuncSetAttribute(kTrainTc<S, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainTc<S>::kSmem), err);
-    CL_TRY(params_.alloc(n * 4, err));
-    CL_TRY(grad_.alloc(n * 4, err));
-    CL_TRY(m_.alloc(n * 4, err));
-    CL_TRY(v_.alloc(n * 4, err));
-    CL_TRY(table_.alloc(hashParams_ * 2, err));
-    CL_TRY(wt_.alloc(TcLayout<S>::kWBytes, err));
-    CL_TRY(scal_.alloc(64, err));
     {
         const size_t tiles = (size_t(cfg_.batch) + kTcRows - 1) / kTcRows;
-        CL_TRY(enc_.alloc(tiles * TrainTc<S>::kA0, err));
-        CL_TRY(aux_.alloc(tiles * kTcRows * 32, err));
+        Carver       cv;
+        for (ScratchBuf* b : {&params_, &grad_, &m_, &v_}) cv.take(*b, n * 4);
+        cv.take(table_, hashParams_ * 2);
+        cv.take(wt_, TcLayout<S>::kWBytes);
+        cv.take(scal_, 64);
+        cv.take(enc_, tiles * TrainTc<S>::kA0);
+        cv.take(aux_, tiles * kTcRows * 32);
+        CL_TRY(mem_.alloc(cv.peak(), err));
+        cv.bind(mem_.p);
     }
     kInitParams<S><<<gridFor(n, 256, numSMs_ * 8), 256, 0, st_>>>(params_.f(), hashParams_, cfg_.seed);
     CL_CUDA(cudaGetLastError(), err);

@@ -70,13 +70,14 @@ private:
     int             numSMs_ = 148;
     uint64_t        step_ = 0;
 
-    DevBuf params_, grad_, m_, v_; // FP32 [hash | mlp]
-    DevBuf table_;                 // bf16 copy of the hash table
-    DevBuf wt_;                    // bf16 weights in the tensor-core canonical layout
-    DevBuf scal_;                  // {sum w, loss, count (u32), sum of clamped w}; byte 48: inference error
+    DevBuf     mem_;                   // holds the network's state below
+    ScratchBuf params_, grad_, m_, v_; // FP32 [hash | mlp]
+    ScratchBuf table_;                 // bf16 copy of the hash table
+    ScratchBuf wt_;                    // bf16 weights in the tensor-core canonical layout
+    ScratchBuf scal_;              // {sum w, loss, count (u32), sum of clamped w}; byte 48: inference error
                                    // flags; byte 52: training error flags
     DevBuf rec_, io_, io2_;        // host-entry staging
-    DevBuf enc_, aux_;             // training: encoded batch in tensor-core tiles, per-sample loss inputs
+    ScratchBuf enc_, aux_;         // training: encoded batch in tensor-core tiles, per-sample loss inputs
 };
 
 using GuideNet = HashNet<guide::GuideShape, GuideLoss>;

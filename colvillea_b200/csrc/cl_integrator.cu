@@ -2439,31 +2439,24 @@ cl_status Integrator::ensureQueues(std::string* err)
 {
     CL_TRY(checkPathSlots(err));
     uint32_t slots = cfg_.path_slots ? cfg_.path_slots : (1u << 21);
-    if (slots == slots_ && rqO_[0].p) return CL_OK;
-    size_t s = slots;
+    if (slots == slots_ && queues_.p) return CL_OK;
+    const size_t s  = slots;
+    const bool   dl = type_ == CL_INTEGRATOR_DIRECT_LIGHTING;
+    Carver       cv;
     for (int q = 0; q < 2; ++q)
     {
-        CL_TRY(rqO_[q].alloc(s * 16, err));
-        CL_TRY(rqD_[q].alloc(s * 16, err));
-        CL_TRY(rqSlot_[q].alloc(s * 4, err));
+        cv.take(rqO_[q], s * 16);
+        cv.take(rqD_[q], s * 16);
+        cv.take(rqSlot_[q], s * 4);
     }
-    CL_TRY(hit_.alloc(s * 16, err));
-    CL_TRY(hitIdx_.alloc(s * 16, err));
-    CL_TRY(hitInst_.alloc(s * 4, err));
-    CL_TRY(sqO_.alloc(s * 16, err));
-    CL_TRY(sqD_.alloc(s * 16, err));
-    CL_TRY(sqL_.alloc(s * 16, err));
-    if (type_ == CL_INTEGRATOR_DIRECT_LIGHTING)
-    {
-        CL_TRY(sqD2_.alloc(s * 16, err));
-        CL_TRY(sqL2_.alloc(s * 16, err));
-    }
-    CL_TRY(vis_.alloc(s * 2, err));
-    CL_TRY(classIdx_.alloc(s * 4 * 4, err));
-    CL_TRY(psInfo_.alloc(s * 16, err));
-    CL_TRY(psT_.alloc(s * 16, err));
-    CL_TRY(psE_.alloc(s * 16, err));
-    CL_TRY(psL_.alloc(s * 16, err));
+    for (ScratchBuf* b : {&hit_, &hitIdx_, &sqO_, &sqD_, &sqL_, &psInfo_, &psT_, &psE_, &psL_, &classIdx_})
+        cv.take(*b, s * 16);
+    cv.take(hitInst_, s * 4);
+    cv.take(sqD2_, dl ? s * 16 : 16);
+    cv.take(sqL2_, dl ? s * 16 : 16);
+    cv.take(vis_, s * 2);
+    CL_TRY(queues_.alloc(cv.peak(), err));
+    cv.bind(queues_.p);
     slots_      = slots;
     shadowCap_  = slots;
     graphValid_ = false;

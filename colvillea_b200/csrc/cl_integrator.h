@@ -276,8 +276,10 @@ private:
     DevBuf       resolve_;
     cudaStream_t copyStream_ = nullptr;
     cudaEvent_t  evResolved_ = nullptr, evCopied_ = nullptr;
-    DevBuf rqO_[2], rqD_[2], rqSlot_[2], hit_, hitIdx_, hitInst_, sqO_, sqD_, sqL_, sqD2_, sqL2_;
-    DevBuf psInfo_, psT_, psE_, psL_, ctr_, wp_, vis_, classIdx_;
+    DevBuf     ctr_, wp_;
+    DevBuf     queues_; // holds the queues and the path state below
+    ScratchBuf rqO_[2], rqD_[2], rqSlot_[2], hit_, hitIdx_, hitInst_, sqO_, sqD_, sqL_, sqD2_, sqL2_;
+    ScratchBuf psInfo_, psT_, psE_, psL_, vis_, classIdx_;
     uint32_t slots_ = 0, shadowCap_ = 0;
     WaveParams* hostWp_ = nullptr;   // pinned
     uint32_t*   hostCount_ = nullptr; // pinned
