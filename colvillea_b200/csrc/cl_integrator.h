@@ -73,6 +73,8 @@ struct Counters
     uint32_t           cacheRec;   // radiance cache: training records appended (may exceed the capacity)
     uint32_t           cacheTrainCount; // radiance cache: records the training step reads (clamped)
     uint32_t           tailBlocks; // blocks of kPathTail that have ended
+    uint32_t           tailNow;    // kPathTail takes the next wave's queue
+    uint32_t           resolveBlocks; // blocks of kShadowResolve that have ended
     unsigned long long cacheQueries; // radiance cache: network evaluations
 };
 
@@ -183,7 +185,7 @@ public:
     cl_status domeAliasTables(uint32_t* aliasRow, uint32_t* aliasCol, std::string* err);
     cl_status waveRays(uint64_t* out, uint32_t cap, uint32_t* count, std::string* err) const;
     cl_status guideProbe(uint32_t cap, float* rows, uint32_t* count, std::string* err);
-    cl_status beginPass(uint32_t spp, bool record, bool cacheTrain, uint32_t* initSlots, std::string* err);
+    cl_status beginPass(uint32_t spp, bool record, bool cacheTrain, uint32_t* initSlots, bool* tailOnly, std::string* err);
     cl_status domeAliasSample(const float* u2, float* dir, float* pdf, float* val, uint32_t n, std::string* err);
 
     cl_status setGuiding(const cl_guide_config* cfg, std::string* err);
@@ -211,7 +213,7 @@ private:
     cl_status captureGraph(std::string* err);
     cl_status launchWave(int cur, bool profile, std::string* err);
     bool      usesTail() const;
-    cl_status launchTail(int cur, std::string* err);
+    cl_status launchTail(int cur, cudaStream_t st, std::string* err);
     Params    params() const;
     ClassifyView classifyView() const;
     BvhView      bvhView() const;
@@ -297,8 +299,8 @@ private:
     float     msBvhWall_ = 0, msBvhAlloc_ = 0; // last full build: host wall time, and its cudaMalloc share
     std::vector<uint64_t> waveRays_;       // CL_PROFILE_STAGES: closest-hit rays of each wave of the last render
     unsigned long long    waveRaysSeen_ = 0;
-    cudaStream_t shadeStream_[3] = {}; // branches of a captured wave
-    cudaEvent_t  evFork_ = nullptr, evJoin_[3] = {};
+    cudaStream_t shadeStream_[3] = {}, shadowStream_ = nullptr; // branches of a captured wave
+    cudaEvent_t  evFork_ = nullptr, evJoin_[4] = {};
     cudaEvent_t evA_ = nullptr, evB_ = nullptr, evS_[6] = {};
 
     // Guiding.
