@@ -4,13 +4,22 @@
 // (src/core/devices/optixdevice.cpp:136-233, src/core/devices/optix.cu:38-110):
 // B200 has no RT cores, so traversal runs on the SMs.
 //
-// Node (80 bytes = 5 x uint4), after the compressed wide BVH of Ylitie,
+// Node (96 bytes = 6 x uint4), after the compressed wide BVH of Ylitie,
 // Karras and Laine (HPG 2017):
 //   n0 = {p.x, p.y, p.z, ex | ey<<8 | ez<<16 | imask<<24}
 //   n1 = {childBase, triBase, meta[0..3], meta[4..7]}
 //   n2 = {qlo.x[0..3], qlo.x[4..7], qlo.y[0..3], qlo.y[4..7]}
 //   n3 = {qlo.z[0..3], qlo.z[4..7], qhi.x[0..3], qhi.x[4..7]}
 //   n4 = {qhi.y[0..3], qhi.y[4..7], qhi.z[0..3], qhi.z[4..7]}
+//   n5 = {leaf word, 2^(ex-127), 2^(ey-127), 2^(ez-127)}
+// Three 32-byte loads fetch a node (five of 16 bytes before); n5 repeats what
+// the traversal would unpack from n0 and n1: the scales as floats and, in bits
+// 3 s .. 3 s + 2 of the leaf word, the unary triangle count of leaf slot s, so
+// that the triangles of the hit leaf slots are one table lookup and one AND
+// instead of a loop over the slots (which ran at the warp's longest count, for a
+// few lanes).  A node of 80 bytes without n5: config 2's 16.6 M paths took 45.7
+// ms, 45.3 with the wide loads, 43.8 with the leaf word, 43.5 with the scales.
+// cl_get_bvh returns the first 80 bytes.
 // Child box of slot s: p + 2^(e-127) * q.  imask bit s: slot s is an inner
 // node, stored at childBase + popc(imask & ((1<<s)-1)).  Leaf slot meta:
 // (unary triangle count << 5) | offset from triBase (at most 3 triangles per
@@ -29,6 +38,8 @@ namespace clb
 {
 constexpr int kStackDepth    = 24; // bound checked against the built tree depth
 constexpr int kTraceBlock    = 128;
+constexpr int kNodeU4        = 6; // uint4 per node in device memory
+constexpr int kTriF4         = 3; // float4 per triangle
 constexpr uint32_t kMissPrim = 0xffffffffu;
 
 // Two-level scenes (CL_TWO_LEVEL): one tree per mesh in object space, and a
@@ -60,16 +71,18 @@ struct BvhView
     uint32_t stackDepth;
 };
 
-// Lane refill in the persistent traversal kernels of flattened scenes: a lane
+// Lane refill in the persistent traversal kernels: a lane
 // runs up to kRefillSteps traversal steps with no warp-synchronous operation
 // (a vote in every step would make the warp reconverge at each step, which
 // cost more than the idle lanes it saves), then the warp votes and, when at
 // least kRefillIdle lanes are idle, gives them the next rays.  Measured on
-// config 2 (1920x1080, 4.7 M triangles): 2-6 idle lanes and 3-6 steps are
-// within 1% of each other; 1 step (a vote per step) was 60% slower than no
-// refill at all, 16 steps 4% slower than 4.
-constexpr uint32_t kRefillIdle  = 4;
-constexpr uint32_t kRefillSteps = 4;
+// config 2 (1920x1080, 4.7 M triangles): 3-6 idle lanes and 3-6 steps are
+// within 0.5% of each other; 1 step (a vote per step) was 60% slower than no
+// refill at all, 16 steps 4% slower than 4.  Two-level scenes: 6 steps, 2%
+// faster than 4 (1280x720 over 577 instances).
+constexpr uint32_t kRefillIdle     = 4;
+constexpr uint32_t kRefillSteps    = 4;
+constexpr uint32_t kRefillStepsTwo = 6;
 
 __host__ __device__ constexpr size_t traceStackBytes(uint32_t depth) { return size_t(depth) * kTraceBlock * 8u; }
 
@@ -88,6 +101,38 @@ __device__ __forceinline__ float2 bytePair(uint32_t wa, uint32_t wb, int b)
                        __uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7440u | uint32_t(b))));
 }
 
+// One 32-byte load (32-byte aligned) of read-only memory.
+__device__ __forceinline__ void ldg256(const void* p, uint4& a, uint4& b)
+{
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+        : "l"(p));
+}
+__device__ __forceinline__ void loadTri(const float4* __restrict__ tris, uint32_t i, float4& a, float4& b, float4& c)
+{
+    const float4* tp = tris + size_t(i) * kTriF4;
+    a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+}
+
+// Reciprocals of a ray direction's components for the box tests (components
+// below 1e-30 count as that): the hardware approximation and one Newton step,
+// within an ulp of the IEEE quotient, whose three calls were a sixth of the work
+// of giving a lane its next ray.  Components beyond the approximation's range
+// take the quotient.
+__device__ __forceinline__ float boxRcp(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return __fmaf_rn(r, __fmaf_rn(-x, r, 1.0f), r);
+}
+__device__ __forceinline__ f3 boxReciprocals(f3 d)
+{
+    const f3 c{fabsf(d.x) < 1e-30f ? copysignf(1e-30f, d.x) : d.x, fabsf(d.y) < 1e-30f ? copysignf(1e-30f, d.y) : d.y,
+               fabsf(d.z) < 1e-30f ? copysignf(1e-30f, d.z) : d.z};
+    if (!(fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))) < 1e37f)) return {1.0f / c.x, 1.0f / c.y, 1.0f / c.z};
+    return {boxRcp(c.x), boxRcp(c.y), boxRcp(c.z)};
+}
+
 // Three-input minimum and maximum (sm_100 min.f32 / max.f32 with three
 // operands; exact, like the nested two-input forms).
 __device__ __forceinline__ float max3f(float a, float b, float c)
@@ -103,11 +148,13 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
     return r;
 }
 
-// Child-key table (shared memory, kKeyLutBytes per block): entry oct * 256 + m
+// Tables in shared memory (kLutBytes per block).  Child keys: entry oct * 256 + m
 // is the 8-bit slot mask m with each slot s moved to bit s ^ oct, the order in
 // which a ray of octant oct visits the children.  One table lookup per node
-// replaces three conditional bit swaps on the busiest (integer) pipe.
+// replaces three conditional bit swaps on the busiest (integer) pipe.  After
+// them, 256 words: entry m has bits 3 s .. 3 s + 2 set for each slot s of m.
 constexpr int kKeyLutBytes = 8 * 256;
+constexpr int kLutBytes    = kKeyLutBytes + 4 * 256;
 __device__ __forceinline__ void fillKeyLut(uint8_t* lut)
 {
     for (int i = threadIdx.x; i < kKeyLutBytes; i += blockDim.x)
@@ -118,21 +165,31 @@ __device__ __forceinline__ void fillKeyLut(uint8_t* lut)
         k = (oct & 4u) ? (((k & 0x0fu) << 4) | ((k >> 4) & 0x0fu)) : k;
         lut[i] = uint8_t(k);
     }
+    for (int i = threadIdx.x; i < 256; i += blockDim.x)
+    {
+        uint32_t m = 0u;
+        for (int b = 0; b < 8; ++b)
+            if (i & (1 << b)) m |= 7u << (3 * b);
+        reinterpret_cast<uint32_t*>(lut + kKeyLutBytes)[i] = m;
+    }
     __syncthreads();
 }
 
 // Intersects the ray with the 8 children of one node; returns the hit mask:
-// bits 24..31 inner-child keys (slot ^ octant), bits 0..23 triangle offsets.
+// bits 24..31 inner-child keys (slot ^ octant), bits 0..23 the hit leaf slots'
+// triangles, bit 3 s + k for triangle k of slot s (the popc(leafWord & (bit -
+// 1))-th triangle of the node).
 __device__ __forceinline__ uint32_t intersectNode(const uint4* __restrict__ nodes, uint32_t idx, f3 o, f3 inv, uint32_t oct,
                                                   float tmin, float tmax, uint32_t* childBase, uint32_t* triBase,
-                                                  uint32_t* imaskOut, const uint8_t* keyLut)
+                                                  uint32_t* imaskOut, const uint8_t* keyLut, uint32_t* leafWord)
 {
-    const uint4* np = nodes + size_t(idx) * 5;
-    const uint4  n0 = __ldg(np + 0), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
+    const uint4* np = nodes + size_t(idx) * kNodeU4;
+    uint4        n0, n1, n2, n3, n4, n5;
+    ldg256(np, n0, n1);
+    ldg256(np + 2, n2, n3);
+    ldg256(np + 4, n4, n5);
     float px = __uint_as_float(n0.x), py = __uint_as_float(n0.y), pz = __uint_as_float(n0.z);
-    float sx = __uint_as_float((n0.w & 0xffu) << 23);
-    float sy = __uint_as_float(((n0.w >> 8) & 0xffu) << 23);
-    float sz = __uint_as_float(((n0.w >> 16) & 0xffu) << 23);
+    float sx = __uint_as_float(n5.y), sy = __uint_as_float(n5.z), sz = __uint_as_float(n5.w);
     uint32_t imask = n0.w >> 24;
     *childBase     = n1.x;
     *triBase       = n1.y;
@@ -167,16 +224,9 @@ __device__ __forceinline__ uint32_t intersectNode(const uint4* __restrict__ node
     }
     // Inner children: slot s -> key s ^ oct (bit permutation of the mask, from the table).
     uint32_t hits = uint32_t(keyLut[(oct << 8) | (hitSlots & imask)]) << 24;
-    // Leaf children: their triangle ranges (unary count << 5 | offset).
-    uint32_t leaf = hitSlots & ~imask;
-    while (leaf)
-    {
-        uint32_t sl   = __ffs(leaf) - 1;
-        leaf &= leaf - 1u;
-        uint32_t meta = ((sl < 4 ? n1.z : n1.w) >> (8 * (sl & 3u))) & 0xffu;
-        hits |= (meta >> 5) << (meta & 31u);
-    }
-    return hits;
+    // Leaf children: bit 3 s + k for triangle k of hit leaf slot s.
+    *leafWord = n5.x;
+    return hits | (reinterpret_cast<const uint32_t*>(keyLut + kKeyLutBytes)[hitSlots & ~imask] & n5.x);
 }
 
 // Per-ray traversal state, advanced one step at a time: a node test (when no
@@ -193,6 +243,7 @@ struct Trav
     uint32_t oct;
     float    tmin, tmax;
     uint2    ng, tg;
+    uint32_t tv; // leaf word of tg's node
     int      sp;
     uint32_t best;
     float    bt, b1, b2;
@@ -201,9 +252,7 @@ struct Trav
 __device__ __forceinline__ void travInit(Trav& s, f3 o, f3 d, float tmin, float tmax)
 {
     s.pre   = rayPrepare(o, d);
-    s.inv.x = 1.0f / (fabsf(d.x) < 1e-30f ? copysignf(1e-30f, d.x) : d.x);
-    s.inv.y = 1.0f / (fabsf(d.y) < 1e-30f ? copysignf(1e-30f, d.y) : d.y);
-    s.inv.z = 1.0f / (fabsf(d.z) < 1e-30f ? copysignf(1e-30f, d.z) : d.z);
+    s.inv   = boxReciprocals(d);
     s.oct   = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin  = tmin;
     s.tmax  = tmax;
@@ -245,7 +294,7 @@ __device__ __forceinline__ bool travStep(const BvhView& bvh, Trav& s, uint2* sta
             ++s.sp;
         }
         uint32_t cb, tb, im;
-        uint32_t hits = intersectNode(bvh.nodes, child, s.pre.o, s.inv, s.oct, s.tmin, s.bt, &cb, &tb, &im, keyLut);
+        uint32_t hits = intersectNode(bvh.nodes, child, s.pre.o, s.inv, s.oct, s.tmin, s.bt, &cb, &tb, &im, keyLut, &s.tv);
         if (STATS) cnt->nodes++;
         s.ng = make_uint2(cb, (hits & 0xff000000u) | im);
         s.tg = make_uint2(tb, hits & 0x00ffffffu);
@@ -254,10 +303,8 @@ __device__ __forceinline__ bool travStep(const BvhView& bvh, Trav& s, uint2* sta
     {
         uint32_t k = __ffs(s.tg.y) - 1;
         s.tg.y &= ~(1u << k);
-        const float4* tp = bvh.tris + size_t(s.tg.x + k) * 3;
-        float4        a  = __ldg(tp + 0);
-        float4        b  = __ldg(tp + 1);
-        float4        c  = __ldg(tp + 2);
+        float4 a, b, c;
+        loadTri(bvh.tris, s.tg.x + __popc(s.tv & ((1u << k) - 1u)), a, b, c);
         if (STATS) cnt->tris++;
         float t, u, v;
         if (intersectTri(s.pre, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, f3{c.x, c.y, c.z}, &t, &u, &v) && t > s.tmin)
@@ -323,6 +370,7 @@ struct Trav2
     uint32_t      oct;
     float         tmin, tmax;
     uint2         ng, tg;
+    uint32_t      tv; // leaf word of tg's node
     int           sp, blasSp;
     uint32_t      inst;     // current instance, kMissPrim in the top tree
     uint32_t      best, bestInst;
@@ -335,9 +383,7 @@ struct Trav2
 __device__ __forceinline__ void trav2SetRay(Trav2& s, f3 o, f3 d)
 {
     s.pre   = rayPrepare(o, d);
-    s.inv.x = 1.0f / (fabsf(d.x) < 1e-30f ? copysignf(1e-30f, d.x) : d.x);
-    s.inv.y = 1.0f / (fabsf(d.y) < 1e-30f ? copysignf(1e-30f, d.y) : d.y);
-    s.inv.z = 1.0f / (fabsf(d.z) < 1e-30f ? copysignf(1e-30f, d.z) : d.z);
+    s.inv   = boxReciprocals(d);
     s.oct   = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
 }
 
@@ -395,7 +441,7 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
             ++s.sp;
         }
         uint32_t cb, tb, im;
-        uint32_t hits = intersectNode(s.nodes, child, s.pre.o, s.inv, s.oct, s.tmin, s.bt, &cb, &tb, &im, keyLut);
+        uint32_t hits = intersectNode(s.nodes, child, s.pre.o, s.inv, s.oct, s.tmin, s.bt, &cb, &tb, &im, keyLut, &s.tv);
         if (STATS) cnt->nodes++;
         s.ng = make_uint2(cb, (hits & 0xff000000u) | im);
         s.tg = make_uint2(tb, hits & 0x00ffffffu);
@@ -404,12 +450,11 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
     {
         uint32_t k = __ffs(s.tg.y) - 1;
         s.tg.y &= ~(1u << k);
-        const float4* tp = s.tris + size_t(s.tg.x + k) * 3;
+        const uint32_t ti = s.tg.x + __popc(s.tv & ((1u << k) - 1u));
         if (s.inst != kMissPrim)
         {
-            float4 a = __ldg(tp + 0);
-            float4 b = __ldg(tp + 1);
-            float4 c = __ldg(tp + 2);
+            float4 a, b, c;
+            loadTri(s.tris, ti, a, b, c);
             if (STATS) cnt->tris++;
             float t, u, v;
             if (intersectTri(s.pre, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, f3{c.x, c.y, c.z}, &t, &u, &v) && t > s.tmin)
@@ -438,7 +483,7 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
         else
         {
             // An instance entry of the top tree: keep the rest of this node on the stack, enter the mesh tree.
-            const uint32_t id = __float_as_uint(__ldg(&tp->w));
+            const uint32_t id = __float_as_uint(__ldg(&s.tris[size_t(ti) * kTriF4].w));
             const int      need = (s.ng.y > 0x00ffffffu ? 1 : 0) + (s.tg.y ? 1 : 0);
             if (s.sp + need > int(bvh.stackDepth))
             {
@@ -447,7 +492,13 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
                 return true;
             }
             if (s.ng.y > 0x00ffffffu) stack[(s.sp++) * kTraceBlock] = s.ng;
-            if (s.tg.y) stack[(s.sp++) * kTraceBlock] = s.tg;
+            if (s.tg.y)
+            {
+                // Without the leaf word: the entries' own ranks as bits (tv all ones when popped).
+                uint32_t left = s.tg.y, rest = 0u;
+                for (; left; left &= left - 1u) rest |= 1u << __popc(s.tv & ((left & (0u - left)) - 1u));
+                stack[(s.sp++) * kTraceBlock] = make_uint2(s.tg.x, rest);
+            }
             const InstDev* in = bvh.inst + id;
             s.blasSp          = s.sp;
             s.inst            = id;
@@ -480,6 +531,7 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
         else
         {
             s.tg = e;
+            s.tv = 0x00ffffffu;
             s.ng = make_uint2(0u, 0u);
         }
     }

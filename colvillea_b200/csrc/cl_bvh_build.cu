@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseArgs A, co
             {
                 const uint32_t tid = A.ids[x & ~kLeafFlag];
                 const float*   tp  = A.triPos + 9 * size_t(tid);
-                float4*        dst = A.tris + size_t(tbase + triOff + got) * 3;
+                float4*        dst = A.tris + size_t(tbase + triOff + got) * kTriF4;
                 dst[0]             = make_float4(tp[0], tp[1], tp[2], __uint_as_float(tid));
                 dst[1]             = make_float4(tp[3], tp[4], tp[5], 0.0f);
                 dst[2]             = make_float4(tp[6], tp[7], tp[8], 0.0f);
@@ -1023,7 +1023,7 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseArgs A, co
     }
     if (q == 0u)
     {
-        uint4* np = A.nodes + size_t(wide) * 5;
+        uint4* np = A.nodes + size_t(wide) * kNodeU4;
         np[0]     = make_uint4(__float_as_uint(plo[0]), __float_as_uint(plo[1]), __float_as_uint(plo[2]),
                                ex[0] | (ex[1] << 8) | (ex[2] << 16) | (imask << 24));
         np[1]     = make_uint4(base, tbase, wd[6], w1[6]);
@@ -1031,6 +1031,10 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseArgs A, co
         np[3]     = make_uint4(wd[2], w1[2], wd[3], w1[3]);
         np[4]     = make_uint4(wd[4], w1[4], wd[5], w1[5]);
     }
+    // Leaf word and scales (n5).
+    uint32_t lv = (meta >> 5) << (3u * q);
+    for (int o = 1; o < 8; o <<= 1) lv |= __shfl_xor_sync(gm, lv, o, 8);
+    if (q == 0u) A.nodes[size_t(wide) * kNodeU4 + 5] = make_uint4(lv, ex[0] << 23, ex[1] << 23, ex[2] << 23);
 }
 
 // Validation of a built tree (error bits: 1 exponent outside 1..254, 2 child
@@ -1040,7 +1044,7 @@ __global__ void kValidateNodes(const uint4* __restrict__ nodes, uint32_t numNode
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= numNodes) return;
-    uint4    n0 = nodes[size_t(i) * 5], n1 = nodes[size_t(i) * 5 + 1];
+    uint4    n0 = nodes[size_t(i) * kNodeU4], n1 = nodes[size_t(i) * kNodeU4 + 1];
     uint32_t imask = n0.w >> 24, bits = 0u;
     for (int a = 0; a < 3; ++a)
     {
@@ -1064,7 +1068,7 @@ __global__ void kValidateTris(const float4* __restrict__ tris, uint32_t n, uint3
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t id = __float_as_uint(tris[size_t(i) * 3].w);
+    uint32_t id = __float_as_uint(tris[size_t(i) * kTriF4].w);
     if (id >= n)
     {
         atomicOr(err, 8u);
@@ -1134,8 +1138,8 @@ cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh*
     cv.take(dpLeafParent, nn * 4);
     cv.take(tasksA, taskCap * 8);
     cv.take(tasksB, taskCap * 8);
-    cv.take(nodes, size_t(maxNodes) * 80);
-    cv.take(tris, nn * 48);
+    cv.take(nodes, size_t(maxNodes) * kNodeU4 * 16);
+    cv.take(tris, nn * kTriF4 * 16);
     cv.take(verr, 4);
     cv.take(seen, (nn + 31) / 32 * 4);
     CL_TRY(mem.reserve(cv.peak(), err));
@@ -1315,8 +1319,8 @@ cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh*
     // per node), so that a refit allocates nothing.
     {
         Carver keep;
-        keep.take(out->nodes, size_t(out->numNodes) * 80);
-        keep.take(out->tris, nn * 48);
+        keep.take(out->nodes, size_t(out->numNodes) * kNodeU4 * 16);
+        keep.take(out->tris, nn * kTriF4 * 16);
         keep.take(out->exact, size_t(out->numNodes) * 24);
         keep.take(out->scene, 64);
         CL_TRY(out->mem.alloc(keep.peak(), err));
@@ -1367,7 +1371,7 @@ __global__ void __launch_bounds__(256) kRefitTris(float4* __restrict__ tris, uin
     uint32_t            ol[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, oh[3] = {0u, 0u, 0u};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
-        float4*  t   = tris + 3 * size_t(i);
+        float4*  t   = tris + kTriF4 * size_t(i);
         uint32_t tid = __float_as_uint(t[0].w);
         uint4    ix  = triIdx[tid];
         float4   a = vtx[3 * size_t(ix.x)], b = vtx[3 * size_t(ix.y)], c = vtx[3 * size_t(ix.z)];
@@ -1432,7 +1436,7 @@ __global__ void __launch_bounds__(128) kRefitLevel(uint4* __restrict__ nodes, co
         sh[a] = funordered(bounds[3 + a]);
     }
     float  margin = sceneMargin(sl, sh);
-    uint4* np     = nodes + size_t(node) * 5;
+    uint4* np     = nodes + size_t(node) * kNodeU4;
     uint4  n0 = make_uint4(0, 0, 0, 0), n1 = make_uint4(0, 0, 0, 0);
     if (valid)
     {
@@ -1463,7 +1467,7 @@ __global__ void __launch_bounds__(128) kRefitLevel(uint4* __restrict__ nodes, co
                 uint32_t off = m & 31u, cnt = __popc(m >> 5);
                 for (uint32_t j = 0; j < cnt; ++j)
                 {
-                    const float4* tp = tris + size_t(n1.y + off + j) * 3;
+                    const float4* tp = tris + size_t(n1.y + off + j) * kTriF4;
                     for (int v = 0; v < 3; ++v)
                     {
                         float4 p = tp[v];
@@ -1529,6 +1533,7 @@ __global__ void __launch_bounds__(128) kRefitLevel(uint4* __restrict__ nodes, co
         np[2] = make_uint4(wl[0], wl1[0], wl[1], wl1[1]);
         np[3] = make_uint4(wl[2], wl1[2], wh[0], wh1[0]);
         np[4] = make_uint4(wh[1], wh1[1], wh[2], wh1[2]);
+        np[5] = make_uint4(np[5].x, ex[0] << 23, ex[1] << 23, ex[2] << 23);
         float* x = exact + 6 * size_t(node);
         for (int a = 0; a < 3; ++a)
         {
@@ -1552,7 +1557,7 @@ __global__ void kSahSum(const uint4* __restrict__ nodes, uint32_t n, double* sum
     double   c = 0.0;
     if (i < n)
     {
-        const uint4* np = nodes + size_t(i) * 5;
+        const uint4* np = nodes + size_t(i) * kNodeU4;
         uint4        n0 = np[0], n1 = np[1], n2 = np[2], n3 = np[3], n4 = np[4];
         float        px = __uint_as_float(n0.x), py = __uint_as_float(n0.y), pz = __uint_as_float(n0.z);
         float        ex = __uint_as_float((n0.w & 0xffu) << 23), ey = __uint_as_float(((n0.w >> 8) & 0xffu) << 23),

@@ -359,11 +359,11 @@ __device__ __forceinline__ void warpStats(const TraceCounters& tc, unsigned long
     }
 }
 
-// Resident blocks per SM of the traversal kernels.  Flattened scenes: 7
-// (72 registers; 8 blocks at 64 registers was 3% slower on config 2 with the
-// lane refill, 6 blocks the same as 7).  Two-level scenes: 5 (their state is
-// larger; 8 blocks would spill).
-constexpr int kTraceBlocksFlat = 7;
+// Resident blocks per SM of the traversal kernels.  Flattened scenes: 8 (64
+// registers; config 2's 16.6 M paths 42.9 ms, with 7 blocks 43.6, with 6 45.4).
+// Two-level scenes: 5 (their state is larger; 4 blocks 6% slower, 6 blocks
+// equal).
+constexpr int kTraceBlocksFlat = 8;
 constexpr int kTraceBlocksTwo  = 5;
 
 struct ClassifyView
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
                                                                 Counters* ctr, ClassifyView cv)
 {
     extern __shared__ uint2 stack[];
-    __shared__ uint8_t      keyLut[kKeyLutBytes];
+    __shared__ __align__(16) uint8_t keyLut[kLutBytes];
     __shared__ uint2        supply[kTraceBlock / 32];
     const uint32_t   n = waveCount(ctr, count);
     if (n == 0u) return;
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
             if (__all_sync(kFull, ray == kMissPrim)) break;
         }
         if (ray != kMissPrim)
-            for (uint32_t k = 0; k < kRefillSteps; ++k)
+            for (uint32_t k = 0; k < (TWO ? kRefillStepsTwo : kRefillSteps); ++k)
             {
                 bool done;
                 if constexpr (TWO)
@@ -632,7 +632,7 @@ template <bool DL, bool STATS, bool TWO = false>
 __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlocksFlat) kTraceShadow(Params P)
 {
     extern __shared__ uint2 stack[];
-    __shared__ uint8_t      keyLut[kKeyLutBytes];
+    __shared__ __align__(16) uint8_t keyLut[kLutBytes];
     __shared__ uint2        supply[kTraceBlock / 32];
     const uint32_t   n = loadCount(&P.q.ctr->shadowCount) * (DL ? 2u : 1u);
     if (n == 0u) return;
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
             if (__all_sync(kFull, ray == kMissPrim) && ws->x == kMissPrim) break;
         }
         if (ray != kMissPrim)
-            for (uint32_t k = 0; k < kRefillSteps; ++k)
+            for (uint32_t k = 0; k < (TWO ? kRefillStepsTwo : kRefillSteps); ++k)
             {
                 bool done;
                 if constexpr (TWO)
@@ -1135,7 +1135,7 @@ template <int CMP, bool ALIAS, bool TWO>
 __global__ void __launch_bounds__(kTraceBlock, kTailBlocks) kPathTail(Params P, int cur)
 {
     extern __shared__ uint2 stack[];
-    __shared__ uint8_t      keyLut[kKeyLutBytes];
+    __shared__ __align__(16) uint8_t keyLut[kLutBytes];
     __shared__ uint2        supply[kTraceBlock / 32];
     Counters* const  c = P.q.ctr;
     const uint32_t   n = loadCount(&c->rayCount[cur]);
@@ -1250,7 +1250,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTailBlocks) kPathTail(Params P, 
             continue;
         }
         if (state == kTailClosest || state == kTailShadow)
-            for (uint32_t k = 0; k < kRefillSteps; ++k)
+            for (uint32_t k = 0; k < (TWO ? kRefillStepsTwo : kRefillSteps); ++k)
             {
                 bool done;
                 if constexpr (TWO)
@@ -1584,7 +1584,7 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
                                                               uint32_t n, QueryOut out, Counters* ctr)
 {
     extern __shared__ uint2 stack[];
-    __shared__ uint8_t      keyLut[kKeyLutBytes];
+    __shared__ __align__(16) uint8_t keyLut[kLutBytes];
     __shared__ uint2        supply[kTraceBlock / 32];
     fillKeyLut(keyLut);
     TraceCounters tc{0u, 0u};
@@ -1613,7 +1613,7 @@ __global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlo
             if (__all_sync(kFull, ray == kMissPrim)) break;
         }
         if (ray != kMissPrim)
-            for (uint32_t k = 0; k < kRefillSteps; ++k)
+            for (uint32_t k = 0; k < (TWO ? kRefillStepsTwo : kRefillSteps); ++k)
             {
                 bool done;
                 if constexpr (TWO)
@@ -3250,7 +3250,8 @@ cl_status Integrator::getBvh(void* nodes, size_t nodeBytes, void* tris, size_t t
         return CL_ERR_INVALID_ARG;
     }
     CL_CUDA(cudaStreamSynchronize(stream_), err);
-    if (nodes) CL_CUDA(cudaMemcpy(nodes, bvh_.nodes.p, nb, cudaMemcpyDeviceToHost), err);
+    if (nodes) // without a node's last 16 bytes, which repeat the others
+        CL_CUDA(cudaMemcpy2D(nodes, 80, bvh_.nodes.p, kNodeU4 * 16, 80, bvh_.numNodes, cudaMemcpyDeviceToHost), err);
     if (tris) CL_CUDA(cudaMemcpy(tris, bvh_.tris.p, tb, cudaMemcpyDeviceToHost), err);
     return CL_OK;
 }

@@ -122,7 +122,7 @@ private:
 struct WideBvh
 {
     DevBuf     mem;   // holds the four below
-    ScratchBuf nodes; // 5 uint4 per node
+    ScratchBuf nodes; // 6 uint4 per node
     ScratchBuf tris;  // 3 float4 per triangle, leaf order
     ScratchBuf exact; // refit: 6 floats per node, the unquantised box of its triangles
     ScratchBuf scene; // scene bounds (6 ordered ints, refit) and the SAH sum (double at byte 32)
