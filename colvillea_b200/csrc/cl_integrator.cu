@@ -193,16 +193,40 @@ __device__ __forceinline__ HitAttr hitAttributesTri(const SceneDev& sc, uint4 ti
     return h;
 }
 
+// A pixel's random stream.  The column and row come from a multiplication by
+// floor(2^32 / W) (an integer division by a variable takes 25 instructions per
+// vertex): its quotient is the true one or one less, since pix < 2^32.
+__device__ __forceinline__ Rng pixelRng(const WaveParams& wp, uint32_t pix, uint32_t frame, uint32_t ctr)
+{
+    uint32_t y = __umulhi(pix, wp.invW), x = pix - y * wp.W;
+    if (x >= wp.W)
+    {
+        x -= wp.W;
+        ++y;
+    }
+    return Rng{x, y, frame, ctr};
+}
+
 // Camera path start (generateCameraRays, raygeneration.cu:83-102): path index
 // p -> pixel p mod W*H, frame frame0 + p / (W*H).
 __device__ __forceinline__ void startPath(const Params& P, const WaveParams& wp, uint32_t slot, unsigned long long p,
                                           int q, uint32_t idx)
 {
-    unsigned long long wh = (unsigned long long)wp.W * wp.H;
-    uint32_t pix   = uint32_t(p % wh);
-    uint32_t frame = wp.frame0 + uint32_t(p / wh);
-    uint32_t px = pix % wp.W, py = pix / wp.W;
-    Rng      rng{px, py, frame, 0u};
+    const unsigned long long wh = (unsigned long long)wp.W * wp.H;
+    uint32_t pix, frame;
+    if (((p | wh) >> 32) == 0ull)
+    {
+        frame = uint32_t(p) / uint32_t(wh);
+        pix   = uint32_t(p) - frame * uint32_t(wh);
+    }
+    else
+    {
+        pix   = uint32_t(p % wh);
+        frame = uint32_t(p / wh);
+    }
+    frame += wp.frame0;
+    Rng            rng = pixelRng(wp, pix, frame, 0u);
+    const uint32_t px = rng.px, py = rng.py;
     f2       j = rng.next2D();
     f2       screen{(float(px) + j.x) / float(wp.W), (float(py) + j.y) / float(wp.H)};
     f3       pos{wp.cam[0], wp.cam[1], wp.cam[2]}, d00{wp.cam[3], wp.cam[4], wp.cam[5]};
@@ -283,10 +307,7 @@ __device__ __noinline__ void flushCacheRecords(CacheDev c, uint32_t mask, Counte
 // A finished path's radiance into its pixel's sums.
 __device__ __forceinline__ void addToFilm(const Params& P, uint32_t pix, f3 L)
 {
-    float* f = reinterpret_cast<float*>(P.q.film + pix);
-    atomicAdd(f + 0, L.x);
-    atomicAdd(f + 1, L.y);
-    atomicAdd(f + 2, L.z);
+    atomicAdd(P.q.film + pix, make_float4(L.x, L.y, L.z, 0.0f)); // one 16-byte reduction
     if (P.q.film64)
     {
         double* g = P.q.film64 + 6 * size_t(pix);
@@ -299,35 +320,44 @@ __device__ __forceinline__ void addToFilm(const Params& P, uint32_t pix, f3 L)
     }
 }
 
-// Film write of finished paths, then regeneration of their slots.  Called by
-// every lane of the warp.
-__device__ __forceinline__ void finishPaths(const Params& P, const WaveParams& wp, int nxt, bool finish, uint32_t slot,
-                                            f3 L)
+// Film write and training records of a finished path.
+__device__ __forceinline__ void finishPath(const Params& P, const WaveParams& wp, uint32_t slot, uint32_t pix, f3 L)
 {
-    if (finish && wp.recStride && slot % wp.recStride == 0u)
+    if (wp.recStride && slot % wp.recStride == 0u)
         flushRecords(P.g, P.q.psInfo, P.q.ctr, slot, wp.recStride, L.x, L.y, L.z);
-    if (finish && wp.cacheTrain)
+    if (wp.cacheTrain)
     {
         const uint32_t mask = __float_as_uint(P.q.psE[slot].w) & ~kCacheTrainBit;
         if (mask) flushCacheRecords(P.c, mask, P.q.ctr, slot, L.x, L.y, L.z);
     }
-    if (finish) addToFilm(P, P.q.psInfo[slot].x, L);
-    uint32_t mask = __ballot_sync(kFull, finish);
-    if (mask == 0u) return;
-    uint32_t           leader = __ffs(mask) - 1u;
+    addToFilm(P, pix, L);
+}
+
+// Next camera path of each lane whose path has finished (regeneration);
+// returns whether there is one.  Every lane of the warp calls it.
+__device__ __forceinline__ bool nextPath(const Params& P, const WaveParams& wp, bool finish, unsigned long long* path)
+{
+    const uint32_t mask = __ballot_sync(kFull, finish);
+    if (mask == 0u) return false;
+    const uint32_t     leader = __ffs(mask) - 1u;
     unsigned long long base   = 0ull;
     if (laneId() == leader) base = atomicAdd(&P.q.ctr->pathNext, (unsigned long long)__popc(mask));
-    base                  = __shfl_sync(kFull, base, leader);
-    unsigned long long p  = base + __popc(mask & ((1u << laneId()) - 1u));
-    bool               gen = finish && p < wp.totalPaths;
-    uint32_t           idx = warpAppend(&P.q.ctr->rayCount[nxt], gen);
-    if (gen)
-    {
-        if (idx < P.q.slots)
-            startPath(P, wp, slot, p, nxt, idx);
-        else
-            atomicOr(&P.q.ctr->error, 8u);
-    }
+    *path = __shfl_sync(kFull, base, leader) + __popc(mask & ((1u << laneId()) - 1u));
+    return finish && *path < wp.totalPaths;
+}
+
+// Places of the lanes' new rays in queue nxt and of their shadow rays, from one
+// atomicAdd on the queue's two counts per warp.
+__device__ __forceinline__ void appendBoth(Counters* c, int nxt, bool ray, bool shadow, uint32_t* rIdx, uint32_t* sIdx)
+{
+    const uint32_t     rm = __ballot_sync(kFull, ray), sm = __ballot_sync(kFull, shadow), lt = (1u << laneId()) - 1u;
+    unsigned long long base = 0ull;
+    if ((rm | sm) == 0u) return;
+    if (laneId() == 0u)
+        base = atomicAdd(&c->queued[nxt], (unsigned long long)__popc(rm) | ((unsigned long long)__popc(sm) << 32));
+    base  = __shfl_sync(kFull, base, 0);
+    *rIdx = uint32_t(base) + __popc(rm & lt);
+    *sIdx = uint32_t(base >> 32) + __popc(sm & lt);
 }
 
 __device__ __forceinline__ f3 ld3(float4 v) { return {v.x, v.y, v.z}; }
@@ -629,12 +659,12 @@ __global__ void __launch_bounds__(kClassifyThreads) kClassifyHits(BvhView bvh, f
 // tracing) or ray k&1 of entry k>>1 (direct lighting, two rays per entry).
 // vis[k] = 1 when the ray reaches its light, 0 otherwise.
 template <bool DL, bool STATS, bool TWO = false>
-__global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlocksFlat) kTraceShadow(Params P)
+__global__ void __launch_bounds__(kTraceBlock, TWO ? kTraceBlocksTwo : kTraceBlocksFlat) kTraceShadow(Params P, int cur)
 {
     extern __shared__ uint2 stack[];
     __shared__ __align__(16) uint8_t keyLut[kLutBytes];
     __shared__ uint2        supply[kTraceBlock / 32];
-    const uint32_t   n = loadCount(&P.q.ctr->shadowCount) * (DL ? 2u : 1u);
+    const uint32_t   n = loadCount(P.q.ctr->shadowCount(cur)) * (DL ? 2u : 1u);
     if (n == 0u) return;
     fillKeyLut(keyLut);
     TraceCounters    tc{0u, 0u};
@@ -984,6 +1014,7 @@ __global__ void __launch_bounds__(128) kShade(Params P, int cur)
         uint32_t    i = base + laneId();
         const bool  valid = i < n;
         VertexState v{};
+        uint32_t    pix = 0u;
         if (valid)
         {
             i             = P.q.classIdx[size_t(MAT) * P.q.slots + i];
@@ -997,7 +1028,8 @@ __global__ void __launch_bounds__(128) kShade(Params P, int cur)
             if constexpr (MAT != kClassEscaped) a0 = hitAttributesTri(sc, ti, hh.z, hh.w);
             uint4  info = P.q.psInfo[v.slot];
             v.depth     = info.z & 0xffu;
-            Rng    rng{info.x % wp.W, info.x / wp.W, info.y, info.z >> 8};
+            pix         = info.x;
+            Rng    rng  = pixelRng(wp, info.x, info.y, info.z >> 8);
             v.T         = ld3(P.q.psT[v.slot]);
             float4 e4   = P.q.psE[v.slot];
             v.E         = ld3(e4);
@@ -1007,8 +1039,18 @@ __global__ void __launch_bounds__(128) kShade(Params P, int cur)
             shadeVertex<DL, CMP, ALIAS, MAT, GUIDE>(P, wp, v, rng, i, hh, ti, a0);
         }
         const bool pushShadow = v.shadow1 || v.shadow2;
+        const bool ended = v.finish && !pushShadow;
+        if (ended) finishPath(P, wp, v.slot, pix, v.L);
+        unsigned long long path = 0ull;
+        const bool         gen  = nextPath(P, wp, ended, &path);
+        uint32_t           rIdx = 0u, sIdx = 0u;
+        appendBoth(P.q.ctr, nxt, v.pushRay || gen, pushShadow, &rIdx, &sIdx);
+        if ((v.pushRay || gen) && rIdx >= P.q.slots)
+        {
+            atomicOr(&P.q.ctr->error, 8u);
+            continue;
+        }
         // Shadow queue (one entry per path vertex).
-        uint32_t sIdx = warpAppend(&P.q.ctr->shadowCount, pushShadow);
         if (pushShadow)
         {
             if (sIdx < P.q.shadowCap)
@@ -1027,12 +1069,6 @@ __global__ void __launch_bounds__(128) kShade(Params P, int cur)
                 atomicOr(&P.q.ctr->error, 4u);
         }
         // Next-bounce ray queue.
-        uint32_t rIdx = warpAppend(&P.q.ctr->rayCount[nxt], v.pushRay);
-        if (v.pushRay && rIdx >= P.q.slots)
-        {
-            atomicOr(&P.q.ctr->error, 8u);
-            v.pushRay = false;
-        }
         if (v.pushRay)
         {
             P.q.rqO[nxt][rIdx]    = make_float4(v.pHit.x, v.pHit.y, v.pHit.z, kRayEps);
@@ -1044,7 +1080,7 @@ __global__ void __launch_bounds__(128) kShade(Params P, int cur)
             P.q.psE[v.slot]         = make_float4(v.E.x, v.E.y, v.E.z, __uint_as_float(v.cst));
         }
         if (v.pushRay || (pushShadow && v.finish)) P.q.psL[v.slot] = make_float4(v.L.x, v.L.y, v.L.z, 0.0f);
-        finishPaths(P, wp, nxt, v.finish && !pushShadow, v.slot, v.L);
+        if (gen) startPath(P, wp, v.slot, path, nxt, rIdx);
     }
 }
 
@@ -1054,7 +1090,7 @@ template <bool DL>
 __global__ void __launch_bounds__(128) kShadowResolve(Params P, int cur)
 {
     const WaveParams wp  = *P.wp;
-    const uint32_t   n   = loadCount(&P.q.ctr->shadowCount);
+    const uint32_t   n   = loadCount(P.q.ctr->shadowCount(cur));
     const int        nxt = cur ^ 1;
     const uint32_t gw = gridDim.x * (blockDim.x >> 5); // static 32-entry batches, as in kShade
     for (uint32_t base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32u; base < n; base += gw * 32u)
@@ -1085,7 +1121,18 @@ __global__ void __launch_bounds__(128) kShadowResolve(Params P, int cur)
             else
                 P.q.psL[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         }
-        finishPaths(P, wp, nxt, finish, slot, L);
+        if (finish) finishPath(P, wp, slot, P.q.psInfo[slot].x, L);
+        unsigned long long path = 0ull;
+        const bool         gen  = nextPath(P, wp, finish, &path);
+        uint32_t           rIdx = 0u, sIdx = 0u;
+        appendBoth(P.q.ctr, nxt, gen, false, &rIdx, &sIdx);
+        if (gen)
+        {
+            if (rIdx < P.q.slots)
+                startPath(P, wp, slot, path, nxt, rIdx);
+            else
+                atomicOr(&P.q.ctr->error, 8u);
+        }
     }
     // The last block to end empties the shadow queue for this wave's vertices
     // (every block has read its count by then).
@@ -1097,7 +1144,7 @@ __global__ void __launch_bounds__(128) kShadowResolve(Params P, int cur)
         if (atomicAdd(&c->resolveBlocks, 1u) == gridDim.x - 1u)
         {
             c->raysShadow += n;
-            c->shadowCount   = 0u;
+            *c->shadowCount(cur) = 0u;
             c->fetchShadow   = 0u;
             c->resolveBlocks = 0u;
         }
@@ -1138,7 +1185,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTailBlocks) kPathTail(Params P, 
     __shared__ __align__(16) uint8_t keyLut[kLutBytes];
     __shared__ uint2        supply[kTraceBlock / 32];
     Counters* const  c = P.q.ctr;
-    const uint32_t   n = loadCount(&c->rayCount[cur]);
+    const uint32_t   n = loadCount(c->rayCount(cur));
     const WaveParams wp = *P.wp;
     if (n == 0u || !loadCount(&c->tailNow)) return; // the same in every block
     fillKeyLut(keyLut);
@@ -1217,7 +1264,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTailBlocks) kPathTail(Params P, 
                 const uint4  info = P.q.psInfo[v.slot];
                 const float4 e4   = P.q.psE[v.slot];
                 pix               = info.x;
-                rng               = Rng{info.x % wp.W, info.x / wp.W, info.y, info.z >> 8};
+                rng               = pixelRng(wp, info.x, info.y, info.z >> 8);
                 v.depth           = info.z & 0xffu;
                 v.T               = ld3(P.q.psT[v.slot]);
                 v.E               = ld3(e4);
@@ -1281,9 +1328,9 @@ __global__ void __launch_bounds__(kTraceBlock, kTailBlocks) kPathTail(Params P, 
         __threadfence();
         if (atomicAdd(&c->tailBlocks, 1u) == gridDim.x - 1u)
         {
-            c->rayCount[cur] = 0u;
-            c->fetchTrace    = 0u;
-            c->tailBlocks    = 0u;
+            *c->rayCount(cur) = 0u;
+            c->fetchTrace     = 0u;
+            c->tailBlocks     = 0u;
         }
     }
 }
@@ -1553,10 +1600,10 @@ __global__ void kAdvance(Counters* c, const WaveParams* wp, int cur)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     if (c->pathNext >= wp->totalPaths) c->drained += 1u;
-    c->raysClosest += c->rayCount[cur];
-    c->rayCount[cur] = 0u;
+    c->raysClosest += *c->rayCount(cur);
+    *c->rayCount(cur) = 0u;
     c->fetchTrace    = 0u;
-    const uint32_t n = c->rayCount[cur ^ 1];
+    const uint32_t n = *c->rayCount(cur ^ 1);
     c->tailNow       = n > 0u && n <= wp->tailMax && c->drained >= wp->tailNeed ? 1u : 0u;
     c->fetchInfer    = 0u;
     c->cacheCount    = 0u;
@@ -2601,11 +2648,11 @@ cl_status Integrator::launchWave(int cur, bool profile, std::string* err)
     {
         auto k = st ? (twoLevel_ ? kTraceClosest<true, true> : kTraceClosest<true, false>)
                     : (twoLevel_ ? kTraceClosest<false, true> : kTraceClosest<false, false>);
-        k<<<tBlocks(), kTraceBlock, sb, stream_>>>(P.sc.bvh, P.q.rqO[cur], P.q.rqD[cur], &c->rayCount[cur],
+        k<<<tBlocks(), kTraceBlock, sb, stream_>>>(P.sc.bvh, P.q.rqO[cur], P.q.rqD[cur], c->rayCount(cur),
                                                       &c->fetchTrace, P.q.hit, c, classifyView());
         if (profile) CL_CUDA(cudaEventRecord(evS_[5], stream_), err);
         (twoLevel_ ? kClassifyHits<true> : kClassifyHits<false>)<<<numSMs_ * 8, kClassifyThreads, 0, stream_>>>(
-            P.sc.bvh, P.q.hit, &c->rayCount[cur], c, classifyView());
+            P.sc.bvh, P.q.hit, c->rayCount(cur), c, classifyView());
     }
     if (profile) CL_CUDA(cudaEventRecord(evS_[1], stream_), err);
     const uint32_t gmask = guide_ ? guideCfg_.class_mask : 0u;
@@ -2624,13 +2671,13 @@ cl_status Integrator::launchWave(int cur, bool profile, std::string* err)
     {
         cudaStream_t sh = profile ? stream_ : shadowStream_;
         if (!profile) CL_CUDA(cudaStreamWaitEvent(sh, evFork_, 0), err);
-        using ShadowFn = void (*)(Params);
+        using ShadowFn = void (*)(Params, int);
         const ShadowFn table[2][2][2] = {
             {{kTraceShadow<false, false, false>, kTraceShadow<false, false, true>},
              {kTraceShadow<false, true, false>, kTraceShadow<false, true, true>}},
             {{kTraceShadow<true, false, false>, kTraceShadow<true, false, true>},
              {kTraceShadow<true, true, false>, kTraceShadow<true, true, true>}}};
-        table[dl][st][twoLevel_]<<<tBlocks(), kTraceBlock, sb, sh>>>(P);
+        table[dl][st][twoLevel_]<<<tBlocks(), kTraceBlock, sb, sh>>>(P, cur);
         if (dl)
             kShadowResolve<true><<<shadowBlocks_, 128, 0, sh>>>(P, cur);
         else
@@ -2794,6 +2841,7 @@ cl_status Integrator::beginPass(uint32_t spp, bool record, bool cacheTrain, uint
     WaveParams& wp = *hostWp_;
     wp.W           = W_;
     wp.H           = H_;
+    wp.invW        = uint32_t(std::min<uint64_t>((1ull << 32) / W_, 0xffffffffull));
     wp.frame0      = iteration_;
     wp.maxDepth    = dl ? 1u : cfg_.max_depth;
     wp.rrStart     = cfg_.rr_start_depth;
@@ -2808,7 +2856,7 @@ cl_status Integrator::beginPass(uint32_t spp, bool record, bool cacheTrain, uint
     CL_CUDA(cudaMemcpyAsync(wp_.p, hostWp_, sizeof(WaveParams), cudaMemcpyHostToDevice, stream_), err);
     uint32_t init = uint32_t(std::min<unsigned long long>(slots_, wp.totalPaths));
     Counters c0{};
-    c0.rayCount[0] = init;
+    c0.queued[0]   = init;
     c0.pathNext    = init;
     c0.drained     = init == wp.totalPaths ? 1u : 0u;
     // A pass whose camera rays already fit the tail launch needs no wave.
@@ -2878,9 +2926,9 @@ cl_status Integrator::renderPass(uint32_t spp, bool record, bool cacheTrain, std
         else
             CL_CUDA(cudaGraphLaunch(graph_, stream_), err);
         waves_ += 4;
-        CL_CUDA(cudaMemcpyAsync(hostCount_, &dc->rayCount[0], 12, cudaMemcpyDeviceToHost, stream_), err);
+        CL_CUDA(cudaMemcpyAsync(hostCount_, &dc->queued[0], 8, cudaMemcpyDeviceToHost, stream_), err);
         CL_CUDA(cudaStreamSynchronize(stream_), err);
-        if (hostCount_[0] == 0u && hostCount_[2] == 0u) break; // no ray, no shadow ray
+        if (hostCount_[0] == 0u && hostCount_[1] == 0u) break; // no ray, no shadow ray
     }
     CL_CUDA(cudaEventRecord(evB_, stream_), err);
     Counters ch;
@@ -3423,9 +3471,9 @@ cl_status Integrator::guideProbe(uint32_t cap, float* rows, uint32_t* count, std
     kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(P, init);
     (twoLevel_ ? kTraceClosest<false, true> : kTraceClosest<false, false>)
         <<<tBlocks(), kTraceBlock, traceStackBytes(P.sc.bvh.stackDepth), stream_>>>(
-            P.sc.bvh, P.q.rqO[0], P.q.rqD[0], &c->rayCount[0], &c->fetchTrace, P.q.hit, c, classifyView());
+            P.sc.bvh, P.q.rqO[0], P.q.rqD[0], c->rayCount(0), &c->fetchTrace, P.q.hit, c, classifyView());
     (twoLevel_ ? kClassifyHits<true> : kClassifyHits<false>)<<<numSMs_ * 8, kClassifyThreads, 0, stream_>>>(
-        P.sc.bvh, P.q.hit, &c->rayCount[0], c, classifyView());
+        P.sc.bvh, P.q.hit, c->rayCount(0), c, classifyView());
     kGuideInfer<<<inferBlocks_, guide::kTcThreads, kGuideMlpSmem, stream_>>>(
         P, guide_->grid(), 0, guide_->tcWeights(), guideCfg_.learn_selection ? -1.0f : 1.0f - guideCfg_.bsdf_fraction);
     CL_CUDA(cudaGetLastError(), err);

@@ -50,13 +50,14 @@ struct WaveParams
     unsigned long long totalPaths;
     float              cam[12];
     uint32_t           tailNeed;   // and Counters::drained has reached this
-    uint32_t           pad3;
+    uint32_t           invW;       // floor(2^32 / W), at most 2^32 - 1
 };
 
 struct Counters
 {
-    uint32_t           rayCount[2];
-    uint32_t           shadowCount;
+    // Entries of ray queue q (low word) and of the shadow queue that was filled
+    // with it (high word): the shading of a wave appends to both with one atomic.
+    unsigned long long queued[2];
     uint32_t           fetchTrace, fetchShadow; // traversal kernels' ray supplies
     uint32_t           error;
     uint32_t           classCount[4]; // per shading class: diffuse, conductor, dielectric, escaped
@@ -76,6 +77,9 @@ struct Counters
     uint32_t           tailNow;    // kPathTail takes the next wave's queue
     uint32_t           resolveBlocks; // blocks of kShadowResolve that have ended
     unsigned long long cacheQueries; // radiance cache: network evaluations
+
+    __host__ __device__ uint32_t* rayCount(int q) { return reinterpret_cast<uint32_t*>(queued + q); }
+    __host__ __device__ uint32_t* shadowCount(int q) { return reinterpret_cast<uint32_t*>(queued + q) + 1; }
 };
 
 struct QueueDev
