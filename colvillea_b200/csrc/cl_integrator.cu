@@ -1587,13 +1587,19 @@ __global__ void kClampCacheRecords(Counters* c, uint32_t cap)
     if (threadIdx.x == 0 && blockIdx.x == 0) c->cacheTrainCount = min(c->cacheRec, cap);
 }
 
-// Initial fill: slot s starts path s.
-__global__ void kRaygen(Params P, uint32_t count)
+// Initial fill: slot s starts path s.  The pass's parameters and first counters
+// arrive as kernel arguments and are left in device memory for the waves
+// (instead of two copies and a wait before every pass).
+__global__ void kRaygen(Params P, const __grid_constant__ WaveParams wp, const __grid_constant__ Counters c0,
+                        WaveParams* wpOut, uint32_t count)
 {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= count) return;
-    const WaveParams wp = *P.wp;
-    startPath(P, wp, s, s, 0, s);
+    if (s == 0u)
+    {
+        *wpOut   = wp;
+        *P.q.ctr = c0;
+    }
+    if (s < count) startPath(P, wp, s, s, 0, s);
 }
 
 __global__ void kAdvance(Counters* c, const WaveParams* wp, int cur)
@@ -1790,8 +1796,7 @@ Integrator::~Integrator()
     if (evB_) cudaEventDestroy(evB_);
     for (auto& e : evS_)
         if (e) cudaEventDestroy(e);
-    if (hostWp_) cudaFreeHost(hostWp_);
-    if (hostCount_) cudaFreeHost(hostCount_);
+    if (hostCtr_) cudaFreeHost(hostCtr_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -1822,8 +1827,8 @@ cl_status Integrator::init(std::string* err)
     CL_CUDA(cudaEventCreate(&evA_), err);
     CL_CUDA(cudaEventCreate(&evB_), err);
     for (auto& e : evS_) CL_CUDA(cudaEventCreate(&e), err);
-    CL_CUDA(cudaMallocHost((void**)&hostWp_, sizeof(WaveParams)), err);
-    CL_CUDA(cudaMallocHost((void**)&hostCount_, 64), err);
+    CL_CUDA(cudaMallocHost((void**)&hostCtr_, sizeof(Counters) + 64), err);
+    hostCount_ = reinterpret_cast<uint32_t*>(hostCtr_ + 1);
     int b = 0;
     // Occupancy at the deepest supported stack (the launches use less).
     CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTraceClosest<false, false>, kTraceBlock,
@@ -2838,7 +2843,7 @@ cl_status Integrator::beginPass(uint32_t spp, bool record, bool cacheTrain, uint
                                 std::string* err)
 {
     const bool  dl = type_ == CL_INTEGRATOR_DIRECT_LIGHTING;
-    WaveParams& wp = *hostWp_;
+    WaveParams& wp = passWp_;
     wp.W           = W_;
     wp.H           = H_;
     wp.invW        = uint32_t(std::min<uint64_t>((1ull << 32) / W_, 0xffffffffull));
@@ -2853,19 +2858,26 @@ cl_status Integrator::beginPass(uint32_t spp, bool record, bool cacheTrain, uint
     wp.tailMax     = usesTail() ? kTailMaxRays : 0u;
     wp.tailNeed    = cache_ ? cacheCfg_.prefix_bounces + 2u : 1u;
     memcpy(wp.cam, &camera_, sizeof(camera_));
-    CL_CUDA(cudaMemcpyAsync(wp_.p, hostWp_, sizeof(WaveParams), cudaMemcpyHostToDevice, stream_), err);
-    uint32_t init = uint32_t(std::min<unsigned long long>(slots_, wp.totalPaths));
-    Counters c0{};
+    uint32_t  init = uint32_t(std::min<unsigned long long>(slots_, wp.totalPaths));
+    Counters& c0   = passCtr_;
+    c0             = Counters{};
     c0.queued[0]   = init;
     c0.pathNext    = init;
     c0.drained     = init == wp.totalPaths ? 1u : 0u;
     // A pass whose camera rays already fit the tail launch needs no wave.
     c0.tailNow     = c0.drained && init <= wp.tailMax && wp.tailNeed <= 1u ? 1u : 0u;
     *tailOnly      = c0.tailNow != 0u;
-    CL_CUDA(cudaMemcpyAsync(ctr_.p, &c0, sizeof(Counters), cudaMemcpyHostToDevice, stream_), err);
-    CL_CUDA(cudaStreamSynchronize(stream_), err); // hostWp_/c0 reused next call
     waveRaysSeen_ = 0ull;
     *initSlots    = init;
+    return CL_OK;
+}
+
+// Waits for the pass so far: its end time (evB_) and its counters.
+cl_status Integrator::fetchCounters(std::string* err)
+{
+    CL_CUDA(cudaEventRecord(evB_, stream_), err);
+    CL_CUDA(cudaMemcpyAsync(hostCtr_, ctr_.p, sizeof(Counters), cudaMemcpyDeviceToHost, stream_), err);
+    CL_CUDA(cudaStreamSynchronize(stream_), err);
     return CL_OK;
 }
 
@@ -2875,10 +2887,10 @@ cl_status Integrator::renderPass(uint32_t spp, bool record, bool cacheTrain, std
     uint32_t   init    = 0u;
     bool       tailOnly = false;
     CL_TRY(beginPass(spp, record, cacheTrain, &init, &tailOnly, err));
-    const WaveParams& wp = *hostWp_;
+    const WaveParams& wp = passWp_;
 
     CL_CUDA(cudaEventRecord(evA_, stream_), err);
-    kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(params(), init);
+    kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(params(), passWp_, passCtr_, wp_.as<WaveParams>(), init);
     CL_CUDA(cudaGetLastError(), err);
     if (tailOnly)
     {
@@ -2926,15 +2938,12 @@ cl_status Integrator::renderPass(uint32_t spp, bool record, bool cacheTrain, std
         else
             CL_CUDA(cudaGraphLaunch(graph_, stream_), err);
         waves_ += 4;
-        CL_CUDA(cudaMemcpyAsync(hostCount_, &dc->queued[0], 8, cudaMemcpyDeviceToHost, stream_), err);
-        CL_CUDA(cudaStreamSynchronize(stream_), err);
-        if (hostCount_[0] == 0u && hostCount_[1] == 0u) break; // no ray, no shadow ray
+        CL_TRY(fetchCounters(err));
+        if (hostCtr_->queued[0] == 0ull) break; // no ray, no shadow ray
     }
-    CL_CUDA(cudaEventRecord(evB_, stream_), err);
-    Counters ch;
-    CL_CUDA(cudaMemcpyAsync(&ch, ctr_.p, sizeof(Counters), cudaMemcpyDeviceToHost, stream_), err);
-    CL_CUDA(cudaEventSynchronize(evB_), err);
-    float msPass = 0.0f;
+    if (tailOnly) CL_TRY(fetchCounters(err));
+    const Counters& ch = *hostCtr_;
+    float           msPass = 0.0f;
     CL_CUDA(cudaEventElapsedTime(&msPass, evA_, evB_), err);
     msRender_ += msPass;
     if (ch.error)
@@ -3468,7 +3477,7 @@ cl_status Integrator::guideProbe(uint32_t cap, float* rows, uint32_t* count, std
     P.g.probe      = probe.f();
     P.g.probeCap   = cap;
     Counters* c    = ctr_.as<Counters>();
-    kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(P, init);
+    kRaygen<<<(init + 255) / 256, 256, 0, stream_>>>(P, passWp_, passCtr_, wp_.as<WaveParams>(), init);
     (twoLevel_ ? kTraceClosest<false, true> : kTraceClosest<false, false>)
         <<<tBlocks(), kTraceBlock, traceStackBytes(P.sc.bvh.stackDepth), stream_>>>(
             P.sc.bvh, P.q.rqO[0], P.q.rqD[0], c->rayCount(0), &c->fetchTrace, P.q.hit, c, classifyView());
