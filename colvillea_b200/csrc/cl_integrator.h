@@ -216,6 +216,7 @@ private:
     cl_status clearFilm(std::string* err);
     cl_status captureGraph(std::string* err);
     cl_status launchWave(int cur, bool profile, std::string* err);
+    cl_status fetchCounters(std::string* err);
     bool      usesTail() const;
     cl_status launchTail(int cur, cudaStream_t st, std::string* err);
     Params    params() const;
@@ -287,8 +288,10 @@ private:
     ScratchBuf rqO_[2], rqD_[2], rqSlot_[2], hit_, hitIdx_, hitInst_, sqO_, sqD_, sqL_, sqD2_, sqL2_;
     ScratchBuf psInfo_, psT_, psE_, psL_, vis_, classIdx_;
     uint32_t slots_ = 0, shadowCap_ = 0;
-    WaveParams* hostWp_ = nullptr;   // pinned
-    uint32_t*   hostCount_ = nullptr; // pinned
+    WaveParams passWp_{};             // the current pass's parameters
+    Counters   passCtr_{};            // and first counters
+    Counters*  hostCtr_   = nullptr;  // page-locked: counters read back
+    uint32_t*  hostCount_ = nullptr;  // page-locked, 16 words: training counts
     cudaGraphExec_t graph_ = nullptr;
     bool            graphValid_ = false;
 
