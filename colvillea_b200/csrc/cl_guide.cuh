@@ -240,17 +240,35 @@ __device__ __forceinline__ void headLobes(const float* o, Lobes* L, float alpha 
 }
 
 // vMF density kappa / (2 pi (1 - e^{-2 kappa})) e^{kappa (mu.d - 1)}.
-__device__ __forceinline__ float vmfPdf(float4 l, f3 d)
+__device__ __forceinline__ float vmfNorm(float kappa) { return kappa / (2.0f * kPiF * -expm1f(-2.0f * kappa)); }
+__device__ __forceinline__ float vmfPdf(float4 l, f3 d, float norm)
 {
     float c = l.x * d.x + l.y * d.y + l.z * d.z;
-    return l.w / (2.0f * kPiF * -expm1f(-2.0f * l.w)) * expf(l.w * (c - 1.0f));
+    return norm * expf(l.w * (c - 1.0f));
 }
+__device__ __forceinline__ float vmfPdf(float4 l, f3 d) { return vmfPdf(l, d, vmfNorm(l.w)); }
 
 __device__ __forceinline__ float mixturePdf(const Lobes& L, f3 d)
 {
     float p = 0.0f;
 #pragma unroll
     for (int k = 0; k < kLobes; ++k) p = fmaf(L.w[k], vmfPdf(L.l[k], d), p);
+    return p;
+}
+
+// The same over a ray's stored lobes {mu, kappa} x 8, weights 0-3, 4-7, norms 0-3, 4-7.
+__device__ __forceinline__ float mixturePdf(const float4* __restrict__ lb, f3 d)
+{
+    float p = 0.0f;
+#pragma unroll 2
+    for (int k = 0; k < kLobes; k += 4)
+    {
+        const float4 w = lb[kLobes + k / 4], n = lb[kLobes + 2 + k / 4];
+        p = fmaf(w.x, vmfPdf(lb[k], d, n.x), p);
+        p = fmaf(w.y, vmfPdf(lb[k + 1], d, n.y), p);
+        p = fmaf(w.z, vmfPdf(lb[k + 2], d, n.z), p);
+        p = fmaf(w.w, vmfPdf(lb[k + 3], d, n.w), p);
+    }
     return p;
 }
 
@@ -267,6 +285,21 @@ __device__ __forceinline__ void onb(f3 n, f3* t, f3* b)
 // Lobe by u0 in [0, sum of weights) over the weights' CDF; direction by
 // Jakob's inversion (2012):
 // w = 1 + log(u1 + (1 - u1) e^{-2 kappa}) / kappa, phi = 2 pi u2.
+__device__ __forceinline__ f3 lobeSample(float4 l, float u1, float u2);
+__device__ __forceinline__ f3 mixtureSample(const float4* __restrict__ lb, float u0, float u1, float u2)
+{
+    const float4 w0 = lb[kLobes], w1 = lb[kLobes + 1];
+    const float  w[kLobes] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+    int   k   = kLobes - 1;
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kLobes; ++j)
+    {
+        acc += w[j];
+        if (u0 < acc && k == kLobes - 1 && j < kLobes - 1) k = j;
+    }
+    return lobeSample(lb[k], u1, u2);
+}
 __device__ __forceinline__ f3 mixtureSample(const Lobes& L, float u0, float u1, float u2)
 {
     int   k   = kLobes - 1;
@@ -282,6 +315,10 @@ __device__ __forceinline__ f3 mixtureSample(const Lobes& L, float u0, float u1, 
 #pragma unroll
     for (int j = 1; j < kLobes; ++j)
         if (j == k) l = L.l[j];
+    return lobeSample(l, u1, u2);
+}
+__device__ __forceinline__ f3 lobeSample(float4 l, float u1, float u2)
+{
     float kap = l.w;
     float w   = 1.0f + logf(u1 + (1.0f - u1) * expf(-2.0f * kap)) / kap;
     w         = fminf(fmaxf(w, -1.0f), 1.0f);

@@ -811,28 +811,18 @@ __device__ __forceinline__ void shadeVertex(const Params& P, const WaveParams& w
         if (MAT >= 0) bsdf.type = uint32_t(MAT);
         pHit         = a.p;
         f3    wo     = -d;
-        guide::Lobes G;
         float        gf = 1.0f; // probability of BSDF sampling: 1 - sum of the lobe weights
         // Vertices shallower than the guide's minimum depth were not inferred, and near-specular
         // ones (GGX alpha below the guide's minimum) are not guided: BSDF sampling alone (zero
         // lobe weights), no training record.
         const bool guided =
             GUIDE && depth >= P.g.minDepth && (bsdf.type == kDiffuse || bsdf.alpha >= P.g.minAlpha);
-        if (GUIDE && !guided)
-#pragma unroll
-            for (int k = 0; k < guide::kLobes; ++k)
-            {
-                G.l[k] = make_float4(0.0f, 0.0f, 1.0f, 1.0f);
-                G.w[k] = 0.0f;
-            }
+        // The lobes stay in memory (L1 after the first pass over them): held in
+        // registers they cost a block per SM.
+        const float4* lb = P.g.lobes + size_t(i) * kLobeF4;
         if (guided)
         {
-            const float4* lb = P.g.lobes + size_t(i) * kLobeF4;
-#pragma unroll
-            for (int k = 0; k < guide::kLobes; ++k) G.l[k] = lb[k];
-            float4 w0 = lb[8], w1 = lb[9];
-            G.w[0] = w0.x, G.w[1] = w0.y, G.w[2] = w0.z, G.w[3] = w0.w;
-            G.w[4] = w1.x, G.w[5] = w1.y, G.w[6] = w1.z, G.w[7] = w1.w;
+            const float4 w0 = lb[8], w1 = lb[9];
             gf = 1.0f - (((w0.x + w0.y) + (w0.z + w0.w)) + ((w1.x + w1.y) + (w1.z + w1.w)));
         }
         f2    u      = rng.next2D();
@@ -870,7 +860,7 @@ __device__ __forceinline__ void shadeVertex(const Params& P, const WaveParams& w
                 if (nonzero(f))
                 {
                     float bp = bsdfPdf(bsdf, woL, wiL, compatPdf);
-                    if (GUIDE) bp = gf * bp + guide::mixturePdf(G, ldir);
+                    if (guided) bp = gf * bp + guide::mixturePdf(lb, ldir);
                     float c  = (DL && compatEsc) ? wiL.z : fabsf(wiL.z);
                     f3    baseV = DL ? value : T * value;
                     float w, pl;
@@ -905,7 +895,7 @@ __device__ __forceinline__ void shadeVertex(const Params& P, const WaveParams& w
             f = bsdfSample(bsdf, woL, u2, &wiL, &bp);
         else
         {
-            gdir = guide::mixtureSample(G, us - gf, u2.x, u2.y);
+            gdir = guide::mixtureSample(lb, us - gf, u2.x, u2.y);
             wiL  = fr.toLocal(gdir);
             f    = bsdfEval(bsdf, woL, wiL);
             bp   = bsdfPdf(bsdf, woL, wiL, false);
@@ -914,7 +904,7 @@ __device__ __forceinline__ void shadeVertex(const Params& P, const WaveParams& w
         if (GUIDE && nonzero(f))
         {
             if (us < gf) gdir = fr.toWorld(wiL);
-            bp = gf * bp + guide::mixturePdf(G, gdir);
+            if (guided) bp = gf * bp + guide::mixturePdf(lb, gdir);
         }
         // The corrected estimator stops paths whose sampled pdf is not
         // positive (0 or NaN at the rim of the cosine warp); the
@@ -1488,6 +1478,8 @@ __global__ void __launch_bounds__(guide::kTcThreads) kGuideInfer(Params P, guide
             for (int j = 0; j < kLobes; ++j) dst[j] = L.l[j];
             dst[8] = make_float4(L.w[0], L.w[1], L.w[2], L.w[3]);
             dst[9] = make_float4(L.w[4], L.w[5], L.w[6], L.w[7]);
+            dst[10] = make_float4(vmfNorm(L.l[0].w), vmfNorm(L.l[1].w), vmfNorm(L.l[2].w), vmfNorm(L.l[3].w));
+            dst[11] = make_float4(vmfNorm(L.l[4].w), vmfNorm(L.l[5].w), vmfNorm(L.l[6].w), vmfNorm(L.l[7].w));
             if (probe)
             {
                 float* q = P.g.probe + size_t(k) * kProbeF;
@@ -1495,7 +1487,7 @@ __global__ void __launch_bounds__(guide::kTcThreads) kGuideInfer(Params P, guide
                 for (int j = 0; j < 9; ++j) q[j] = in9[j];
                 q[9] = __uint_as_float(ray);
 #pragma unroll
-                for (int j = 0; j < kLobeF4; ++j)
+                for (int j = 0; j < 10; ++j)
                 {
                     const float4 v = dst[j];
                     q[10 + 4 * j]  = v.x;
@@ -1843,6 +1835,11 @@ cl_status Integrator::init(std::string* err)
     CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void*)shadeKernel(dl, 2, cfg_.flags), 128, 0),
             err);
     shadeBlocks_ = std::max(1, b) * numSMs_;
+    // Guided kernels hold fewer blocks per SM: a grid of the others' size would
+    // run its static batches in a full and a mostly empty round.
+    CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void*)shadeKernel(dl, 2, cfg_.flags, true), 128, 0),
+            err);
+    shadeBlocksGuided_ = std::max(1, b) * numSMs_;
     CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &b, dl ? (const void*)kShadowResolve<true> : (const void*)kShadowResolve<false>, 128, 0),
             err);
@@ -2700,7 +2697,8 @@ cl_status Integrator::launchWave(int cur, bool profile, std::string* err)
     {
         cudaStream_t s = profile || m == 3 ? stream_ : shadeStream_[m];
         if (s != stream_) CL_CUDA(cudaStreamWaitEvent(s, evFork_, 0), err);
-        shadeKernel(dl, m, cfg_.flags, m < 3 && ((gmask >> m) & 1u))<<<shadeBlocks_, 128, 0, s>>>(P, cur);
+        const bool guided = m < 3 && ((gmask >> m) & 1u);
+        shadeKernel(dl, m, cfg_.flags, guided)<<<guided ? shadeBlocksGuided_ : shadeBlocks_, 128, 0, s>>>(P, cur);
         if (s != stream_) CL_CUDA(cudaEventRecord(evJoin_[m], s), err);
     }
     for (int m = 0; m < 3 && !profile; ++m) CL_CUDA(cudaStreamWaitEvent(stream_, evJoin_[m], 0), err);

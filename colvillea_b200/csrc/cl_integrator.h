@@ -109,7 +109,7 @@ struct QueueDev
 
 // Guided path tracing: per-ray mixtures, per-slot vertex histories and the
 // training records (no counterpart in the reference).
-constexpr int kLobeF4 = 10; // 8 x {mu, kappa}, weights 0-3, weights 4-7
+constexpr int kLobeF4 = 12; // 8 x {mu, kappa}, weights 0-3, 4-7, density norms 0-3, 4-7
 constexpr int kProbeF = 52; // floats per probed guide row
 constexpr int kHistF4 = 5;  // {p, T.x} {n, T.y} {wo, T.z} {omega, BSDF pdf} {L snapshot, -}
 struct GuideDev
@@ -228,7 +228,7 @@ private:
     cl_render_config   cfg_;
     cudaStream_t       stream_ = nullptr;
     int                numSMs_ = 148;
-    int                traceBlocks_ = 0, shadeBlocks_ = 0, shadowBlocks_ = 0, traceBlocksTwo_ = 0;
+    int                traceBlocks_ = 0, shadeBlocks_ = 0, shadeBlocksGuided_ = 0, shadowBlocks_ = 0, traceBlocksTwo_ = 0;
     int                tailBlocks_[2] = {0, 0};
     int                tBlocks() const { return twoLevel_ ? traceBlocksTwo_ : traceBlocks_; }
     int                tailBlocks() const { return tailBlocks_[twoLevel_ ? 1 : 0]; }
