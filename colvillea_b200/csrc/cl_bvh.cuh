@@ -380,16 +380,24 @@ struct Trav2
     const float4* tris;
 };
 
-__device__ __forceinline__ void trav2SetRay(Trav2& s, f3 o, f3 d)
+// The world ray in the top tree, whose leaf entries are instances: box tests
+// only, so it needs no triangle setup (three quotients).
+__device__ __forceinline__ void trav2SetBoxRay(Trav2& s, f3 o, f3 d)
 {
-    s.pre   = rayPrepare(o, d);
+    s.pre.o = o;
     s.inv   = boxReciprocals(d);
     s.oct   = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
+}
+// A ray mapped to an instance's object space.
+__device__ __forceinline__ void trav2SetRay(Trav2& s, f3 o, f3 d)
+{
+    s.pre = rayPrepare(o, d);
+    trav2SetBoxRay(s, o, d);
 }
 
 __device__ __forceinline__ void trav2Init(const BvhView& bvh, Trav2& s, f3 o, f3 d, float tmin, float tmax)
 {
-    trav2SetRay(s, o, d);
+    trav2SetBoxRay(s, o, d);
     s.wo = o;
     s.wd = d;
     s.tmin = tmin;
@@ -518,7 +526,7 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
             s.inst  = kMissPrim;
             s.nodes = bvh.nodes;
             s.tris  = bvh.tris;
-            trav2SetRay(s, s.wo, s.wd);
+            trav2SetBoxRay(s, s.wo, s.wd);
         }
         if (s.sp == 0) return true;
         --s.sp;

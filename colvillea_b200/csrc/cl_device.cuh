@@ -774,9 +774,19 @@ __device__ __forceinline__ f3 directionalSample(const DirectionalLight& e, f2 u,
 struct RayPre
 {
     f3    o;
-    int   kx, ky, kz;
+    int   kz; // largest axis of the direction
     float Sx, Sy, Sz;
 };
+
+// The axes in cyclic order ending with kz.  (The test's authors swap the first
+// two for rays against kz to keep the triangle's winding; without the swap U, V,
+// W, the determinant and T only change sign together, exactly, which t and the
+// barycentrics do not show, and two registers and six selects are saved.)
+__device__ __forceinline__ f3 rotateAxes(f3 v, int kz)
+{
+    const bool z0 = kz == 0, z1 = kz == 1;
+    return {z0 ? v.y : (z1 ? v.z : v.x), z0 ? v.z : (z1 ? v.x : v.y), z0 ? v.x : (z1 ? v.y : v.z)};
+}
 
 __device__ __forceinline__ RayPre rayPrepare(f3 o, f3 d)
 {
@@ -784,17 +794,10 @@ __device__ __forceinline__ RayPre rayPrepare(f3 o, f3 d)
     r.o      = o;
     float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     r.kz     = (ax > ay) ? ((ax > az) ? 0 : 2) : ((ay > az) ? 1 : 2);
-    r.kx     = r.kz + 1 == 3 ? 0 : r.kz + 1;
-    r.ky     = r.kx + 1 == 3 ? 0 : r.kx + 1;
-    float dz = comp(d, r.kz);
-    if (dz < 0.0f)
-    {
-        int t = r.kx;
-        r.kx  = r.ky;
-        r.ky  = t;
-    }
-    r.Sx = comp(d, r.kx) / dz;
-    r.Sy = comp(d, r.ky) / dz;
+    const f3 p = rotateAxes(d, r.kz);
+    const float dz = p.z;
+    r.Sx = p.x / dz;
+    r.Sy = p.y / dz;
     r.Sz = 1.0f / dz;
     return r;
 }
@@ -803,21 +806,21 @@ __device__ __forceinline__ RayPre rayPrepare(f3 o, f3 d)
 // triangle (edges inclusive, det != 0); the t-range test is the caller's.
 __device__ __forceinline__ bool intersectTri(const RayPre& r, f3 v0, f3 v1, f3 v2, float* t, float* b1, float* b2)
 {
-    f3    A = v0 - r.o, B = v1 - r.o, C = v2 - r.o;
-    float Akz = comp(A, r.kz), Bkz = comp(B, r.kz), Ckz = comp(C, r.kz);
-    float Ax = comp(A, r.kx) - r.Sx * Akz, Ay = comp(A, r.ky) - r.Sy * Akz;
-    float Bx = comp(B, r.kx) - r.Sx * Bkz, By = comp(B, r.ky) - r.Sy * Bkz;
-    float Cx = comp(C, r.kx) - r.Sx * Ckz, Cy = comp(C, r.ky) - r.Sy * Ckz;
+    const f3 A = rotateAxes(v0 - r.o, r.kz), B = rotateAxes(v1 - r.o, r.kz), C = rotateAxes(v2 - r.o, r.kz);
+    float Akz = A.z, Bkz = B.z, Ckz = C.z;
+    float Ax = A.x - r.Sx * Akz, Ay = A.y - r.Sy * Akz;
+    float Bx = B.x - r.Sx * Bkz, By = B.y - r.Sy * Bkz;
+    float Cx = C.x - r.Sx * Ckz, Cy = C.y - r.Sy * Ckz;
     float U = Cx * By - Cy * Bx;
     float V = Ax * Cy - Ay * Cx;
     float W = Bx * Ay - By * Ax;
-    if (U == 0.0f || V == 0.0f || W == 0.0f)
+    if (fminf(fabsf(U), fminf(fabsf(V), fabsf(W))) == 0.0f)
     {
         U = float(double(Cx) * double(By) - double(Cy) * double(Bx));
         V = float(double(Ax) * double(Cy) - double(Ay) * double(Cx));
         W = float(double(Bx) * double(Ay) - double(By) * double(Ax));
     }
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
+    if (fminf(U, fminf(V, W)) < 0.0f && fmaxf(U, fmaxf(V, W)) > 0.0f) return false; // (a NaN fails the range test)
     float det = U + V + W;
     if (det == 0.0f) return false;
     float Az = r.Sz * Akz, Bz = r.Sz * Bkz, Cz = r.Sz * Ckz;

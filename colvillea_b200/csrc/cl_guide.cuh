@@ -99,8 +99,9 @@ __device__ __forceinline__ void cornerIndices(const GridView& g, int l, const Ce
     {
         const uint32_t y[2] = {c.y * 2654435761u, c.y * 2654435761u + 2654435761u};
         const uint32_t z[2] = {c.z * 805459861u, c.z * 805459861u + 805459861u};
+        const uint32_t yz[4] = {y[0] ^ z[0], y[1] ^ z[0], y[0] ^ z[1], y[1] ^ z[1]};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) idx[k] = ((c.x + uint32_t(k & 1)) ^ y[(k >> 1) & 1] ^ z[k >> 2]) & g.mask;
+        for (int k = 0; k < 8; ++k) idx[k] = ((c.x + uint32_t(k & 1)) ^ yz[k >> 1]) & g.mask;
     }
 }
 __device__ __forceinline__ f3 clampUnit(f3 p)
@@ -114,18 +115,18 @@ __device__ __forceinline__ float2 encodeLevel(const GridView& g, int l, f3 p)
     const __nv_bfloat162* __restrict__ tl = g.table + (size_t(l) << g.log2T);
     uint32_t                            idx[8];
     cornerIndices(g, l, c, idx);
-    __nv_bfloat162 t[8];
+    uint32_t t[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t[k] = __ldg(tl + idx[k]);
+    for (int k = 0; k < 8; ++k) // 32-bit byte offsets from the level's base
+        t[k] = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(tl) + (idx[k] << 2)));
     float w[8];
     cornerWeights(c, w);
     float f0 = 0.0f, f1 = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
     {
-        float2 v = __bfloat1622float2(t[k]);
-        f0       = fmaf(w[k], v.x, f0);
-        f1       = fmaf(w[k], v.y, f1);
+        f0 = fmaf(w[k], __uint_as_float(t[k] << 16), f0); // the two bf16 features
+        f1 = fmaf(w[k], __uint_as_float(t[k] & 0xffff0000u), f1);
     }
     return {f0, f1};
 }

@@ -389,11 +389,11 @@ __device__ __forceinline__ void warpStats(const TraceCounters& tc, unsigned long
     }
 }
 
-// Resident blocks per SM of the traversal kernels.  Flattened scenes: 8 (64
-// registers; config 2's 16.6 M paths 42.9 ms, with 7 blocks 43.6, with 6 45.4).
-// Two-level scenes: 5 (their state is larger; 4 blocks 6% slower, 6 blocks
-// equal).
-constexpr int kTraceBlocksFlat = 8;
+// Resident blocks per SM of the traversal kernels.  Flattened scenes: 7 (72
+// registers; config 2's 16.6 M paths 40.2 ms, with 8 blocks and 64 registers
+// 40.5).  Two-level scenes: 5 (their state is larger; 6 blocks equal, 4 blocks
+// 6% slower).
+constexpr int kTraceBlocksFlat = 7;
 constexpr int kTraceBlocksTwo  = 5;
 
 struct ClassifyView
