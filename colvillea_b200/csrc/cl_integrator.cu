@@ -1154,17 +1154,18 @@ __global__ void __launch_bounds__(128) kShadowResolve(Params P, int cur)
 // lanes at a time took 1.1 to 1.5 times as long).  With fewer paths than lanes
 // each warp takes an even share of them: a step costs a warp what its lanes'
 // divergent loads and branches cost together.
-// kTailMaxRays: measured with 0 (no tail), 8192, 24576, 32768 and 65536 rays on
-// a 256x256 frame of 10 k triangles (device time 675, 538, 584, 576 and 621
-// us), a 1920x1080 frame of 1.2 M triangles at one sample (3.85, 3.82, 3.71,
-// 3.70 and 3.70 ms), 1280x720x2 over 577 two-level instances at depth 16 (7.5,
-// 6.41, 6.35, 6.36 and 6.40 ms), and four trained samples of the radiance cache
-// at 960x540 (10.3 ms without, 5.35 ms with any of them: after its third wave a
-// pass holds only its 32 k training paths, which last to depth 16).
+// kTailMaxRays: measured with 2048, 4096, 8192, 16384 and 24576 rays on a 256x256
+// frame of 10 k triangles (device time 474, 394, 394, 460 and 455 us), a
+// 1920x1080 frame of 1.2 M triangles at one sample (3.04, 3.04, 3.11, 3.16 and
+// 3.24 ms), 1280x720x2 over 577 two-level instances at depth 16 (4.96, 4.91,
+// 4.96, 5.00 and 5.14 ms; without this launch 7.5 against 6.4 before the
+// traversal's other changes) and 640x360 over 0.7 M triangles (0.92, 0.92, 0.86,
+// 0.86 and 0.90 ms).  Four trained samples of the radiance cache at 960x540 take
+// 4.6 ms with any of them and took 10.3 without.
 // Not for guided passes (every vertex needs its network evaluation first);
 // with the radiance cache only once the waves have brought every path past
 // its query (wp.tailNeed).  kAdvance decides (Counters::tailNow).
-constexpr uint32_t kTailMaxRays = 24576;
+constexpr uint32_t kTailMaxRays = 6144;
 constexpr int      kTailBlocks  = 4; // resident blocks per SM (128 registers)
 enum TailState : uint32_t { kTailIdle, kTailClosest, kTailShadow, kTailShade, kTailResolve };
 

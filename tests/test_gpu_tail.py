@@ -12,7 +12,7 @@ import colvillea_b200 as cb
 from colvillea_b200 import scenes
 
 pytestmark = pytest.mark.gpu
-TAIL = 24576
+TAIL = 6144
 
 
 def render(s, spp, flags, **kw):
@@ -24,7 +24,7 @@ def render(s, spp, flags, **kw):
     return s1, s2, st
 
 
-@pytest.mark.parametrize("w,h,spp,slots", [(1, 1, 1, 0), (7, 5, 1, 0), (33, 31, 3, 0), (TAIL - 1, 1, 1, 0), (192, 128, 1, 0),
+@pytest.mark.parametrize("w,h,spp,slots", [(1, 1, 1, 0), (7, 5, 1, 0), (33, 31, 3, 0), (TAIL - 1, 1, 1, 0), (96, 64, 1, 0),
                                            (TAIL + 1, 1, 1, 0), (256, 200, 2, 0), (300, 200, 2, 30011)])
 @pytest.mark.parametrize("flags", [cb.COMPAT_ALL, cb.DOME_ALIAS, cb.COMPAT_PDF | cb.DOME_ALIAS])
 def test_tail_equals_waves(w, h, spp, slots, flags):
@@ -38,7 +38,7 @@ def test_tail_equals_waves(w, h, spp, slots, flags):
 
 @pytest.mark.parametrize("two", [0, cb.TWO_LEVEL])
 def test_tail_equals_waves_instances(two):
-    s = scenes.config1(6, 160, 150)
+    s = scenes.config1(6, 90, 80)
     rng = np.random.default_rng(3)
     for i in range(1, len(s.instances)):
         mesh, mat, _ = s.instances[i]
