@@ -734,8 +734,7 @@ struct VertexState
 // CMP: 1 = the reference's estimator (all CL_COMPAT_* flags), 0 = the
 // corrected one, 2 = a mix read at run time; ALIAS: alias-table dome sampling.
 // MAT: the shading class served (BSDF type 0-2, or 3 = escaped
-// rays), from the class queues written by kTraceClosest; -1 = every ray of
-// the ray queue.  Specialising keeps each instantiation free of the other
+// rays), or -1 for a vertex of any class (kPathTail).  Specialising keeps each instantiation free of the other
 // modes' and materials' code.
 // GUIDE (path tracing, corrected estimator, BSDF classes): one-sample MIS of
 // the BSDF and the network's vMF mixture for this ray (kGuideMlp), which is
