@@ -91,16 +91,11 @@ struct PoolView
     const uint32_t* __restrict__ idx;
 };
 
-// One thread per flattened vertex of copies inst[0, n) (base: the first one's dstVtx).
-__global__ void __launch_bounds__(kBlock) kFlattenVertices(PoolView P, const FlatInst* __restrict__ inst, uint32_t n,
-                                                           uint32_t base, uint32_t count, float4* __restrict__ vtx)
+// Vertex k of the copy I of its mesh.
+__device__ __forceinline__ void flattenVertex(const PoolView& P, const FlatInst& I, uint32_t k, float4* __restrict__ vtx)
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const uint32_t  dst = base + k;
-    const FlatInst& I = inst[lastAtMost(n, dst, [&](uint32_t i) { return __ldg(&inst[i].dstVtx); })];
-    const size_t    v = I.srcVtx + size_t(dst - I.dstVtx);
-    const uint32_t  flags = I.flags & 3u;
+    const size_t   v     = I.srcVtx + size_t(k);
+    const uint32_t flags = I.flags & 3u;
     float p[3], nn[3] = {0.0f, 0.0f, 0.0f}, t[3], uv[2] = {0.0f, 0.0f};
 #pragma unroll
     for (int q = 0; q < 3; ++q)
@@ -134,10 +129,35 @@ __global__ void __launch_bounds__(kBlock) kFlattenVertices(PoolView P, const Fla
             nn[q] = n2[q];
         }
     }
-    float4* o = vtx + 3 * size_t(dst);
+    float4* o = vtx + 3 * (I.dstVtx + size_t(k));
     o[0]      = make_float4(p[0], p[1], p[2], nn[0]);
     o[1]      = make_float4(nn[1], nn[2], t[0], t[1]);
     o[2]      = make_float4(t[2], uv[0], uv[1], __uint_as_float(flags));
+}
+
+// One thread per flattened vertex of copies inst[0, n) (base: the first one's dstVtx).
+__global__ void __launch_bounds__(kBlock) kFlattenVertices(PoolView P, const FlatInst* __restrict__ inst, uint32_t n,
+                                                           uint32_t base, uint32_t count, float4* __restrict__ vtx)
+{
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const uint32_t  dst = base + k;
+    const FlatInst& I = inst[lastAtMost(n, dst, [&](uint32_t i) { return __ldg(&inst[i].dstVtx); })];
+    flattenVertex(P, I, dst - I.dstVtx, vtx);
+}
+
+// One thread per vertex of one mesh's copies inst[list[..]], nv vertices each.
+// An edit writes all copies in one launch, bound by its fixed costs up to
+// about 100,000 vertices: whole edits of a 12-vertex mesh with 2,000 and 10,000
+// copies took 8.3 and 41 ms with a launch for each copy, 0.14 and 0.15 ms so.
+__global__ void __launch_bounds__(kBlock) kFlattenCopies(PoolView P, const FlatInst* __restrict__ inst,
+                                                         const uint32_t* __restrict__ list, uint32_t nv, uint32_t total,
+                                                         float4* __restrict__ vtx)
+{
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= total) return;
+    const uint32_t c = k / nv;
+    flattenVertex(P, inst[__ldg(list + c)], k - c * nv, vtx);
 }
 
 __global__ void __launch_bounds__(kBlock) kFlattenTriangles(PoolView P, const FlatInst* __restrict__ inst, uint32_t n,
@@ -360,6 +380,18 @@ cl_status MeshPool::flattenVertices(const DevBuf& inst, const FlatInst* host, ui
     kFlattenVertices<<<blocksFor(total), kBlock, 0, st>>>(PoolView{pos(), nrm(), tan(), uv(), idx()},
                                                           inst.as<const FlatInst>() + first, count, base, total,
                                                           static_cast<float4*>(vtx));
+    CL_CUDA(cudaGetLastError(), err);
+    return CL_OK;
+}
+
+cl_status MeshPool::flattenCopies(uint32_t mesh, const DevBuf& inst, const uint32_t* list, uint32_t count, void* vtx,
+                                  cudaStream_t st, std::string* err) const
+{
+    if (count == 0) return CL_OK;
+    const uint32_t nv = info_[mesh].nv, total = nv * count; // at most the scene's vertices
+    kFlattenCopies<<<blocksFor(total), kBlock, 0, st>>>(PoolView{pos(), nrm(), tan(), uv(), idx()},
+                                                        inst.as<const FlatInst>(), list, nv, total,
+                                                        static_cast<float4*>(vtx));
     CL_CUDA(cudaGetLastError(), err);
     return CL_OK;
 }

@@ -46,6 +46,9 @@ public:
     // same table in host memory).  The copies' destinations are consecutive.
     cl_status flattenVertices(const DevBuf& inst, const FlatInst* host, uint32_t first, uint32_t count, void* vtx,
                               cudaStream_t st, std::string* err) const;
+    // The same for `count` copies of one mesh: entries list[0, count) (device) of the table.
+    cl_status flattenCopies(uint32_t mesh, const DevBuf& inst, const uint32_t* list, uint32_t count, void* vtx,
+                            cudaStream_t st, std::string* err) const;
     // Writes the index entries {3 vertex ids, w} of all `count` copies' triangles.
     cl_status flattenTriangles(const DevBuf& inst, const FlatInst* host, uint32_t count, void* triIdx, cudaStream_t st,
                                std::string* err) const;

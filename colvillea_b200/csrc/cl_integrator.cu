@@ -1919,8 +1919,17 @@ cl_status Integrator::buildInstances(const cl_instance_desc* inst, uint32_t n, s
         vo += flat[i].nv;
         to += flat[i].nt;
     }
+    std::vector<uint32_t> start(meshes_.size() + 1, 0u), copies(n);
+    for (uint32_t i = 0; i < n; ++i) ++start[inst[i].mesh_id + 1];
+    for (size_t m = 0; m < meshes_.size(); ++m) start[m + 1] += start[m];
+    {
+        std::vector<uint32_t> at(start);
+        for (uint32_t i = 0; i < n; ++i) copies[at[inst[i].mesh_id]++] = i;
+    }
     sceneBuilt_ = false; // until the new one is complete
     flat_.swap(flat);
+    copies_.swap(copies);
+    copyStart_.swap(start);
     CL_TRY(uploadFlat(err));
     CL_TRY(vtx_.alloc(nv * 48, err));
     CL_TRY(triIdx_.alloc(nt * 16, err));
@@ -1964,9 +1973,10 @@ static const float kIdentity12[12] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0};
 
 cl_status Integrator::uploadFlat(std::string* err)
 {
-    const size_t b = flat_.size() * sizeof(FlatInst);
-    if (flatDev_.bytes < b) CL_TRY(flatDev_.alloc(b, err));
+    const size_t b = flat_.size() * sizeof(FlatInst), c = copies_.size() * 4;
+    if (flatDev_.bytes < b + c) CL_TRY(flatDev_.alloc(b + c, err));
     CL_CUDA(cudaMemcpyAsync(flatDev_.p, flat_.data(), b, cudaMemcpyHostToDevice, stream_), err);
+    if (c) CL_CUDA(cudaMemcpyAsync(flatDev_.as<char>() + b, copies_.data(), c, cudaMemcpyHostToDevice, stream_), err);
     return CL_OK;
 }
 
@@ -2176,6 +2186,7 @@ cl_status Integrator::buildTwoLevel(const cl_instance_desc* inst, uint32_t n, st
                                 &flat[size_t(nm) + i], err));
     sceneBuilt_ = false; // until the new one is complete
     flat_.swap(flat);
+    copies_.clear();
     const auto   w0 = std::chrono::steady_clock::now();
     const double a0 = allocMs();
     CL_CUDA(cudaEventRecord(evA_, stream_), err);
@@ -2281,9 +2292,8 @@ cl_status Integrator::updateMeshVertices(uint32_t meshId, const float* pos, cons
     if (twoLevel_) return updateTwoLevel(meshId, mode, err);
 
     // Re-flatten the instances of this mesh into their vertex ranges.
-    for (uint32_t i = 0; i < inst_.size(); ++i)
-        if (inst_[i].mesh_id == meshId)
-            CL_TRY(meshes_.flattenVertices(flatDev_, flat_.data(), i, 1, vtx_.p, stream_, err));
+    CL_TRY(meshes_.flattenCopies(meshId, flatDev_, copiesDev() + copyStart_[meshId],
+                                 copyStart_[meshId + 1] - copyStart_[meshId], vtx_.p, stream_, err));
 
     // Device time of the refit and/or rebuild (the surface-area cost pass
     // and the vertex upload are not included).

@@ -239,6 +239,10 @@ private:
     // (flattened scenes), or the meshes and then the instances (two-level).
     std::vector<FlatInst> flat_;
     DevBuf                flatDev_;
+    // Flattened scenes: the copies (indices of flat_) mesh by mesh, mesh m's
+    // from copyStart_[m] on; on the device behind flatDev_'s table.
+    std::vector<uint32_t> copies_, copyStart_;
+    const uint32_t*       copiesDev() const { return flatDev_.u() + flat_.size() * (sizeof(FlatInst) / 4); }
     cl_status             uploadFlat(std::string* err);
     void                  setSceneBox(const float lo[3], const float hi[3]);
     // Two-level scenes (CL_TWO_LEVEL): object-space pools, one tree per mesh,
