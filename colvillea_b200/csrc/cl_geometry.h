@@ -33,7 +33,8 @@ public:
     // error the pool keeps what it held.
     cl_status build(const cl_mesh_desc* meshes, uint32_t n, cudaStream_t st, std::string* err);
     // New vertices of one mesh (normals, tangents: null keeps them).  Refuses
-    // positions that are not finite before anything changes.
+    // positions that are not finite before anything changes.  The arrays are
+    // read until the stream has been synchronised.
     cl_status updateVertices(uint32_t mesh, const float* pos, const float* nrm, const float* tan, cudaStream_t st,
                              std::string* err);
 

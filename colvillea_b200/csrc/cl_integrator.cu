@@ -2279,6 +2279,14 @@ cl_status Integrator::updateMeshVertices(uint32_t meshId, const float* pos, cons
         *err = "unknown BVH update mode";
         return CL_ERR_INVALID_ARG;
     }
+    const cl_status s = editMesh(meshId, pos, nrm, tan, mode, err);
+    if (s != CL_OK) cudaStreamSynchronize(stream_); // the caller's arrays may still be read (an edit that succeeds waits itself)
+    return s;
+}
+
+cl_status Integrator::editMesh(uint32_t meshId, const float* pos, const float* nrm, const float* tan, uint32_t mode,
+                               std::string* err)
+{
     const bool hadN = meshes_[meshId].hasN;
     CL_TRY(meshes_.updateVertices(meshId, pos, nrm, tan, stream_, err));
     if (meshes_[meshId].hasN != hadN)

@@ -256,6 +256,7 @@ private:
     cl_status buildBlasAll(const std::vector<uint32_t>& meshes, std::string* err);
     cl_status buildTopLevel(BuildArena* arena, std::string* err);
     cl_status uploadInstances(std::string* err);
+    cl_status editMesh(uint32_t meshId, const float* pos, const float* nrm, const float* tan, uint32_t mode, std::string* err);
     cl_status updateTwoLevel(uint32_t meshId, uint32_t mode, std::string* err);
     // Refit policy (CL_BVH_UPDATE_AUTO): rebuild when the refitted tree's
     // surface-area cost exceeds this multiple of the cost after its build.
