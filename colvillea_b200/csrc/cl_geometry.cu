@@ -245,6 +245,55 @@ __global__ void __launch_bounds__(kBlock) kVertexBounds(const float4* __restrict
     }
 }
 
+// Host arrays to consecutive places of one device allocation.  Arrays below
+// kPackBelow are gathered in a block of host memory first and copied together,
+// since a copy call costs 3.5 us whatever its size.  cl_build_meshes on 2,000
+// meshes of 12 vertices: 17 ms with a call for each array, 0.6 gathered; 1,000
+// of 642: 11.4 and 4.4; 500 of 2,562: 13.1 and 9.3 (with a limit of 16 KB 13.7,
+// of 256 KB 9.5); arrays of 120 KB and more: equal.  Blocks of 256, 128 and 64
+// KB: 1,000 meshes of 642 in 4.6, 5.3 and 5.7 ms.
+constexpr size_t kPackBelow = 65536, kPackBlock = size_t(1) << 20;
+class PackedUpload
+{
+public:
+    PackedUpload(char* dst, size_t total, cudaStream_t st)
+        : dst_(dst), cap_(std::min(kPackBlock, total)), block_(new char[cap_]), st_(st)
+    {
+    }
+    // The next `bytes` of the allocation; src null: left as they are or written with zeros (nothing reads them).
+    cl_status add(const void* src, size_t bytes, std::string* err)
+    {
+        if (bytes >= kPackBelow || bytes > cap_)
+        {
+            CL_TRY(flush(err));
+            if (src) CL_CUDA(cudaMemcpyAsync(dst_ + at_, src, bytes, cudaMemcpyHostToDevice, st_), err);
+            at_ += bytes;
+            return CL_OK;
+        }
+        if (fill_ + bytes > cap_) CL_TRY(flush(err));
+        if (src)
+            memcpy(block_.get() + fill_, src, bytes);
+        else
+            memset(block_.get() + fill_, 0, bytes);
+        fill_ += bytes;
+        return CL_OK;
+    }
+    // Copies what has been gathered (from pageable memory: the block is free again on return).
+    cl_status flush(std::string* err)
+    {
+        if (fill_) CL_CUDA(cudaMemcpyAsync(dst_ + at_, block_.get(), fill_, cudaMemcpyHostToDevice, st_), err);
+        at_ += fill_;
+        fill_ = 0;
+        return CL_OK;
+    }
+
+private:
+    char*                   dst_;
+    size_t                  at_ = 0, fill_ = 0, cap_; // bytes placed; gathered behind them
+    std::unique_ptr<char[]> block_;
+    cudaStream_t            st_;
+};
+
 uint32_t blocksFor(size_t n) { return uint32_t((n + kBlock - 1) / kBlock); }
 } // namespace
 
@@ -278,22 +327,14 @@ cl_status MeshPool::build(const cl_mesh_desc* meshes, uint32_t n, cudaStream_t s
         const size_t words = 11 * nv + 3 * nt, tabAt = (words + 3) / 4 * 4; // 16-byte aligned table
         CL_TRY(mem.alloc(4 * (tabAt + 2 * size_t(n) + 1), err));
         float* f = mem.f();
-        for (uint32_t m = 0; m < n; ++m)
-        {
-            const cl_mesh_desc& d = meshes[m];
-            const MeshInfo&     i = info[m];
-            const struct
-            {
-                const void* src;
-                size_t      at, words;
-            } part[5] = {{d.positions, 3 * size_t(i.vtxBase), 3 * size_t(i.nv)},
-                         {d.normals, 3 * (nv + i.vtxBase), 3 * size_t(i.nv)},
-                         {d.tangents, 3 * (2 * nv + i.vtxBase), 3 * size_t(i.nv)},
-                         {d.uvs, 9 * nv + 2 * size_t(i.vtxBase), 2 * size_t(i.nv)},
-                         {d.indices, 11 * nv + 3 * size_t(i.triBase), 3 * size_t(i.nt)}};
-            for (const auto& p : part)
-                if (p.src) CL_CUDA(cudaMemcpyAsync(f + p.at, p.src, 4 * p.words, cudaMemcpyHostToDevice, st), err);
-        }
+        // The pool's five parts, mesh after mesh.
+        PackedUpload up(reinterpret_cast<char*>(f), 4 * words, st);
+        for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].positions, 12 * size_t(info[m].nv), err));
+        for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].normals, 12 * size_t(info[m].nv), err));
+        for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].tangents, 12 * size_t(info[m].nv), err));
+        for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].uvs, 8 * size_t(info[m].nv), err));
+        for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].indices, 12 * size_t(info[m].nt), err));
+        CL_TRY(up.flush(err));
         uint2*    dTab = reinterpret_cast<uint2*>(f + tabAt);
         uint32_t* dBad = reinterpret_cast<uint32_t*>(dTab + n);
         CL_CUDA(cudaMemcpyAsync(dTab, tab.data(), 8 * size_t(n), cudaMemcpyHostToDevice, st), err);
