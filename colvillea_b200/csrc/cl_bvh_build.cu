@@ -1322,7 +1322,7 @@ cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh*
         keep.take(out->nodes, size_t(out->numNodes) * kNodeU4 * 16);
         keep.take(out->tris, nn * kTriF4 * 16);
         keep.take(out->exact, size_t(out->numNodes) * 24);
-        keep.take(out->scene, 64);
+        keep.take(out->scene, 128);
         CL_TRY(out->mem.alloc(keep.peak(), err));
         keep.bind(out->mem.p);
         CL_CUDA(cudaMemcpyAsync(out->nodes.p, nodes.p, out->nodes.bytes, cudaMemcpyDeviceToDevice, st), err);
@@ -1550,11 +1550,14 @@ __device__ __forceinline__ double boxArea(float lx, float ly, float lz, float hx
 }
 
 // Sum over all child slots of (dequantised box area) x (1 for an inner
-// child, its triangle count for a leaf), into *sum.
+// child, its triangle count for a leaf), into *sum; a copy of the root node
+// goes behind it, so that the host reads both at once (each read of pageable
+// memory waits for itself, 9 us).
 __global__ void kSahSum(const uint4* __restrict__ nodes, uint32_t n, double* sum)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     double   c = 0.0;
+    if (i < 5u) reinterpret_cast<uint4*>(sum)[1 + i] = nodes[i];
     if (i < n)
     {
         const uint4* np = nodes + size_t(i) * kNodeU4;
@@ -1651,11 +1654,12 @@ cl_status wideBvhSahCost(WideBvh& bvh, cudaStream_t st, double* cost, std::strin
     CL_CUDA(cudaMemsetAsync(sum, 0, 8, st), err);
     kSahSum<<<(bvh.numNodes + 255) / 256, 256, 0, st>>>(bvh.nodes.as<const uint4>(), bvh.numNodes, sum);
     CL_CUDA(cudaGetLastError(), err);
-    double                total = 0.0;
-    std::vector<uint32_t> h(20);
-    CL_CUDA(cudaMemcpyAsync(&total, sum, 8, cudaMemcpyDeviceToHost, st), err);
-    CL_CUDA(cudaMemcpyAsync(h.data(), bvh.nodes.p, 80, cudaMemcpyDeviceToHost, st), err);
+    uint32_t back[24]; // the sum, 8 unused bytes, the root node
+    CL_CUDA(cudaMemcpyAsync(back, sum, sizeof(back), cudaMemcpyDeviceToHost, st), err);
     CL_CUDA(cudaStreamSynchronize(st), err);
+    double          total;
+    const uint32_t* h = back + 4;
+    memcpy(&total, back, 8);
     // Root box extent per axis: e * (largest qhi - smallest qlo) over the
     // root's present slots (qlo words at h[8 + 2a + w], qhi at h[14 + 2a + w]).
     double ext[3];

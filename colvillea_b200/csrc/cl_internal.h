@@ -125,7 +125,7 @@ struct WideBvh
     ScratchBuf nodes; // 6 uint4 per node
     ScratchBuf tris;  // 3 float4 per triangle, leaf order
     ScratchBuf exact; // refit: 6 floats per node, the unquantised box of its triangles
-    ScratchBuf scene; // scene bounds (6 ordered ints, refit) and the SAH sum (double at byte 32)
+    ScratchBuf scene; // scene bounds (6 ordered ints, refit); SAH sum (double at byte 32), copy of the root node (byte 48)
     // Nodes of tree level d are [levels[d], levels[d + 1]): the collapse
     // allocates each level's nodes in one launch.
     std::vector<uint32_t> levels;
