@@ -407,6 +407,14 @@ cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns)
     return guarded([&](std::string* e) { return clb::unitTcWaitTimeout(waited_ns, e); });
 }
 
+cl_status cl_unit_limit_stack(cl_integrator* it, uint32_t entries)
+{
+    CL_NEED(it);
+    return guarded([&](std::string*) {
+        it->impl.limitStack(entries);
+        return CL_OK;
+    });
+}
 cl_status cl_unit_binary_version(int32_t* binary_version, int32_t* ptx_version)
 {
     return guarded([&](std::string* e) { return clb::unitBinaryVersion(binary_version, ptx_version, e); });

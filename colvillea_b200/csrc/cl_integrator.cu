@@ -2560,17 +2560,18 @@ BvhView Integrator::bvhView() const
     // Named members (not an aggregate list): the struct's field order is no
     // part of this function's contract.
     BvhView v{};
-    v.nodes = bvh_.nodes.as<const uint4>();
-    v.tris  = bvh_.tris.as<const float4>();
-    if (twoLevel_)
-    {
-        v.inst       = instDev_.as<const InstDev>();
-        v.stackDepth = twoLevelStack_;
-        return v;
-    }
-    v.inst       = nullptr;
-    v.stackDepth = std::min<uint32_t>(bvh_.depth + 1u, uint32_t(kStackDepth));
+    v.nodes      = bvh_.nodes.as<const uint4>();
+    v.tris       = bvh_.tris.as<const float4>();
+    v.inst       = twoLevel_ ? instDev_.as<const InstDev>() : nullptr;
+    v.stackDepth = twoLevel_ ? twoLevelStack_ : std::min<uint32_t>(bvh_.depth + 1u, uint32_t(kStackDepth));
+    v.stackDepth = std::min(v.stackDepth, stackLimit_);
     return v;
+}
+
+void Integrator::limitStack(uint32_t entries)
+{
+    stackLimit_ = entries;
+    graphValid_ = false;
 }
 
 ClassifyView Integrator::classifyView() const
@@ -3329,8 +3330,10 @@ cl_status Integrator::getBvh(void* nodes, size_t nodeBytes, void* tris, size_t t
     return CL_OK;
 }
 
-// Uploads rays [base, base + m) of a query, launches it and fetches its
-// counters.  The buffers hold kQueryChunk rays at most and are kept.
+// Uploads m rays of a query, launches it and queues the read of its counters
+// (ahead of the results' copies to pageable memory, which wait for themselves:
+// behind them it cost a query of one ray 12 us).  The buffers hold kQueryChunk
+// rays at most and are kept.
 cl_status Integrator::launchQuery(const float* rays, uint32_t m, bool any, bool stats, QueryOut* out, std::string* err)
 {
     if (queryIn_.bytes < size_t(m) * 32) CL_TRY(queryIn_.alloc(size_t(m) * 32, err));
@@ -3349,6 +3352,21 @@ cl_status Integrator::launchQuery(const float* rays, uint32_t m, bool any, bool 
     table[any ? 1 : stats ? 2 : 0][twoLevel_]<<<tBlocks(), kTraceBlock, traceStackBytes(v.stackDepth), stream_>>>(
         v, queryIn_.as<const float4>(), m, *out, ctr_.as<Counters>());
     CL_CUDA(cudaGetLastError(), err);
+    CL_CUDA(cudaMemcpyAsync(hostCtr_, ctr_.p, sizeof(Counters), cudaMemcpyDeviceToHost, stream_), err);
+    return CL_OK;
+}
+
+// Waits for a query, its copies and its counters (*hostCtr_).  A ray whose
+// traversal ran out of stack counts as a miss on the device: an error.
+cl_status Integrator::finishQuery(std::string* err)
+{
+    CL_CUDA(cudaStreamSynchronize(stream_), err);
+    if (hostCtr_->error)
+    {
+        *err = "traversal error flags " + std::to_string(hostCtr_->error) +
+               (hostCtr_->error & 1u ? " (traversal stack overflow)" : "");
+        return CL_ERR_STATE;
+    }
     return CL_OK;
 }
 
@@ -3376,14 +3394,7 @@ cl_status Integrator::traceRays(const float* rays, uint32_t n, float* t, uint32_
         CL_CUDA(cudaMemcpyAsync(prim + base, o.prim, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
         CL_CUDA(cudaMemcpyAsync(b1 + base, o.b1, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
         CL_CUDA(cudaMemcpyAsync(b2 + base, o.b2, size_t(m) * 4, cudaMemcpyDeviceToHost, stream_), err);
-        Counters ch;
-        CL_CUDA(cudaMemcpyAsync(&ch, ctr_.p, sizeof(ch), cudaMemcpyDeviceToHost, stream_), err);
-        CL_CUDA(cudaStreamSynchronize(stream_), err);
-        if (ch.error)
-        {
-            *err = "traversal error flags " + std::to_string(ch.error);
-            return CL_ERR_STATE;
-        }
+        CL_TRY(finishQuery(err));
     }
     return CL_OK;
 }
@@ -3407,7 +3418,7 @@ cl_status Integrator::occludedRays(const float* rays, uint32_t n, uint8_t* occ, 
         QueryOut o;
         CL_TRY(launchQuery(rays + 8 * size_t(base), m, true, false, &o, err));
         CL_CUDA(cudaMemcpyAsync(occ + base, o.occ, m, cudaMemcpyDeviceToHost, stream_), err);
-        CL_CUDA(cudaStreamSynchronize(stream_), err);
+        CL_TRY(finishQuery(err));
     }
     return CL_OK;
 }
@@ -3431,11 +3442,9 @@ cl_status Integrator::traceStats(const float* rays, uint32_t n, uint64_t* nodes,
         m = std::min(kQueryChunk, n - base);
         QueryOut o;
         CL_TRY(launchQuery(rays + 8 * size_t(base), m, false, true, &o, err));
-        Counters ch;
-        CL_CUDA(cudaMemcpyAsync(&ch, ctr_.p, sizeof(ch), cudaMemcpyDeviceToHost, stream_), err);
-        CL_CUDA(cudaStreamSynchronize(stream_), err);
-        an += ch.statNodes;
-        at += ch.statTris;
+        CL_TRY(finishQuery(err));
+        an += hostCtr_->statNodes;
+        at += hostCtr_->statTris;
     }
     *nodes = an;
     *tris  = at;

@@ -188,6 +188,8 @@ public:
     cl_status domeTables(float* pU, float* cU, float* pV, float* cV, std::string* err);
     cl_status domeAliasTables(uint32_t* aliasRow, uint32_t* aliasCol, std::string* err);
     cl_status waveRays(uint64_t* out, uint32_t cap, uint32_t* count, std::string* err) const;
+    // Test of the overflow report: traversal stacks hold at most this many entries.
+    void      limitStack(uint32_t entries);
     cl_status guideProbe(uint32_t cap, float* rows, uint32_t* count, std::string* err);
     cl_status beginPass(uint32_t spp, bool record, bool cacheTrain, uint32_t* initSlots, bool* tailOnly, std::string* err);
     cl_status domeAliasSample(const float* u2, float* dir, float* pdf, float* val, uint32_t n, std::string* err);
@@ -212,6 +214,7 @@ private:
     cl_status resolveFilm(std::string* err);
     cl_status checkPathSlots(std::string* err) const;
     cl_status ensureQueues(std::string* err);
+    cl_status finishQuery(std::string* err);
     cl_status launchQuery(const float* rays, uint32_t m, bool any, bool stats, QueryOut* out, std::string* err);
     cl_status clearFilm(std::string* err);
     cl_status captureGraph(std::string* err);
@@ -251,6 +254,7 @@ private:
     std::vector<std::unique_ptr<WideBvh>> blas_; // per mesh (null: not instanced)
     DevBuf                 instDev_;
     uint32_t               twoLevelStack_ = 0;
+    uint32_t               stackLimit_ = 0xffffffffu;
     cl_status buildTwoLevel(const cl_instance_desc* inst, uint32_t n, std::string* err);
     cl_status buildBlas(uint32_t meshId, BuildArena* arena, cudaStream_t st, std::string* err);
     cl_status buildBlasAll(const std::vector<uint32_t>& meshes, std::string* err);

@@ -380,6 +380,12 @@ cl_status cl_unit_normal_frame(const float* in, float* frame, uint32_t count);
  * CL_ERR_TIMEOUT with the time waited, and the context stays usable.  No
  * counterpart in the reference; it tests the failure path without a fault. */
 cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns);
+/* Limits the integrator's traversal stacks to `entries` (0xffffffff: as many
+ * as its trees need, the default): with too few, cl_render, cl_trace_rays,
+ * cl_occluded_rays and cl_trace_stats return CL_ERR_STATE with the overflow
+ * that the kernels' own bounds check records.  No counterpart in the reference;
+ * it tests the failure path without a fault. */
+cl_status cl_unit_limit_stack(cl_integrator* integrator, uint32_t entries);
 /* Target of the library's device code as the CUDA runtime reports it for one
  * of its kernels (cudaFuncGetAttributes: binaryVersion 100 = sm_100a SASS).
  * No counterpart in the reference. */
