@@ -1037,29 +1037,36 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseArgs A, co
     if (q == 0u) A.nodes[size_t(wide) * kNodeU4 + 5] = make_uint4(lv, ex[0] << 23, ex[1] << 23, ex[2] << 23);
 }
 
-// Validation of a built tree (error bits: 1 exponent outside 1..254, 2 child
-// index beyond the node count, 4 leaf triangle range outside the node's 24 or
-// the triangle count, 8 triangle ids not a permutation of 0..n-1).
+// Validation of a built tree (error bits: 1 exponent outside 1..254 or a scale
+// that is not its power of two, 2 child index beyond the node count, 4 leaf
+// word or leaf triangle range that is not the slots' or leaves the node's 24 or
+// the triangle count, 8 triangle ids not a permutation of 0..n-1).  The
+// traversal follows the leaf word (a hit slot's bits and the popcounts below
+// them) and the float scales; the slots' metadata state the same.
 __global__ void kValidateNodes(const uint4* __restrict__ nodes, uint32_t numNodes, uint32_t n, uint32_t* err)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= numNodes) return;
-    uint4    n0 = nodes[size_t(i) * kNodeU4], n1 = nodes[size_t(i) * kNodeU4 + 1];
-    uint32_t imask = n0.w >> 24, bits = 0u;
+    const uint4 n0 = nodes[size_t(i) * kNodeU4], n1 = nodes[size_t(i) * kNodeU4 + 1], n5 = nodes[size_t(i) * kNodeU4 + 5];
+    uint32_t    imask = n0.w >> 24, bits = 0u;
+    const uint32_t scale[3] = {n5.y, n5.z, n5.w};
     for (int a = 0; a < 3; ++a)
     {
         uint32_t e = (n0.w >> (8 * a)) & 0xffu;
-        if (e < 1u || e > 254u) bits |= 1u;
+        if (e < 1u || e > 254u || scale[a] != e << 23) bits |= 1u;
     }
     if (imask && uint64_t(n1.x) + __popc(imask) > numNodes) bits |= 2u;
+    if (n5.x >> 24) bits |= 4u;
     for (int sl = 0; sl < 8; ++sl)
     {
-        if (imask & (1u << sl)) continue;
-        uint32_t meta = ((sl < 4 ? n1.z : n1.w) >> (8 * (sl & 3))) & 0xffu;
-        if (!meta) continue;
-        uint32_t off = meta & 31u, unary = meta >> 5;
-        uint32_t cnt = unary == 1u ? 1u : unary == 3u ? 2u : unary == 7u ? 3u : 99u;
-        if (cnt == 99u || off + cnt > 24u || uint64_t(n1.y) + off + cnt > n) bits |= 4u;
+        const uint32_t meta  = ((sl < 4 ? n1.z : n1.w) >> (8 * (sl & 3))) & 0xffu;
+        const bool     leaf  = !(imask & (1u << sl)) && meta;
+        const uint32_t unary = leaf ? meta >> 5 : 0u, word = (n5.x >> (3 * sl)) & 7u;
+        if (word != unary) bits |= 4u;
+        if (!leaf) continue;
+        const uint32_t off = meta & 31u, cnt = unary == 1u ? 1u : unary == 3u ? 2u : unary == 7u ? 3u : 99u;
+        if (cnt == 99u || off != __popc(n5.x & ((1u << (3 * sl)) - 1u)) || off + cnt > 24u || uint64_t(n1.y) + off + cnt > n)
+            bits |= 4u;
     }
     if (bits) atomicOr(err, bits);
 }
@@ -1078,7 +1085,44 @@ __global__ void kValidateTris(const float4* __restrict__ tris, uint32_t n, uint3
     if (atomicOr(seen + (id >> 5), bit) & bit) atomicOr(err, 8u);
 }
 
+// Error bits of a tree; seen: a bit per triangle, bits: one word (device).  Synchronises.
+cl_status validateBvh(const uint4* nodes, uint32_t numNodes, const float4* tris, uint32_t n, uint32_t* seen,
+                      uint32_t* bits, cudaStream_t st, uint32_t* out, std::string* err)
+{
+    CL_CUDA(cudaMemsetAsync(bits, 0, 4, st), err);
+    CL_CUDA(cudaMemsetAsync(seen, 0, (size_t(n) + 31) / 32 * 4, st), err);
+    kValidateNodes<<<(numNodes + 255) / 256, 256, 0, st>>>(nodes, numNodes, n, bits);
+    kValidateTris<<<(n + 255) / 256, 256, 0, st>>>(tris, n, seen, bits);
+    CL_CUDA(cudaGetLastError(), err);
+    CL_CUDA(cudaMemcpyAsync(out, bits, 4, cudaMemcpyDeviceToHost, st), err);
+    CL_CUDA(cudaStreamSynchronize(st), err);
+    return CL_OK;
+}
+
 } // namespace
+
+cl_status unitValidateBvh(const uint32_t* nodes, uint32_t numNodes, const float* tris, uint32_t n, uint32_t* bits,
+                          std::string* err)
+{
+    if (!nodes || !tris || !bits || numNodes == 0 || n == 0)
+    {
+        *err = "a tree to validate needs nodes and triangles";
+        return CL_ERR_INVALID_ARG;
+    }
+    const size_t nb = size_t(numNodes) * kNodeU4 * 16, tb = size_t(n) * kTriF4 * 16;
+    DevBuf       d;
+    ScratchBuf   dn, dt, seen, word;
+    Carver       cv;
+    cv.take(dn, nb);
+    cv.take(dt, tb);
+    cv.take(seen, (size_t(n) + 31) / 32 * 4);
+    cv.take(word, 4);
+    CL_TRY(d.alloc(cv.peak(), err));
+    cv.bind(d.p);
+    CL_CUDA(cudaMemcpy(dn.p, nodes, nb, cudaMemcpyHostToDevice), err);
+    CL_CUDA(cudaMemcpy(dt.p, tris, tb, cudaMemcpyHostToDevice), err);
+    return validateBvh(dn.as<const uint4>(), numNodes, dt.as<const float4>(), n, seen.u(), word.u(), nullptr, bits, err);
+}
 
 cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh* out, std::string* err,
                        BuildArena* arena)
@@ -1331,18 +1375,12 @@ cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh*
     // Validation of every index the traversal kernels will follow, on the
     // device; one error word comes back.
     {
-        CL_CUDA(cudaMemsetAsync(verr.p, 0, 4, st), err);
-        CL_CUDA(cudaMemsetAsync(seen.p, 0, (size_t(n) + 31) / 32 * 4, st), err);
-        kValidateNodes<<<(out->numNodes + 255) / 256, 256, 0, st>>>(out->nodes.as<const uint4>(), out->numNodes, n,
-                                                                       verr.u());
-        kValidateTris<<<(n + 255) / 256, 256, 0, st>>>(out->tris.as<const float4>(), n, seen.u(), verr.u());
-        CL_CUDA(cudaGetLastError(), err);
         uint32_t bad = 0;
-        CL_CUDA(cudaMemcpyAsync(&bad, verr.p, 4, cudaMemcpyDeviceToHost, st), err);
-        CL_CUDA(cudaStreamSynchronize(st), err);
+        CL_TRY(validateBvh(out->nodes.as<const uint4>(), out->numNodes, out->tris.as<const float4>(), n, seen.u(), verr.u(),
+                           st, &bad, err));
         if (bad)
         {
-            *err = (bad & 1u)   ? "BVH validation: bad exponent"
+            *err = (bad & 1u)   ? "BVH validation: bad exponent or scale"
                    : (bad & 2u) ? "BVH validation: child index out of range"
                    : (bad & 4u) ? "BVH validation: leaf triangle range out of bounds"
                                 : "BVH validation: triangle ids are not a permutation";

@@ -82,6 +82,7 @@ cl_status unitFrame(const float*, const float*, const float*, const float*, floa
 cl_status unitPcg(const uint32_t*, uint32_t*, uint32_t, std::string*);
 cl_status unitNormalFrame(const float*, float*, uint32_t, std::string*);
 cl_status unitTcWaitTimeout(uint64_t*, std::string*);
+cl_status unitValidateBvh(const uint32_t*, uint32_t, const float*, uint32_t, uint32_t*, std::string*);
 cl_status unitBinaryVersion(int32_t*, int32_t*, std::string*);
 cl_status unitTextureLookup(const cl_texture_desc*, const float*, float*, uint32_t, std::string*);
 cl_status unitSeq(const uint32_t*, uint32_t, uint32_t, float*, std::string*);
@@ -415,6 +416,13 @@ cl_status cl_unit_limit_stack(cl_integrator* it, uint32_t entries)
         return CL_OK;
     });
 }
+
+cl_status cl_unit_validate_bvh(const uint32_t* nodes, uint32_t num_nodes, const float* triangles, uint32_t num_triangles,
+                               uint32_t* error_bits)
+{
+    return guarded([&](std::string* e) { return clb::unitValidateBvh(nodes, num_nodes, triangles, num_triangles, error_bits, e); });
+}
+
 cl_status cl_unit_binary_version(int32_t* binary_version, int32_t* ptx_version)
 {
     return guarded([&](std::string* e) { return clb::unitBinaryVersion(binary_version, ptx_version, e); });

@@ -386,6 +386,13 @@ cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns);
  * that the kernels' own bounds check records.  No counterpart in the reference;
  * it tests the failure path without a fault. */
 cl_status cl_unit_limit_stack(cl_integrator* integrator, uint32_t entries);
+/* The validation that every built tree passes, on the caller's tree: nodes of 24
+ * words as the traversal reads them (cl_get_bvh's 20, then the leaf word and
+ * the three scales as floats; layout in cl_bvh.cuh), triangles as from
+ * cl_get_bvh.  error_bits: 1 exponents and scales, 2 child indices, 4 leaf words
+ * and ranges, 8 triangle ids; 0 for a valid tree.  Nothing is traversed. */
+cl_status cl_unit_validate_bvh(const uint32_t* nodes, uint32_t num_nodes, const float* triangles,
+                               uint32_t num_triangles, uint32_t* error_bits);
 /* Target of the library's device code as the CUDA runtime reports it for one
  * of its kernels (cudaFuncGetAttributes: binaryVersion 100 = sm_100a SASS).
  * No counterpart in the reference. */
