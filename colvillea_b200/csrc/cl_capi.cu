@@ -56,6 +56,12 @@ double& allocMs()
     return ms;
 }
 
+int& failAlloc()
+{
+    static thread_local int k = -1;
+    return k;
+}
+
 static std::atomic<bool> gTcSuspect{false};
 bool tcSuspect() { return gTcSuspect.load(); }
 void markTcSuspect() { gTcSuspect.store(true); }
@@ -415,6 +421,12 @@ cl_status cl_unit_limit_stack(cl_integrator* it, uint32_t entries)
         it->impl.limitStack(entries);
         return CL_OK;
     });
+}
+
+cl_status cl_unit_fail_allocation(int32_t after)
+{
+    clb::failAlloc() = after;
+    return CL_OK;
 }
 
 cl_status cl_unit_validate_bvh(const uint32_t* nodes, uint32_t num_nodes, const float* triangles, uint32_t num_triangles,

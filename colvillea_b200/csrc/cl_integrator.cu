@@ -2460,7 +2460,11 @@ cl_status Integrator::buildEmitters(const cl_emitter_desc* e, uint32_t n, std::s
         }
         out.push_back(d);
     }
+    // Until the new ones are complete there are none: a dome whose build fails
+    // leaves no tables that a kernel or the captured graph could still read.
     hasDome_ = false;
+    emitters_.clear();
+    graphValid_ = false;
     if (domeIdx >= 0)
     {
         CL_CUDA(cudaEventRecord(evA_, stream_), err);
@@ -2471,7 +2475,6 @@ cl_status Integrator::buildEmitters(const cl_emitter_desc* e, uint32_t n, std::s
         hasDome_ = true;
     }
     emitters_.swap(out);
-    graphValid_ = false;
     return CL_OK;
 }
 

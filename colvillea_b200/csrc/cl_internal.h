@@ -21,6 +21,10 @@ namespace clb
 // of a build's wall time).
 double& allocMs();
 
+// Fault injection for tests: this thread's device allocation after the next
+// `failAlloc()` ones reports that memory ran out, once (negative: none).
+int& failAlloc();
+
 // Device allocation owned by one object (the reference's DeviceBuffer,
 // src/core/devices/cudabuffer.h:39-96, with errors returned, not exit()).
 struct DevBuf
@@ -47,7 +51,7 @@ struct DevBuf
         release();
         if (n == 0) n = 16;
         const auto  t0 = std::chrono::steady_clock::now();
-        cudaError_t e  = cudaMalloc(&p, n);
+        cudaError_t e  = failAlloc() >= 0 && failAlloc()-- == 0 ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
         allocMs() += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         if (e != cudaSuccess)
         {

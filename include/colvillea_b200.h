@@ -386,6 +386,10 @@ cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns);
  * that the kernels' own bounds check records.  No counterpart in the reference;
  * it tests the failure path without a fault. */
 cl_status cl_unit_limit_stack(cl_integrator* integrator, uint32_t entries);
+/* The device allocation that follows the calling thread's next `after` ones
+ * reports out of memory, once (negative: none, the default).  No counterpart in
+ * the reference; it tests the failure paths on the host. */
+cl_status cl_unit_fail_allocation(int32_t after);
 /* The validation that every built tree passes, on the caller's tree: nodes of 24
  * words as the traversal reads them (cl_get_bvh's 20, then the leaf word and
  * the three scales as floats; layout in cl_bvh.cuh), triangles as from
