@@ -3087,6 +3087,10 @@ cl_status Integrator::ensureCacheBuffers(std::string* err)
     if (cacheL_.bytes != lb)
     {
         CL_TRY(cacheL_.alloc(lb, err));
+        graphValid_ = false;
+    }
+    if (cacheEncIdx_.bytes != size_t(slots_) * 4)
+    {
         CL_TRY(cacheEncIdx_.alloc(size_t(slots_) * 4, err));
         graphValid_ = false;
     }
