@@ -2328,9 +2328,17 @@ cl_status Integrator::editMesh(uint32_t meshId, const float* pos, const float* n
         const auto   w0      = std::chrono::steady_clock::now();
         const double a0      = allocMs();
         CL_CUDA(cudaEventRecord(evA_, stream_), err);
-        CL_TRY(triPos_.alloc(size_t(numTris_) * 36, err));
-        CL_TRY(gatherTrianglePositions(vtx_.p, triIdx_.p, numTris_, triPos_.f(), stream_, err));
-        cl_status st = buildWideBvh(triPos_.f(), numTris_, stream_, &bvh_, err);
+        cl_status st = triPos_.alloc(size_t(numTris_) * 36, err);
+        if (st == CL_OK) st = gatherTrianglePositions(vtx_.p, triIdx_.p, numTris_, triPos_.f(), stream_, err);
+        // Without the memory for a rebuild a refitted tree still fits the new
+        // vertices; an old one does not, nor is there one once the build has begun.
+        if (st != CL_OK && mode == CL_BVH_UPDATE_AUTO)
+        {
+            std::string ignored;
+            resetIteration(&ignored);
+            return st;
+        }
+        if (st == CL_OK) st = buildWideBvh(triPos_.f(), numTris_, stream_, &bvh_, err);
         triPos_.release();
         if (st != CL_OK)
         {

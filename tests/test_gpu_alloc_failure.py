@@ -81,3 +81,56 @@ def test_first_render(mode):
         assert np.isfinite(f).all()
         after += 1
     assert after == {"plain": 3, "guide": 6, "cache": 8}[mode]  # film, FP64 film, queues, the network's buffers
+
+
+@pytest.mark.parametrize("two", [0, cb.TWO_LEVEL])
+def test_rebuild_after_edit(two):
+    """Each allocation of a rebuild fails in turn: the new vertices have no tree then,
+    so a render is refused until the instances are built again."""
+    s = scenes.config1(4, 32, 32)
+    m = s.meshes[1]
+    moved = (m.positions + np.float32(0.1)).astype(np.float32)
+    fresh = scenes.config1(4, 32, 32)
+    fresh.meshes[1].positions = moved
+    it = cb.load_scene(fresh, flags=cb.COMPAT_ALL | two)
+    it.render(1)
+    want = it.readbackFramebuffer().copy()
+    it.close()
+    it = cb.load_scene(s, flags=cb.COMPAT_ALL | two)
+    it.render(1)
+    for after in range(3):
+        failing(after, lambda: it.updateVertices(1, moved, bvh="rebuild"))
+        with pytest.raises(cb.ClError) as e:
+            it.render(1)
+        assert e.value.status == N.CL_ERR_STATE
+        it.buildTLAS(s.instances)
+        it.resetIterationIndex(); it.render(1)
+        np.testing.assert_allclose(it.readbackFramebuffer(), want, rtol=1e-6)
+    it.updateVertices(1, m.positions); it.updateVertices(1, moved, bvh="rebuild")
+    it.render(1)
+    np.testing.assert_allclose(it.readbackFramebuffer(), want, rtol=1e-6)
+    it.close()
+
+
+def test_auto_keeps_a_refitted_tree():
+    """The rebuild that an automatic update adds finds no memory: the error is
+    reported, and the refitted tree serves the new vertices."""
+    def scene():
+        s = scenes.config1(4, 32, 32)
+        s.meshes[1] = scenes.sphere_mesh(4, (0, 1, 0), 1.0)
+        return s
+
+    p = scene().meshes[1].positions
+    p = p[np.random.default_rng(1).permutation(len(p))] * np.float32(4.0)
+    ref = cb.load_scene(scene())
+    ref.updateVertices(1, p, bvh="auto")
+    assert ref.stats()["bvh_rebuilds"] == 1
+    it = cb.load_scene(scene())
+    failing(0, lambda: it.updateVertices(1, p, bvh="auto"))
+    assert it.stats()["bvh_refits"] == 1 and it.stats()["bvh_rebuilds"] == 0
+    rng = np.random.default_rng(2)
+    rays = np.concatenate([rng.uniform(-5, 5, (2000, 3)), np.full((2000, 1), 1e-3), rng.normal(size=(2000, 3)),
+                           np.full((2000, 1), 1e3)], 1).astype(np.float32)
+    for a, b in zip(it.traceRays(rays), ref.traceRays(rays)):
+        np.testing.assert_array_equal(a, b)
+    it.close(); ref.close()
