@@ -121,7 +121,7 @@ _SIGS = {
     "cl_unit_tc_wait_timeout": [ctypes.POINTER(ctypes.c_uint64)],
     "cl_unit_limit_stack": [vp, u32],
     "cl_unit_validate_bvh": [vp, u32, vp, u32, ctypes.POINTER(u32)],
-    "cl_unit_fail_allocation": [ctypes.c_int32],
+    "cl_unit_fail_allocations": [u32, u32],
     "cl_unit_binary_version": [ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32)],
     "cl_unit_texture_lookup": [ctypes.POINTER(TextureDesc), vp, vp, u32],
     "cl_build_emitters": [vp, ctypes.POINTER(EmitterDesc), u32],

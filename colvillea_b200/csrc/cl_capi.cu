@@ -56,10 +56,10 @@ double& allocMs()
     return ms;
 }
 
-int& failAlloc()
+FailAlloc& failAlloc()
 {
-    static thread_local int k = -1;
-    return k;
+    static thread_local FailAlloc f;
+    return f;
 }
 
 static std::atomic<bool> gTcSuspect{false};
@@ -124,6 +124,17 @@ template <class F> cl_status guarded(F&& f)
     return s;
 }
 
+// A call that allocates beside an integrator's meshes: without room for it, once
+// more with the meshes in host memory.  (Each of these calls starts over when it
+// is repeated.)
+template <class F> cl_status guardedBeside(cl_integrator* it, F&& f)
+{
+    return guarded([&](std::string* err) {
+        const cl_status s = f(err);
+        return s == CL_ERR_OOM && it->impl.spillMeshes() ? f(err) : s;
+    });
+}
+
 #define CL_NEED(ptr)                                                                                                   \
     do                                                                                                                 \
     {                                                                                                                  \
@@ -177,7 +188,7 @@ cl_status cl_build_meshes(cl_integrator* it, const cl_mesh_desc* meshes, uint32_
 cl_status cl_build_instances(cl_integrator* it, const cl_instance_desc* instances, uint32_t count)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.buildInstances(instances, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.buildInstances(instances, count, e); });
 }
 
 cl_status cl_update_mesh_vertices(cl_integrator* it, uint32_t mesh_id, const float* positions, const float* normals,
@@ -198,19 +209,19 @@ cl_status cl_get_bvh(cl_integrator* it, void* nodes, size_t node_bytes, void* tr
 cl_status cl_build_textures(cl_integrator* it, const cl_texture_desc* textures, uint32_t count)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.buildTextures(textures, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.buildTextures(textures, count, e); });
 }
 
 cl_status cl_build_materials(cl_integrator* it, const cl_material_desc* materials, uint32_t count)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.buildMaterials(materials, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.buildMaterials(materials, count, e); });
 }
 
 cl_status cl_build_emitters(cl_integrator* it, const cl_emitter_desc* emitters, uint32_t count)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.buildEmitters(emitters, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.buildEmitters(emitters, count, e); });
 }
 
 cl_status cl_update_camera(cl_integrator* it, const cl_camera* camera)
@@ -222,19 +233,19 @@ cl_status cl_update_camera(cl_integrator* it, const cl_camera* camera)
 cl_status cl_render(cl_integrator* it, uint32_t spp)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.render(spp, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.render(spp, e); });
 }
 
 cl_status cl_readback_film(cl_integrator* it, float* rgba, size_t bytes)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.readbackFilm(rgba, bytes, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.readbackFilm(rgba, bytes, e); });
 }
 
 cl_status cl_readback_film_async(cl_integrator* it, float* rgba, size_t bytes)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.readbackFilmAsync(rgba, bytes, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.readbackFilmAsync(rgba, bytes, e); });
 }
 
 cl_status cl_readback_wait(cl_integrator* it)
@@ -246,13 +257,13 @@ cl_status cl_readback_wait(cl_integrator* it)
 cl_status cl_readback_film_stats(cl_integrator* it, double* sum, double* sumsq, size_t count)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.readbackFilmStats(sum, sumsq, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.readbackFilmStats(sum, sumsq, count, e); });
 }
 
 cl_status cl_resize(cl_integrator* it, uint32_t width, uint32_t height)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.resize(width, height, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.resize(width, height, e); });
 }
 
 cl_status cl_get_film_size(cl_integrator* it, uint32_t* width, uint32_t* height)
@@ -300,19 +311,19 @@ cl_status cl_trace_rays(cl_integrator* it, const float* rays, uint32_t count, fl
                         float* b2)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.traceRays(rays, count, t, prim, b1, b2, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.traceRays(rays, count, t, prim, b1, b2, e); });
 }
 
 cl_status cl_occluded_rays(cl_integrator* it, const float* rays, uint32_t count, uint8_t* occluded)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.occludedRays(rays, count, occluded, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.occludedRays(rays, count, occluded, e); });
 }
 
 cl_status cl_trace_stats(cl_integrator* it, const float* rays, uint32_t count, uint64_t* nodes, uint64_t* triangles)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.traceStats(rays, count, nodes, triangles, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.traceStats(rays, count, nodes, triangles, e); });
 }
 
 cl_status cl_get_dome_tables(cl_integrator* it, float* pU, float* cU, float* pV, float* cV)
@@ -330,7 +341,7 @@ cl_status cl_get_wave_rays(cl_integrator* it, uint64_t* rays, uint32_t capacity,
 cl_status cl_integrator_guide_probe(cl_integrator* it, uint32_t capacity, float* rows, uint32_t* count)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.guideProbe(capacity, rows, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.guideProbe(capacity, rows, count, e); });
 }
 
 cl_status cl_get_dome_alias_tables(cl_integrator* it, uint32_t* alias_row, uint32_t* alias_col)
@@ -346,7 +357,7 @@ cl_status cl_dome_alias_sample(cl_integrator* it, const float* u2, float* dir, f
     CL_NEED(dir);
     CL_NEED(pdf);
     CL_NEED(value);
-    return guarded([&](std::string* e) { return it->impl.domeAliasSample(u2, dir, pdf, value, count, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.domeAliasSample(u2, dir, pdf, value, count, e); });
 }
 
 cl_status cl_unit_bsdf_eval(uint32_t type, const float* params, const float* wo, const float* wi, float* value,
@@ -423,9 +434,9 @@ cl_status cl_unit_limit_stack(cl_integrator* it, uint32_t entries)
     });
 }
 
-cl_status cl_unit_fail_allocation(int32_t after)
+cl_status cl_unit_fail_allocations(uint32_t after, uint32_t count)
 {
-    clb::failAlloc() = after;
+    clb::failAlloc() = clb::FailAlloc{after, count};
     return CL_OK;
 }
 
@@ -585,7 +596,7 @@ cl_status cl_guide_pdf(cl_guide* guide, const float* in9, const float* dir3, uin
 cl_status cl_integrator_set_guiding(cl_integrator* it, const cl_guide_config* config)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.setGuiding(config, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.setGuiding(config, e); });
 }
 
 cl_status cl_integrator_get_guide(cl_integrator* it, cl_guide** guide)
@@ -706,7 +717,7 @@ cl_status cl_cache_train_step(cl_cache* cache, const float* rec12, uint32_t coun
 cl_status cl_integrator_set_radiance_cache(cl_integrator* it, const cl_radiance_cache_config* config)
 {
     CL_NEED(it);
-    return guarded([&](std::string* e) { return it->impl.setRadianceCache(config, e); });
+    return guardedBeside(it, [&](std::string* e) { return it->impl.setRadianceCache(config, e); });
 }
 
 cl_status cl_integrator_get_cache(cl_integrator* it, cl_cache** cache)

@@ -55,7 +55,7 @@ double unordered(unsigned long long v)
 }
 
 // Largest i with start(i) <= x, start non-decreasing, start(0) <= x.
-template <class F> __device__ __forceinline__ uint32_t lastAtMost(uint32_t n, uint32_t x, F start)
+template <class T, class F> __device__ __forceinline__ uint32_t lastAtMost(uint32_t n, T x, F start)
 {
     uint32_t lo = 0u, hi = n;
     while (hi - lo > 1u)
@@ -71,14 +71,14 @@ template <class F> __device__ __forceinline__ uint32_t lastAtMost(uint32_t n, ui
 
 // Smallest mesh id with a vertex index out of range.  tab: per mesh {first
 // triangle, vertices} (meshes are not empty, so the bases increase).
-__global__ void kCheckIndices(const uint32_t* __restrict__ idx, uint32_t nt, const uint2* __restrict__ tab, uint32_t n,
-                              uint32_t* bad)
+__global__ void kCheckIndices(const uint32_t* __restrict__ idx, unsigned long long nt, const ulonglong2* __restrict__ tab,
+                              uint32_t n, uint32_t* bad)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned long long t = blockIdx.x * (unsigned long long)(blockDim.x) + threadIdx.x;
     if (t >= nt) return;
-    const uint32_t m  = lastAtMost(n, t, [&](uint32_t i) { return __ldg(&tab[i].x); });
-    const uint32_t nv = __ldg(&tab[m].y);
-    const uint32_t* v = idx + 3 * size_t(t);
+    const uint32_t  m  = lastAtMost(n, t, [&](uint32_t i) { return __ldg(&tab[i].x); });
+    const uint32_t  nv = uint32_t(__ldg(&tab[m].y));
+    const uint32_t* v  = idx + 3 * size_t(t);
     if (v[0] >= nv || v[1] >= nv || v[2] >= nv) atomicMin(bad, m);
 }
 
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kBlock) kVertexBounds(const float4* __restrict
     }
 }
 
-// Host arrays to consecutive places of one device allocation.  Arrays below
+// Host arrays to consecutive places of one allocation.  Arrays below
 // kPackBelow are gathered in a block of host memory first and copied together,
 // since a copy call costs 3.5 us whatever its size.  cl_build_meshes on 2,000
 // meshes of 12 vertices: 17 ms with a call for each array, 0.6 gathered; 1,000
@@ -256,17 +256,20 @@ constexpr size_t kPackBelow = 65536, kPackBlock = size_t(1) << 20;
 class PackedUpload
 {
 public:
-    PackedUpload(char* dst, size_t total, cudaStream_t st)
-        : dst_(dst), cap_(std::min(kPackBlock, total)), block_(new char[cap_]), st_(st)
+    PackedUpload(const DevBuf& dst, size_t total, cudaStream_t st)
+        : dst_(dst.as<char>()), host_(dst.pinned), cap_(std::min(kPackBlock, total)), block_(new char[cap_]), st_(st)
     {
     }
     // The next `bytes` of the allocation; src null: left as they are or written with zeros (nothing reads them).
     cl_status add(const void* src, size_t bytes, std::string* err)
     {
-        if (bytes >= kPackBelow || bytes > cap_)
+        if (host_ || bytes >= kPackBelow || bytes > cap_)
         {
             CL_TRY(flush(err));
-            if (src) CL_CUDA(cudaMemcpyAsync(dst_ + at_, src, bytes, cudaMemcpyHostToDevice, st_), err);
+            if (src && host_)
+                memcpy(dst_ + at_, src, bytes);
+            else if (src)
+                CL_CUDA(cudaMemcpyAsync(dst_ + at_, src, bytes, cudaMemcpyHostToDevice, st_), err);
             at_ += bytes;
             return CL_OK;
         }
@@ -289,6 +292,7 @@ public:
 
 private:
     char*                   dst_;
+    bool                    host_;
     size_t                  at_ = 0, fill_ = 0, cap_; // bytes placed; gathered behind them
     std::unique_ptr<char[]> block_;
     cudaStream_t            st_;
@@ -299,9 +303,9 @@ uint32_t blocksFor(size_t n) { return uint32_t((n + kBlock - 1) / kBlock); }
 
 cl_status MeshPool::build(const cl_mesh_desc* meshes, uint32_t n, cudaStream_t st, std::string* err)
 {
-    std::vector<MeshInfo> info(n);
-    std::vector<uint2>    tab(n);
-    size_t                nv = 0, nt = 0;
+    std::vector<MeshInfo>   info(n);
+    std::vector<ulonglong2> tab(n);
+    size_t                  nv = 0, nt = 0;
     for (uint32_t m = 0; m < n; ++m)
     {
         const cl_mesh_desc& d = meshes[m];
@@ -310,49 +314,83 @@ cl_status MeshPool::build(const cl_mesh_desc* meshes, uint32_t n, cudaStream_t s
             *err = "mesh " + std::to_string(m) + ": positions, tangents and indices are required";
             return CL_ERR_INVALID_ARG;
         }
-        info[m] = MeshInfo{d.num_vertices, d.num_triangles, uint32_t(nv), uint32_t(nt), d.normals != nullptr,
-                           d.uvs != nullptr};
-        tab[m]  = make_uint2(uint32_t(nt), d.num_vertices);
+        info[m] = MeshInfo{d.num_vertices, d.num_triangles, nv, nt, d.normals != nullptr, d.uvs != nullptr};
+        tab[m]  = make_ulonglong2(nt, d.num_vertices);
         nv += d.num_vertices;
         nt += d.num_triangles;
-    }
-    if (nt >= 0x7fffffffu || nv >= 0xffffffffu)
-    {
-        *err = "meshes too large";
-        return CL_ERR_INVALID_ARG;
     }
     DevBuf mem;
     if (n)
     {
         const size_t words = 11 * nv + 3 * nt, tabAt = (words + 3) / 4 * 4; // 16-byte aligned table
-        CL_TRY(mem.alloc(4 * (tabAt + 2 * size_t(n) + 1), err));
-        float* f = mem.f();
+        cl_status    s     = mem.alloc(4 * (tabAt + 4 * size_t(n) + 1), err);
+        if (s == CL_ERR_OOM) s = mem.allocPinned(4 * words, err);
+        if (s != CL_OK) return s;
+        float*   f   = mem.f();
+        uint32_t bad = kNoMesh;
         // The pool's five parts, mesh after mesh.
-        PackedUpload up(reinterpret_cast<char*>(f), 4 * words, st);
+        PackedUpload up(mem, 4 * words, st);
         for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].positions, 12 * size_t(info[m].nv), err));
         for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].normals, 12 * size_t(info[m].nv), err));
         for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].tangents, 12 * size_t(info[m].nv), err));
         for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].uvs, 8 * size_t(info[m].nv), err));
         for (uint32_t m = 0; m < n; ++m) CL_TRY(up.add(meshes[m].indices, 12 * size_t(info[m].nt), err));
         CL_TRY(up.flush(err));
-        uint2*    dTab = reinterpret_cast<uint2*>(f + tabAt);
-        uint32_t* dBad = reinterpret_cast<uint32_t*>(dTab + n);
-        CL_CUDA(cudaMemcpyAsync(dTab, tab.data(), 8 * size_t(n), cudaMemcpyHostToDevice, st), err);
-        CL_CUDA(cudaMemsetAsync(dBad, 0xff, 4, st), err);
-        kCheckIndices<<<blocksFor(nt), kBlock, 0, st>>>(mem.u() + 11 * nv, uint32_t(nt), dTab, n, dBad);
-        CL_CUDA(cudaGetLastError(), err);
-        uint32_t bad = kNoMesh;
-        CL_CUDA(cudaMemcpyAsync(&bad, dBad, 4, cudaMemcpyDeviceToHost, st), err);
-        CL_CUDA(cudaStreamSynchronize(st), err); // the caller's arrays are free again
+        if (mem.pinned)
+        {
+            for (uint32_t m = 0; m < n && bad == kNoMesh; ++m)
+                for (size_t k = 0; k < 3 * size_t(info[m].nt); ++k)
+                    if (meshes[m].indices[k] >= info[m].nv)
+                    {
+                        bad = m;
+                        break;
+                    }
+        }
+        else
+        {
+            auto* dTab = reinterpret_cast<ulonglong2*>(f + tabAt);
+            auto* dBad = reinterpret_cast<uint32_t*>(dTab + n);
+            CL_CUDA(cudaMemcpyAsync(dTab, tab.data(), 16 * size_t(n), cudaMemcpyHostToDevice, st), err);
+            CL_CUDA(cudaMemsetAsync(dBad, 0xff, 4, st), err);
+            kCheckIndices<<<blocksFor(nt), kBlock, 0, st>>>(mem.u() + 11 * nv, nt, dTab, n, dBad);
+            CL_CUDA(cudaGetLastError(), err);
+            CL_CUDA(cudaMemcpyAsync(&bad, dBad, 4, cudaMemcpyDeviceToHost, st), err);
+        }
+        CL_CUDA(cudaStreamSynchronize(st), err); // the caller's arrays are free again, and nothing reads the old pool
         if (bad != kNoMesh)
         {
             *err = "mesh " + std::to_string(bad) + ": vertex index out of range";
             return CL_ERR_INVALID_ARG;
         }
     }
+    else
+        CL_CUDA(cudaStreamSynchronize(st), err);
     mem_.swap(mem);
     info_.swap(info);
     nv_ = nv;
+    return CL_OK;
+}
+
+bool MeshPool::spill(cudaStream_t st)
+{
+    std::string err;
+    DevBuf      h;
+    if (!mem_.p || mem_.pinned || h.allocPinned(mem_.bytes, &err) != CL_OK) return false;
+    if (cudaMemcpyAsync(h.p, mem_.p, mem_.bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return false;
+    mem_.swap(h);
+    edit_.release();
+    return true;
+}
+
+// Into the pool; host memory is written at once (the stream has been synchronised).
+cl_status MeshPool::put(float* dst, const float* src, size_t bytes, cudaStream_t st, std::string* err)
+{
+    if (mem_.pinned)
+        memcpy(dst, src, bytes);
+    else
+        CL_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st), err);
     return CL_OK;
 }
 
@@ -360,8 +398,8 @@ cl_status MeshPool::updateVertices(uint32_t mesh, const float* pos, const float*
                                    std::string* err)
 {
     MeshInfo&    i = info_[mesh];
-    const size_t n = 3 * size_t(i.nv), b = 4 * n, at = 3 * size_t(i.vtxBase), errAt = (3 * n + 1) / 2 * 2;
-    if (n <= kHostCheckFloats)
+    const size_t n = 3 * size_t(i.nv), b = 4 * n, at = 3 * i.vtxBase, errAt = (3 * n + 1) / 2 * 2;
+    if (mem_.pinned || n <= kHostCheckFloats)
     {
         for (size_t k = 0; k < n; ++k)
             if (!std::isfinite(pos[k]))
@@ -369,9 +407,10 @@ cl_status MeshPool::updateVertices(uint32_t mesh, const float* pos, const float*
                 *err = "vertex " + std::to_string(k / 3) + ": position is not finite";
                 return CL_ERR_INVALID_ARG;
             }
-        CL_CUDA(cudaMemcpyAsync(this->pos() + at, pos, b, cudaMemcpyHostToDevice, st), err);
-        if (nrm) CL_CUDA(cudaMemcpyAsync(this->nrm() + at, nrm, b, cudaMemcpyHostToDevice, st), err);
-        if (tan) CL_CUDA(cudaMemcpyAsync(this->tan() + at, tan, b, cudaMemcpyHostToDevice, st), err);
+        if (mem_.pinned) CL_CUDA(cudaStreamSynchronize(st), err);
+        CL_TRY(put(this->pos() + at, pos, b, st, err));
+        if (nrm) CL_TRY(put(this->nrm() + at, nrm, b, st, err));
+        if (tan) CL_TRY(put(this->tan() + at, tan, b, st, err));
         if (nrm) i.hasN = true;
         return CL_OK;
     }

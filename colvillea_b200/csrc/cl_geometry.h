@@ -10,7 +10,8 @@ namespace clb
 {
 struct MeshInfo
 {
-    uint32_t nv = 0, nt = 0, vtxBase = 0, triBase = 0; // counts; first vertex and triangle in the pool
+    uint32_t nv = 0, nt = 0;           // vertices, triangles
+    size_t   vtxBase = 0, triBase = 0; // the first ones in the pool
     bool     hasN = false, hasUV = false;
 };
 
@@ -21,7 +22,8 @@ struct FlatInst
 {
     double   it[9];  // inverse transpose of the linear part (normals); unused when ident
     float    m[12];
-    uint32_t srcVtx, dstVtx, nv, srcTri, dstTri, nt;
+    uint64_t srcVtx, srcTri;
+    uint32_t dstVtx, nv, dstTri, nt;
     uint32_t w;      // 4th word of the triangles' index entries (the material)
     uint32_t flags;  // 1: normals, 2: uvs, 4: the transform is the identity
 };
@@ -30,13 +32,17 @@ class MeshPool
 {
 public:
     // Uploads the meshes as given and checks their vertex indices.  On an
-    // error the pool keeps what it held.
+    // error the pool keeps what it held.  Without room on the device the pool is
+    // page-locked host memory.
     cl_status build(const cl_mesh_desc* meshes, uint32_t n, cudaStream_t st, std::string* err);
     // New vertices of one mesh (normals, tangents: null keeps them).  Refuses
     // positions that are not finite before anything changes.  The arrays are
     // read until the stream has been synchronised.
     cl_status updateVertices(uint32_t mesh, const float* pos, const float* nrm, const float* tan, cudaStream_t st,
                              std::string* err);
+    // Moves a pool on the device to page-locked host memory and releases the
+    // edits' staging; false where there is nothing to release or no host memory.
+    bool spill(cudaStream_t st);
 
     // The copy of `mesh` at (dstVtx, dstTri) under `M`; refuses a singular M.
     // `what` names it in the message.
@@ -66,6 +72,8 @@ private:
     float*    tan() const { return mem_.f() + 6 * nv_; }
     float*    uv() const { return mem_.f() + 9 * nv_; }
     uint32_t* idx() const { return mem_.u() + 11 * nv_; }
+
+    cl_status put(float* dst, const float* src, size_t bytes, cudaStream_t st, std::string* err);
 
     std::vector<MeshInfo> info_;
     DevBuf                mem_;    // positions | normals | tangents | uvs | triangle indices, mesh after mesh

@@ -2156,7 +2156,7 @@ cl_status Integrator::uploadInstances(std::string* err)
         r.nodes    = blas_[mid]->nodes.as<const uint4>();
         r.tris     = blas_[mid]->tris.as<const float4>();
         r.primBase = primBase;
-        r.triBase  = meshes_[mid].triBase;
+        r.triBase  = uint32_t(meshes_[mid].triBase); // below 2^32, as buildTwoLevel checks
         r.material = inst_[i].material_index;
         r.flags    = det < 0.0 ? 1u : 0u;
         primBase += meshes_[mid].nt;
@@ -2177,9 +2177,14 @@ cl_status Integrator::buildTwoLevel(const cl_instance_desc* inst, uint32_t n, st
     for (uint32_t m = 0; m < nm; ++m)
     {
         const MeshInfo& i = meshes_[m];
-        CL_TRY(meshes_.flatInst(m, kIdentity12, i.vtxBase, i.triBase, 0u, "mesh", &flat[m], err));
         nv += i.nv;
         nt += i.nt;
+        if (nv >= 0xffffffffu || nt >= 0xffffffffu)
+        {
+            *err = "meshes too large for a two-level scene";
+            return CL_ERR_INVALID_ARG;
+        }
+        CL_TRY(meshes_.flatInst(m, kIdentity12, uint32_t(i.vtxBase), uint32_t(i.triBase), 0u, "mesh", &flat[m], err));
     }
     for (uint32_t i = 0; i < n; ++i)
         CL_TRY(meshes_.flatInst(inst[i].mesh_id, inst[i].transform, 0u, 0u, 0u, "instance " + std::to_string(i),
@@ -2279,7 +2284,9 @@ cl_status Integrator::updateMeshVertices(uint32_t meshId, const float* pos, cons
         *err = "unknown BVH update mode";
         return CL_ERR_INVALID_ARG;
     }
-    const cl_status s = editMesh(meshId, pos, nrm, tan, mode, err);
+    cl_status s = editMesh(meshId, pos, nrm, tan, mode, err);
+    if (s == CL_ERR_OOM && spillMeshes()) // again with the meshes in host memory; a tree that is gone is rebuilt
+        s = editMesh(meshId, pos, nrm, tan, twoLevel_ || bvh_.nodes.p ? mode : uint32_t(CL_BVH_UPDATE_REBUILD), err);
     if (s != CL_OK) cudaStreamSynchronize(stream_); // the caller's arrays may still be read (an edit that succeeds waits itself)
     return s;
 }
@@ -2292,7 +2299,7 @@ cl_status Integrator::editMesh(uint32_t meshId, const float* pos, const float* n
     if (meshes_[meshId].hasN != hadN)
     {
         // The mesh's copies have normals from now on.
-        const uint32_t src = meshes_[meshId].vtxBase;
+        const size_t src = meshes_[meshId].vtxBase;
         for (FlatInst& f : flat_)
             if (f.srcVtx == src) f.flags |= 1u;
         CL_TRY(uploadFlat(err));
@@ -2358,6 +2365,7 @@ cl_status Integrator::editMesh(uint32_t meshId, const float* pos, const float* n
         ++rebuilds_;
     }
     msBvhUpdate_ = ms;
+    sceneBuilt_  = true;
     // RenderEngine::compileAccelStructs (renderengine.cpp:65-77): a shape
     // edit restarts progressive accumulation.
     return resetIteration(err);

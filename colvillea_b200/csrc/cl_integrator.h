@@ -188,6 +188,8 @@ public:
     cl_status domeTables(float* pU, float* cU, float* pV, float* cV, std::string* err);
     cl_status domeAliasTables(uint32_t* aliasRow, uint32_t* aliasCol, std::string* err);
     cl_status waveRays(uint64_t* out, uint32_t cap, uint32_t* count, std::string* err) const;
+    // Makes room on the device: the meshes go to host memory (false: nothing to move).
+    bool      spillMeshes() { return meshes_.spill(stream_); }
     // Test of the overflow report: traversal stacks hold at most this many entries.
     void      limitStack(uint32_t entries);
     cl_status guideProbe(uint32_t cap, float* rows, uint32_t* count, std::string* err);

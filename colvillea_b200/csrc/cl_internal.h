@@ -21,16 +21,33 @@ namespace clb
 // of a build's wall time).
 double& allocMs();
 
-// Fault injection for tests: this thread's device allocation after the next
-// `failAlloc()` ones reports that memory ran out, once (negative: none).
-int& failAlloc();
+// Fault injection for tests: of this thread's device allocations the next `after`
+// are made and the `count` that follow report that memory ran out.
+struct FailAlloc
+{
+    uint32_t after = 0, count = 0;
+    bool     now()
+    {
+        if (count == 0u) return false;
+        if (after > 0u)
+        {
+            --after;
+            return false;
+        }
+        --count;
+        return true;
+    }
+};
+FailAlloc& failAlloc();
 
 // Device allocation owned by one object (the reference's DeviceBuffer,
-// src/core/devices/cudabuffer.h:39-96, with errors returned, not exit()).
+// src/core/devices/cudabuffer.h:39-96, with errors returned, not exit()), or
+// page-locked host memory that kernels read in place.
 struct DevBuf
 {
-    void*  p     = nullptr;
-    size_t bytes = 0;
+    void*  p      = nullptr;
+    size_t bytes  = 0;
+    bool   pinned = false; // host memory; its owner waits for its readers before a release
     DevBuf()     = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -39,19 +56,36 @@ struct DevBuf
     {
         std::swap(p, o.p);
         std::swap(bytes, o.bytes);
+        std::swap(pinned, o.pinned);
     }
     void release()
     {
-        if (p) cudaFree(p);
-        p     = nullptr;
-        bytes = 0;
+        if (p) pinned ? cudaFreeHost(p) : cudaFree(p);
+        p      = nullptr;
+        bytes  = 0;
+        pinned = false;
+    }
+    cl_status allocPinned(size_t n, std::string* err)
+    {
+        release();
+        const cudaError_t e = cudaHostAlloc(&p, n, cudaHostAllocDefault);
+        if (e != cudaSuccess)
+        {
+            p    = nullptr;
+            *err = std::string("cudaHostAlloc(") + std::to_string(n) + ") failed: " + cudaGetErrorString(e);
+            cudaGetLastError();
+            return e == cudaErrorMemoryAllocation ? CL_ERR_OOM : CL_ERR_CUDA;
+        }
+        bytes  = n;
+        pinned = true;
+        return CL_OK;
     }
     cl_status alloc(size_t n, std::string* err)
     {
         release();
         if (n == 0) n = 16;
         const auto  t0 = std::chrono::steady_clock::now();
-        cudaError_t e  = failAlloc() >= 0 && failAlloc()-- == 0 ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
+        cudaError_t e  = failAlloc().now() ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
         allocMs() += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         if (e != cudaSuccess)
         {

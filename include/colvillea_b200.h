@@ -249,7 +249,13 @@ cl_status cl_integrator_create(cl_integrator_type type, uint32_t width, uint32_t
                                const cl_render_config* config, cl_integrator** out);
 cl_status cl_integrator_destroy(cl_integrator* integrator);
 
-/* Integrator::buildBLAS (integrator.h:47). */
+/* Integrator::buildBLAS (integrator.h:47).  The meshes stay in device memory as
+ * given (44 bytes per vertex, 12 per triangle) until the next call or the
+ * integrator's end; with no room for them there, or when a later call finds none
+ * beside them, in page-locked host memory, which builds and edits then read in
+ * place.  Ray queries keep 48 bytes per ray of the largest call (at most 2^21
+ * rays), edits 36 bytes per vertex of the largest edited mesh, the networks'
+ * host entry points the rows of their largest call. */
 cl_status cl_build_meshes(cl_integrator* integrator, const cl_mesh_desc* meshes, uint32_t count);
 /* Integrator::buildTLAS + buildGeometryEntities (integrator.h:49-54): builds the
  * 8-wide BVH on the device over all instances. */
@@ -386,10 +392,10 @@ cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns);
  * that the kernels' own bounds check records.  No counterpart in the reference;
  * it tests the failure path without a fault. */
 cl_status cl_unit_limit_stack(cl_integrator* integrator, uint32_t entries);
-/* The device allocation that follows the calling thread's next `after` ones
- * reports out of memory, once (negative: none, the default).  No counterpart in
- * the reference; it tests the failure paths on the host. */
-cl_status cl_unit_fail_allocation(int32_t after);
+/* Of the calling thread's device allocations the next `after` are made and the
+ * `count` that follow report out of memory (0: none, the default).  No
+ * counterpart in the reference; it tests the failure paths on the host. */
+cl_status cl_unit_fail_allocations(uint32_t after, uint32_t count);
 /* The validation that every built tree passes, on the caller's tree: nodes of 24
  * words as the traversal reads them (cl_get_bvh's 20, then the leaf word and
  * the three scales as floats; layout in cl_bvh.cuh), triangles as from

@@ -1,4 +1,5 @@
-"""Device allocations that fail, injected on the host: the call reports CL_ERR_OOM,
+"""Device allocations that fail, injected on the host (from the given one on, so
+that what a call repeats with more room fails too): the call reports CL_ERR_OOM,
 what follows uses nothing of what it replaced, and the same call succeeds
 afterwards with the results that it has always had."""
 import numpy as np
@@ -12,13 +13,13 @@ pytestmark = pytest.mark.gpu
 
 
 def failing(after, call):
-    N.call("cl_unit_fail_allocation", after)
+    N.call("cl_unit_fail_allocations", after, 1000)
     try:
         with pytest.raises(cb.ClError) as e:
             call()
         assert e.value.status == N.CL_ERR_OOM
     finally:
-        N.call("cl_unit_fail_allocation", -1)
+        N.call("cl_unit_fail_allocations", 0, 0)
 
 
 def test_dome_build():
@@ -63,14 +64,14 @@ def test_first_render(mode):
     after = 0
     while True:
         it = make()
-        N.call("cl_unit_fail_allocation", after)
+        N.call("cl_unit_fail_allocations", after, 1000)
         try:
             it.render(1)
             done = True
         except cb.ClError as e:
             assert e.status == N.CL_ERR_OOM
             done = False
-        N.call("cl_unit_fail_allocation", -1)
+        N.call("cl_unit_fail_allocations", 0, 0)
         if done:
             it.close()
             break
@@ -127,7 +128,7 @@ def test_auto_keeps_a_refitted_tree():
     assert ref.stats()["bvh_rebuilds"] == 1
     it = cb.load_scene(scene())
     failing(0, lambda: it.updateVertices(1, p, bvh="auto"))
-    assert it.stats()["bvh_refits"] == 1 and it.stats()["bvh_rebuilds"] == 0
+    assert it.stats()["bvh_refits"] >= 1 and it.stats()["bvh_rebuilds"] == 0
     rng = np.random.default_rng(2)
     rays = np.concatenate([rng.uniform(-5, 5, (2000, 3)), np.full((2000, 1), 1e-3), rng.normal(size=(2000, 3)),
                            np.full((2000, 1), 1e3)], 1).astype(np.float32)
