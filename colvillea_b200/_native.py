@@ -119,6 +119,7 @@ _SIGS = {
     "cl_build_textures": [vp, ctypes.POINTER(TextureDesc), u32],
     "cl_unit_normal_frame": [vp, vp, u32],
     "cl_unit_tc_wait_timeout": [ctypes.POINTER(ctypes.c_uint64)],
+    "cl_unit_box_reciprocals": [vp, vp, u32],
     "cl_unit_limit_stack": [vp, u32],
     "cl_unit_validate_bvh": [vp, u32, vp, u32, ctypes.POINTER(u32)],
     "cl_unit_fail_allocations": [u32, u32],

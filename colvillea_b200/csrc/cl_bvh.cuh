@@ -116,9 +116,10 @@ __device__ __forceinline__ void loadTri(const float4* __restrict__ tris, uint32_
 
 // Reciprocals of a ray direction's components for the box tests (components
 // below 1e-30 count as that): the hardware approximation and one Newton step,
-// within an ulp of the IEEE quotient, whose three calls were a sixth of the work
-// of giving a lane its next ray.  Components beyond the approximation's range
-// take the quotient.
+// the IEEE quotient itself for all 2^23 mantissas of a binade and within an ulp
+// of it over the range; its three calls were a sixth of the work of giving a
+// lane its next ray.  Components beyond the approximation's range take the
+// quotient.
 __device__ __forceinline__ float boxRcp(float x)
 {
     float r;

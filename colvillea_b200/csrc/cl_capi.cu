@@ -88,6 +88,7 @@ cl_status unitFrame(const float*, const float*, const float*, const float*, floa
 cl_status unitPcg(const uint32_t*, uint32_t*, uint32_t, std::string*);
 cl_status unitNormalFrame(const float*, float*, uint32_t, std::string*);
 cl_status unitTcWaitTimeout(uint64_t*, std::string*);
+cl_status unitBoxReciprocals(const float*, float*, uint32_t, std::string*);
 cl_status unitValidateBvh(const uint32_t*, uint32_t, const float*, uint32_t, uint32_t*, std::string*);
 cl_status unitBinaryVersion(int32_t*, int32_t*, std::string*);
 cl_status unitTextureLookup(const cl_texture_desc*, const float*, float*, uint32_t, std::string*);
@@ -423,6 +424,11 @@ cl_status cl_unit_normal_frame(const float* in, float* frame, uint32_t count)
 cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns)
 {
     return guarded([&](std::string* e) { return clb::unitTcWaitTimeout(waited_ns, e); });
+}
+
+cl_status cl_unit_box_reciprocals(const float* direction, float* inverse, uint32_t count)
+{
+    return guarded([&](std::string* e) { return clb::unitBoxReciprocals(direction, inverse, count, e); });
 }
 
 cl_status cl_unit_limit_stack(cl_integrator* it, uint32_t entries)

@@ -2,6 +2,7 @@
 // tests against the CPU oracle: the same inlined code the integrator kernels
 // run, one item per thread, host buffers in and out.
 #include "cl_device.cuh"
+#include "cl_bvh.cuh"
 #include "cl_internal.h"
 #include "cl_mlp_tc.cuh"
 #include "cl_texture.h"
@@ -408,6 +409,28 @@ __global__ void kTexLookup(const unsigned long long* tex, const float* uv, float
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = tex2D<float4>(cudaTextureObject_t(tex[0]), uv[2 * size_t(i)], uv[2 * size_t(i) + 1]);
+}
+
+__global__ void kBoxReciprocals(const float* d, float* inv, uint32_t n)
+{
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const f3 r = boxReciprocals(f3{d[3 * size_t(i)], d[3 * size_t(i) + 1], d[3 * size_t(i) + 2]});
+    inv[3 * size_t(i)]     = r.x;
+    inv[3 * size_t(i) + 1] = r.y;
+    inv[3 * size_t(i) + 2] = r.z;
+}
+
+cl_status unitBoxReciprocals(const float* d, float* inv, uint32_t n, std::string* err)
+{
+    CL_REQ(d && inv);
+    if (!n) return CL_OK;
+    Batch  b(err);
+    float *x, *y;
+    CL_TRY(b.in(d, 3 * size_t(n), &x));
+    CL_TRY(b.out(inv, 3 * size_t(n), &y));
+    kBoxReciprocals<<<grid(n), 128>>>(x, y, n);
+    return b.finish();
 }
 
 cl_status unitNormalFrame(const float* in, float* out, uint32_t n, std::string* err)

@@ -386,6 +386,8 @@ cl_status cl_unit_normal_frame(const float* in, float* frame, uint32_t count);
  * CL_ERR_TIMEOUT with the time waited, and the context stays usable.  No
  * counterpart in the reference; it tests the failure path without a fault. */
 cl_status cl_unit_tc_wait_timeout(uint64_t* waited_ns);
+/* The box tests' reciprocals of ray directions: 3 floats in, 3 out per item. */
+cl_status cl_unit_box_reciprocals(const float* direction, float* inverse, uint32_t count);
 /* Limits the integrator's traversal stacks to `entries` (0xffffffff: as many
  * as its trees need, the default): with too few, cl_render, cl_trace_rays,
  * cl_occluded_rays and cl_trace_stats return CL_ERR_STATE with the overflow
