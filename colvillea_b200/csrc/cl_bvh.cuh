@@ -344,23 +344,6 @@ __device__ __forceinline__ bool travStep(const BvhView& bvh, Trav& s, uint2* sta
     return false;
 }
 
-// Whole traversal of one ray (used where lanes are not refilled).
-template <bool ANY, bool STATS>
-__device__ __forceinline__ uint32_t traverse(const BvhView& bvh, f3 o, f3 d, float tmin, float tmax, float* tHit,
-                                             float* b1Hit, float* b2Hit, uint2* stack, TraceCounters* cnt,
-                                             uint32_t* err, const uint8_t* keyLut)
-{
-    Trav s;
-    travInit(s, o, d, tmin, tmax);
-    while (!travStep<STATS>(bvh, s, stack, cnt, err, keyLut, ANY))
-    {
-    }
-    *tHit  = s.bt;
-    *b1Hit = s.b1;
-    *b2Hit = s.b2;
-    return s.best;
-}
-
 // ---------------------------------------------------------------------------
 // Two-level traversal (CL_TWO_LEVEL).  The same node and triangle steps as
 // travStep, over the top tree and, inside an instance, over its mesh's tree.
@@ -551,25 +534,6 @@ __device__ __forceinline__ bool trav2Step(const BvhView& bvh, Trav2& s, uint2* s
         }
     }
     return false;
-}
-
-// Whole two-level traversal of one ray: *inst = the hit's instance, the
-// return value its triangle id within the instance's mesh (kMissPrim: none).
-template <bool ANY, bool STATS>
-__device__ __forceinline__ uint32_t traverse2(const BvhView& bvh, f3 o, f3 d, float tmin, float tmax, float* tHit,
-                                              float* b1Hit, float* b2Hit, uint32_t* inst, uint2* stack,
-                                              TraceCounters* cnt, uint32_t* err, const uint8_t* keyLut)
-{
-    Trav2 s;
-    trav2Init(bvh, s, o, d, tmin, tmax);
-    while (!trav2Step<STATS>(bvh, s, stack, cnt, err, keyLut, ANY))
-    {
-    }
-    *tHit  = s.bt;
-    *b1Hit = s.b1;
-    *b2Hit = s.b2;
-    *inst  = s.bestInst;
-    return s.best;
 }
 
 } // namespace clb

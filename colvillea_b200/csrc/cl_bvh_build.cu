@@ -1248,9 +1248,7 @@ cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh*
             CL_CUDA(cudaMemcpyAsync(&rootRef, list[cur].C, 4, cudaMemcpyDeviceToHost, st), err);
             CL_CUDA(cudaStreamSynchronize(st), err);
         }
-        if (m == 1)
-            out->buildIterations = uint32_t(iters);
-        else
+        if (m != 1)
         {
             // Fall back to the LBVH radix tree (Karras 2012) with bottom-up boxes
             // (rank: the arrival counters).
@@ -1262,7 +1260,6 @@ cl_status buildWideBvh(const float* dTri9, uint32_t n, cudaStream_t st, WideBvh*
                                               nlo.f(), nhi.f(), count.u(), rank.u());
             CL_CUDA(cudaGetLastError(), err);
             rootRef = 0u;
-            out->buildIterations = 0;
         }
     }
     else

@@ -51,7 +51,6 @@ __device__ __forceinline__ f3 cross(f3 a, f3 b)
 }
 __device__ __forceinline__ f3 normalize(f3 a) { return a * (1.0f / sqrtf(dot(a, a))); }
 __device__ __forceinline__ bool nonzero(f3 v) { return v.x > 0.0f || v.y > 0.0f || v.z > 0.0f; }
-__device__ __forceinline__ float comp(f3 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : v.z); }
 
 // ---------------------------------------------------------------------------
 // Sampler (libkernel/base/sampler.h:16-78): pcg4d hash of
@@ -779,9 +778,10 @@ struct RayPre
 };
 
 // The axes in cyclic order ending with kz.  (The test's authors swap the first
-// two for rays against kz to keep the triangle's winding; without the swap U, V,
-// W, the determinant and T only change sign together, exactly, which t and the
-// barycentrics do not show, and two registers and six selects are saved.)
+// two for rays against kz to keep the triangle's winding.  Without the swap U, V,
+// W, the determinant and T of such a ray change sign together, exactly, so t and
+// the barycentrics keep their values, but for the sign of a barycentric that is
+// exactly zero; two registers and six selects are saved.)
 __device__ __forceinline__ f3 rotateAxes(f3 v, int kz)
 {
     const bool z0 = kz == 0, z1 = kz == 1;

@@ -36,7 +36,6 @@ template <int NH, int NO> struct MlpShape
 using GuideShape = MlpShape<3, 48>;
 using CacheShape = MlpShape<1, 16>;
 constexpr int kOut       = GuideShape::kOut;
-constexpr int kMlpParams = GuideShape::kParams; // 21504
 
 // Hash grid: table[l * T + index] holds the 2 features of an entry.
 struct GridView

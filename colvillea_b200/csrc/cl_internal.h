@@ -167,7 +167,7 @@ struct WideBvh
     // Nodes of tree level d are [levels[d], levels[d + 1]): the collapse
     // allocates each level's nodes in one launch.
     std::vector<uint32_t> levels;
-    uint32_t numNodes = 0, depth = 0, numTris = 0, buildIterations = 0;
+    uint32_t numNodes = 0, depth = 0, numTris = 0;
     void     release()
     {
         mem.release();
