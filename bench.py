@@ -31,7 +31,7 @@ sys.path.insert(0, ROOT)
 METRIC = "Mpaths/s and equal-time relMSE vs FP64 oracle, neural-guided vs plain, 1 B200"
 UNIT = "Mpaths/s"
 L2_BYTES = 126 * 1024 * 1024
-RAY_IN, HIT_OUT, NODE_BYTES, TRI_BYTES = 32, 16, 80, 48
+RAY_IN, HIT_OUT, NODE_BYTES, TRI_BYTES = 32, 16, 96, 48  # a node visit is three 32-byte loads
 
 
 def parse():
@@ -604,8 +604,8 @@ def main():
         ms_dev += st["ms_last_render"]
         rays_c += st["last_rays_closest"]; rays_s += st["last_rays_shadow"]
         # kRaygen, then per wave: kTraceClosest, kClassifyHits, 4 x kShade, kTraceShadow, kShadowResolve,
-        # kAdvance, kPathTail
-        launches += 1 + 10 * st["waves"]
+        # kAdvance, kPathTail; a pass that fits kPathTail (counted as one wave) is that launch alone.
+        launches += 2 if st["waves"] == 1 else 1 + 10 * st["waves"]
     ev1.record()
     torch.cuda.synchronize()
     clk = clocks.stop()
@@ -703,7 +703,8 @@ def main():
                      "traffic": round(traffic * prays_c / max(1, trace_launches)) if traffic else None,
                      "bytes_per_ray": round(bytes_per_ray, 1), "nodes_per_ray": round(nodes_per_ray, 2),
                      "tris_per_ray": round(tris_per_ray, 2),
-                     "formula": "per closest-hit ray: 32 B ray + 16 B hit + 80 B x nodes + 48 B x triangles",
+                     "formula": "bytes touched per closest-hit ray (most come from L1 and L2; traffic is DRAM's): "
+                                "32 B ray + 16 B hit + 96 B x nodes + 48 B x triangles",
                      "timing": "kTraceClosest's CUDA-event time on its stream, in a stage-profiled pass of the "
                                "same steps"},
         "clocks": clk, "gpu_launches": launches,

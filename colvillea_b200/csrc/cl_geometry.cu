@@ -2,13 +2,13 @@
 //
 // The meshes are copied to the device as the caller gives them and stay there;
 // flattening (the reference's TLAS has no transforms, optix.cu:115), edits and
-// the two-level scenes' pools and boxes read them from there.  These passes ran
-// on one host core before: for 1.17 M triangles (0.6 M vertices) 7 ms of mesh
-// copies and 40 ms of flattening and uploads when a scene is opened, and 2.5 ms
-// per edit of a 262 k vertex mesh.  Here they are bound by memory: each vertex
-// reads 44 B and writes 48 B, each triangle reads 12 B and writes 16 B (about
-// 0.1 ms for that scene), so an upload costs what its copies from pageable
-// memory cost.  The arithmetic is the host's, in double and in the same order.
+// the two-level scenes' pools and boxes read them from there.  The passes are
+// bound by memory: each vertex reads 44 B and writes 48 B, each triangle reads
+// 12 B and writes 16 B (0.1 ms for 1.17 M triangles; one host core took 47 ms
+// for their copies and flattening), so an upload costs what its copies from
+// pageable memory cost.  The arithmetic is in double and in a host loop's order.
+// Where the meshes find no room on the device they lie in page-locked host
+// memory, and the same kernels read them over PCIe.
 #include "cl_geometry.h"
 
 #include <cfloat>

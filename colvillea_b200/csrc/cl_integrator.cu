@@ -1153,14 +1153,15 @@ __global__ void __launch_bounds__(128) kShadowResolve(Params P, int cur)
 // lanes at a time took 1.1 to 1.5 times as long).  With fewer paths than lanes
 // each warp takes an even share of them: a step costs a warp what its lanes'
 // divergent loads and branches cost together.
-// kTailMaxRays: measured with 2048, 4096, 8192, 16384 and 24576 rays on a 256x256
-// frame of 10 k triangles (device time 474, 394, 394, 460 and 455 us), a
-// 1920x1080 frame of 1.2 M triangles at one sample (3.04, 3.04, 3.11, 3.16 and
-// 3.24 ms), 1280x720x2 over 577 two-level instances at depth 16 (4.96, 4.91,
-// 4.96, 5.00 and 5.14 ms; without this launch 7.5 against 6.4 before the
-// traversal's other changes) and 640x360 over 0.7 M triangles (0.92, 0.92, 0.86,
-// 0.86 and 0.90 ms).  Four trained samples of the radiance cache at 960x540 take
-// 4.6 ms with any of them and took 10.3 without.
+// kTailMaxRays: two to three rays for each of the 2,368 resident warps.  Measured
+// with 2048, 4096, 6144, 8192, 16384 and 24576 rays on a 256x256 frame of 10 k
+// triangles (device time 477, 390, 389, 390, 458 and 457 us), a 1920x1080 frame of
+// 1.2 M triangles at one sample (3.06, 3.07, 3.10, 3.13, 3.16 and 3.25 ms),
+// 1280x720x2 over 577 two-level instances at depth 16 (4.98, 4.90, 4.96, 4.95,
+// 5.03 and 5.14 ms) and 640x360 over 0.7 M triangles (0.93, 0.92, 0.87, 0.87, 0.87
+// and 0.90 ms): which wave the tail takes over after makes the steps.  Four trained
+// samples of the radiance cache at 960x540 take 4.6 ms with any of them and took
+// 10.3 without this launch.
 // Not for guided passes (every vertex needs its network evaluation first);
 // with the radiance cache only once the waves have brought every path past
 // its query (wp.tailNeed).  kAdvance decides (Counters::tailNow).
